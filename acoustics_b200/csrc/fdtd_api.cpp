@@ -376,7 +376,7 @@ fdtd_status run_classification(fdtd_solver* s) {
     ClsBoxes& B = s->hP.boxes;
     classification_boxes(s, B);
     CUDA_TRY(s, fdtd::counted_copyAsync(s, &s->dP->boxes, &B, sizeof(ClsBoxes), cudaMemcpyHostToDevice, s->stream));
-    CUDA_TRY(s, launch_classify(s->dP, s->N, B, false, s->stream));
+    CUDA_TRY(s, launch_classify(s->dP, s->N, B, false, !s->mesh_alloc.empty(), s->stream));
     s->cls_boxes_current = true;
     s->launches += B.ufirst[B.n] > 0 ? 3 : 2;
     return FDTD_OK;
@@ -1060,13 +1060,16 @@ fdtd_status fdtd_solver_create(const fdtd_scene_desc* sc, const fdtd_options* op
         const MeshHost& M = s->meshes[m];
         if (M.tris.empty()) continue;
         const size_t nb = M.nodes.size() * sizeof(MeshNode), tb = M.tris.size() * sizeof(MeshTri);
+        const size_t pb = M.top.size() * sizeof(int);
         void* d = nullptr;
-        CUDA_TRY(nullptr, cudaMalloc(&d, nb + tb));
+        CUDA_TRY(nullptr, cudaMalloc(&d, nb + tb + pb));
         s->mesh_alloc.push_back(d);
-        s->arena_bytes += nb + tb;
+        s->arena_bytes += nb + tb + pb;
         CUDA_TRY(nullptr, fdtd::counted_copy(s.get(), d, M.nodes.data(), nb, cudaMemcpyHostToDevice));
         CUDA_TRY(nullptr, fdtd::counted_copy(s.get(), (char*)d + nb, M.tris.data(), tb, cudaMemcpyHostToDevice));
-        const MeshView v{(const MeshNode*)d, (const MeshTri*)((char*)d + nb), (int)M.nodes.size(), (int)M.tris.size()};
+        CUDA_TRY(nullptr, fdtd::counted_copy(s.get(), (char*)d + nb + tb, M.top.data(), pb, cudaMemcpyHostToDevice));
+        const MeshView v{(const MeshNode*)d, (const MeshTri*)((char*)d + nb), (int)M.nodes.size(), (int)M.tris.size(),
+                         (const int*)((char*)d + nb + tb), (int)M.top.size()};
         for (auto& o : s->objs)
             if (o.d.shape == FDTD_SHAPE_MESH && o.d.mesh == (int)m) o.mview = v;
     }
@@ -1371,7 +1374,8 @@ fdtd_status fdtd_scene_info(const fdtd_scene_desc* sc, const fdtd_options* opt, 
         const int m = sc->objects[i].shape == FDTD_SHAPE_MESH ? sc->objects[i].mesh : -1;
         if (m < 0 || counted[m]) continue;
         counted[m] = 1;
-        info->device_bytes += (int64_t)sc->meshes[m].n_triangles * (int64_t)(sizeof(MeshTri) + 2 * sizeof(MeshNode));
+        info->device_bytes += (int64_t)sc->meshes[m].n_triangles * (int64_t)(sizeof(MeshTri) + 2 * sizeof(MeshNode)) +
+                              MESH_TOP * (int64_t)sizeof(int);
     }
     info->time = sc->start_time;
     info->time_step = s.k;

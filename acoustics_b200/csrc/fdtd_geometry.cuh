@@ -81,25 +81,69 @@ FDTD_HD bool occupy_by_constraint(const SolveParams& P, const double p[3]) {
     return false;
 }
 
+// How far from a cell's centre its solid-test samples lie (h/4), with a margin
+// over rounding: a body farther than this from the centre holds no sample.
+FDTD_HD double sample_reach(const SolveParams& P) { return 0.25 * P.h * (1.0 + 1e-6); }
+
+// True when p is farther than `reach` from the body's bounding box.
+FDTD_HD bool beyond_bbox(const DevObject& o, const double p[3], double reach) {
+    for (int d = 0; d < 3; ++d)
+        if (p[d] < o.bmin[d] - reach || p[d] > o.bmax[d] + reach) return true;
+    return false;
+}
+
 // isFluid lambda of classifyCells_FAST (MAC_Grid.cpp:3566-3577): the centre and
 // the six points centre +- h/4 along each axis must be outside every object.
+// The samples are tried only against the bodies that can reach one: a body
+// whose box, or whose surface, is farther than h/4 from the centre cannot (the
+// distances of spheres, boxes and meshes are exact; an ellipsoid's is an
+// estimate with the exact sign, so its samples are always tried).
 FDTD_HD bool is_fluid(const SolveParams& P, const double pos[3], int& type) {
-    bool fluid = !occupy_by_constraint(P, pos) && occupy_by_object(P, pos) < 0;
-    for (int d = 0; d < 3 && fluid; ++d) {
+    bool fluid = !occupy_by_constraint(P, pos);
+    const double reach = sample_reach(P);
+    unsigned near = 0;
+    for (int o = 0; o < P.n_obj && fluid; ++o) {
+        if (beyond_bbox(P.obj[o], pos, reach)) continue;
+        const double dist = sdf_local(P.obj[o], pos);
+        if (dist < DISTANCE_TOLERANCE) fluid = false;
+        else if (dist <= reach || P.obj[o].shape == 2) near |= 1u << o;
+    }
+    for (int d = 0; d < 3 && fluid && near; ++d) {
         for (int s = -1; s <= 1 && fluid; s += 2) {
             double q[3] = {pos[0], pos[1], pos[2]};
             q[d] = q[d] + (s > 0 ? 1.0 : -1.0) * 0.25 * P.h;
-            fluid = occupy_by_object(P, q) < 0;
+            for (int o = 0; o < P.n_obj && fluid; ++o)
+                if ((near >> o) & 1u) fluid = !(distance_to_mesh(P.obj[o], q) < DISTANCE_TOLERANCE);
         }
     }
     if (!fluid) type = occupy_by_constraint(P, pos) ? 1 : 0;
     return fluid;
 }
 
+// p lies in the body's scaled box, where distance_to_mesh evaluates the distance.
+FDTD_HD bool in_scaled_bbox(const DevObject& o, const double p[3]) {
+    for (int d = 0; d < 3; ++d) {
+        const double sd = o.bdim[d] * AABB_CHECK_TOLERANCE_SCALE;
+        if (!(p[d] < (o.bcen[d] + sd) && p[d] > (o.bcen[d] - sd))) return false;
+    }
+    return true;
+}
+
 // FDTD_Objects::LowestObjectDistance (FDTD_Objects.cpp:240-257): first object
-// with the smallest |distance|; -1 when the scene has no objects.
+// with the smallest |distance|; -1 when the scene has no objects.  Without
+// `distance` a distance is only evaluated where two bodies' scaled boxes hold p:
+// the distance to the others is DBL_MAX, which never replaces the first body.
 FDTD_HD int lowest_object(const SolveParams& P, const double p[3], double* distance = nullptr) {
     if (P.n_obj == 0) return -1;
+    if (!distance) {
+        int held = 0, only = 0;
+        for (int o = 0; o < P.n_obj; ++o)
+            if (in_scaled_bbox(P.obj[o], p)) {
+                ++held;
+                only = o;
+            }
+        if (held <= 1) return only;
+    }
     double dist = DBL_MAX;
     int id = 0;
     for (int o = 0; o < P.n_obj; ++o) {
@@ -108,6 +152,39 @@ FDTD_HD int lowest_object(const SolveParams& P, const double p[3], double* dista
     }
     if (distance) *distance = dist;
     return id;
+}
+
+// x in the body's frame
+FDTD_HD void to_object_frame(const DevObject& o, const double x[3], double q[3]) {
+    const double r[3] = {x[0] - o.c[0], x[1] - o.c[1], x[2] - o.c[2]};
+    for (int j = 0; j < 3; ++j) q[j] = o.R[0 * 3 + j] * r[0] + o.R[1 * 3 + j] * r[1] + o.R[2 * 3 + j] * r[2];
+}
+
+// The mesh branch of ReflectAgainstBoundary from the closest point cpo (object
+// frame, on triangle tri, signed distance dist) of the reference's search
+// (FDTD_RigidObject.cpp:453-512; KD_NEAREST_TOLERANCE is 0, so its
+// push-along-the-normal branch never runs).
+FDTD_HD void reflect_from_closest(const DevObject& o, const double x[3], const double cpo[3], int tri, double image[3],
+                                  double bp[3], double nrm[3], double dist) {
+    for (int i = 0; i < 3; ++i)
+        bp[i] = o.c[i] + (o.R[i * 3 + 0] * cpo[0] + o.R[i * 3 + 1] * cpo[1] + o.R[i * 3 + 2] * cpo[2]);
+    const double g[3] = {bp[0] - x[0], bp[1] - x[1], bp[2] - x[2]};
+    double e[3];
+    if (sqrt(g[0] * g[0] + g[1] * g[1] + g[2] * g[2]) > 1e-10) {  // EPS, config.h:45
+        if (dist < 0.0) {
+            for (int i = 0; i < 3; ++i) e[i] = bp[i] - x[i];
+            for (int i = 0; i < 3; ++i) image[i] = bp[i] + e[i];
+        } else {
+            for (int i = 0; i < 3; ++i) e[i] = -bp[i] + x[i];
+            for (int i = 0; i < 3; ++i) image[i] = x[i] + e[i];
+        }
+    } else {  // on the triangle: its normal
+        const double* n = o.mesh.tris[tri].nf;
+        for (int i = 0; i < 3; ++i) e[i] = o.R[i * 3 + 0] * n[0] + o.R[i * 3 + 1] * n[1] + o.R[i * 3 + 2] * n[2];
+        for (int i = 0; i < 3; ++i) image[i] = x[i];
+    }
+    const double en = sqrt(e[0] * e[0] + e[1] * e[1] + e[2] * e[2]);
+    for (int i = 0; i < 3; ++i) nrm[i] = en > 0.0 ? e[i] / en : 0.0;
 }
 
 // FDTD_RigidObject::ReflectAgainstBoundary (FDTD_RigidObject.cpp:429-536, closest
@@ -120,31 +197,11 @@ FDTD_HD void reflect_against_boundary(const DevObject& o, const double x[3], dou
                                       double nrm[3], double& dist) {
     const double r[3] = {x[0] - o.c[0], x[1] - o.c[1], x[2] - o.c[2]};
     if (o.shape == 3) {
-        // mesh: closest point of the reference's search (FDTD_RigidObject.cpp:453-512;
-        // KD_NEAREST_TOLERANCE is 0, so its push-along-the-normal branch never runs)
         double q[3], cpo[3];
-        for (int j = 0; j < 3; ++j) q[j] = o.R[0 * 3 + j] * r[0] + o.R[1 * 3 + j] * r[1] + o.R[2 * 3 + j] * r[2];
+        to_object_frame(o, x, q);
         int tri = 0;
         dist = mesh_closest_ref(o.mesh, q, cpo, tri);
-        for (int i = 0; i < 3; ++i)
-            bp[i] = o.c[i] + (o.R[i * 3 + 0] * cpo[0] + o.R[i * 3 + 1] * cpo[1] + o.R[i * 3 + 2] * cpo[2]);
-        const double g[3] = {bp[0] - x[0], bp[1] - x[1], bp[2] - x[2]};
-        double e[3];
-        if (sqrt(g[0] * g[0] + g[1] * g[1] + g[2] * g[2]) > 1e-10) {  // EPS, config.h:45
-            if (dist < 0.0) {
-                for (int i = 0; i < 3; ++i) e[i] = bp[i] - x[i];
-                for (int i = 0; i < 3; ++i) image[i] = bp[i] + e[i];
-            } else {
-                for (int i = 0; i < 3; ++i) e[i] = -bp[i] + x[i];
-                for (int i = 0; i < 3; ++i) image[i] = x[i] + e[i];
-            }
-        } else {  // on the triangle: its normal
-            const double* n = o.mesh.tris[tri].nf;
-            for (int i = 0; i < 3; ++i) e[i] = o.R[i * 3 + 0] * n[0] + o.R[i * 3 + 1] * n[1] + o.R[i * 3 + 2] * n[2];
-            for (int i = 0; i < 3; ++i) image[i] = x[i];
-        }
-        const double en = sqrt(e[0] * e[0] + e[1] * e[1] + e[2] * e[2]);
-        for (int i = 0; i < 3; ++i) nrm[i] = en > 0.0 ? e[i] / en : 0.0;
+        reflect_from_closest(o, x, cpo, tri, image, bp, nrm, dist);
         return;
     }
     if (o.shape == 0) {

@@ -33,6 +33,7 @@ struct HostObject {
 struct MeshHost {
     std::vector<MeshNode> nodes;
     std::vector<MeshTri> tris;  // leaf order
+    std::vector<int> top;       // MeshView::top
     std::vector<double> vertices;
 };
 bool build_mesh(const fdtd_mesh_desc& md, MeshHost& out, std::string& err);

@@ -39,7 +39,8 @@ cudaError_t launch_listeners(const SolveParams* dP, int precision, int newp, int
 // (3 launches; the last only when some box has cells).  With `prev` (the boxes
 // of the classification before, when every cell outside them is known to hold
 // the default flags) the first sweep visits only the units those reached.
-cudaError_t launch_classify(const SolveParams* dP, const int N[3], const ClsBoxes& B, bool collect_fresh,
+// `meshes`: some body is a triangle mesh (the solid test by warps).
+cudaError_t launch_classify(const SolveParams* dP, const int N[3], const ClsBoxes& B, bool collect_fresh, bool meshes,
                             cudaStream_t s, const ClsBoxes* prev = nullptr);
 cudaError_t launch_cls_history(const SolveParams* dP, long long ncell, int* count, int* list, int cap, cudaStream_t s);
 cudaError_t launch_fresh_cells(const SolveParams* dP, int precision, int cur, long long ncell, int* d_status,

@@ -190,6 +190,20 @@ bool build_mesh(const fdtd_mesh_desc& md, MeshHost& out, std::string& err) {
         return false;
     }
     out.nodes = B.nodes;
+    // the nodes five levels down, with the leaves above them
+    out.top.assign(1, 0);
+    for (int level = 0; level < 5; ++level) {
+        std::vector<int> next;
+        for (int n : out.top) {
+            if (out.nodes[n].count > 0) {
+                next.push_back(n);
+            } else {
+                next.push_back(out.nodes[n].first);
+                next.push_back(out.nodes[n].first + 1);
+            }
+        }
+        out.top.swap(next);
+    }
     out.tris.resize(nt);
     for (int k = 0; k < nt; ++k) out.tris[k] = tris[B.order[k]];
     out.vertices.assign(md.vertices, md.vertices + 3 * (size_t)nv);

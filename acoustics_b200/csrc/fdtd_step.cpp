@@ -33,7 +33,7 @@ void classification_launches(fdtd_solver* s, fdtd_status& st, const ClsBoxes* pr
     const ClsBoxes& B = s->hP.boxes;
     // pageable source: the copy is staged before the call returns
     cudaError_t e = fdtd::counted_copyAsync(s, &s->dP->boxes, &B, sizeof(ClsBoxes), cudaMemcpyHostToDevice, s->stream);
-    if (e == cudaSuccess) e = launch_classify(s->dP, s->N, B, s->moving, s->stream, prev);
+    if (e == cudaSuccess) e = launch_classify(s->dP, s->N, B, s->moving, !s->mesh_alloc.empty(), s->stream, prev);
     s->launches += B.ufirst[B.n] > 0 ? 3 : 2;
     if (e != cudaSuccess) {
         set_error(s, std::string("classification launch: ") + cudaGetErrorString(e));
