@@ -1287,6 +1287,7 @@ fdtd_status fdtd_solver_reset(fdtd_solver* s, double t0) {
     s->launches = 0;
     st = run_classification(s);
     if (st != FDTD_OK) return st;
+    s->lis_clear = listeners_clear_of(s, P.boxes);
     // ResetCellHistory(true): every cell has a valid history after reset (the
     // classification kernels keep it in bit 6; set it on all cells), and the
     // solid cells inside the PML, re-zeroed every step of a static scene

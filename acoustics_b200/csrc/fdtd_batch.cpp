@@ -54,6 +54,9 @@ struct fdtd_batch {
     cudaStream_t stream4 = nullptr;
     cudaEvent_t ev_step = nullptr, ev_lis[2] = {nullptr, nullptr}, ev_lis_join = nullptr;
     bool lis_pending[2] = {false, false};
+    // some member's listener stencil may hold a ghost cell, whose rows also read
+    // p^n in the buffer the next step writes: rows on the batch stream, before it
+    bool rows_inline = false;
     // the interior arguments in the kernel's parameter bank, one table per step
     // parity (BatchIntParams<T>); empty when more members have interior tiles
     // than the table holds (the tile table path then)
@@ -186,6 +189,7 @@ fdtd_status rebuild(fdtd_batch* b) {
     std::vector<IntEntry> int_list;
     std::vector<ListenerRef> refs;
     int max_ghost = 0, max_src = 0, max_solid = 0;
+    b->rows_inline = false;
     for (size_t m = 0; m < nm; ++m) {
         Member& mb = b->members[m];
         if (!mb.s) continue;
@@ -221,6 +225,7 @@ fdtd_status rebuild(fdtd_batch* b) {
                 for (int u = 0; u < B.tu[bx]; ++u) tab.push_back({(int)m, bx, u, 0, x});
         mb.tiles = (int64_t)(it.size() + st.size() + st_full.size() - tiles0);
         for (int li = 0; li < mb.s->L; ++li) refs.push_back({(int)m, li});
+        if (mb.s->L > 0 && !mb.s->lis_clear) b->rows_inline = true;
         max_ghost = std::max(max_ghost, (mb.s->region.ghost_cap + 127) / 128);
         max_solid = std::max(max_solid, (mb.s->n_solid_pml + 255) / 256);
         if (mb.s->hP.n_src > 0) {
@@ -297,7 +302,8 @@ fdtd_status enqueue(fdtd_batch* b) {
                         ? launch_batch_fp64(L, SS, &l)
                         : launch_batch_fp32(L, SS, &l);
     // listener rows of this step beside the next step
-    const bool rows = L.n_refs > 0;
+    const bool rows = L.n_refs > 0 && !b->rows_inline;
+    if (e == cudaSuccess && b->rows_inline && L.n_refs > 0) e = launch_batch_listeners_any(b->precision, L, b->stream, &l);
     if (e == cudaSuccess && rows) e = cudaEventRecord(b->ev_step, b->stream);
     if (e == cudaSuccess && rows) e = cudaStreamWaitEvent(b->stream4, b->ev_step, 0);
     if (e == cudaSuccess && rows) e = launch_batch_listeners_any(b->precision, L, b->stream4, &l);

@@ -76,6 +76,7 @@ struct fdtd_solver {
     // hP.boxes are the boxes of the classification the cell flags hold (the
     // solid cells lie in them); cleared when the flags are loaded from elsewhere
     bool cls_boxes_current = false;
+    bool lis_clear = false;         // listeners_clear_of the boxes of the last reset
     long long overlapped_steps = 0;
     // geometry
     double h = 0, c = 0, rho = 0, k = 0, end_time = 0, start_time = 0;
@@ -153,6 +154,8 @@ inline cudaError_t counted_copyAsync(fdtd_solver* s, void* dst, const void* src,
     return cudaMemcpyAsync(dst, src, n, kind, stream);
 }
 void set_error(fdtd_solver* s, const std::string& msg);
+// no listener stencil meets a classification box (fdtd_step.cpp)
+bool listeners_clear_of(const fdtd_solver* s, const ClsBoxes& B);
 // moving bodies two cells clear of the PML through [start_time, end_time]
 bool moving_clear_of_pml(fdtd_solver* s);
 // A batch member made outside the batch: its solver created and its first step

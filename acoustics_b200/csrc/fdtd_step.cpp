@@ -83,13 +83,12 @@ StepStreams step_streams(const fdtd_solver* s) {
     return StepStreams{s->stream, s->stream2, s->stream3, s->ev_fork, s->ev_join, s->ev_ghost};
 }
 
-// Listener rows of static scenes run on stream4 beside the next step.  Not for
-// moving bodies or solid cells inside the PML: the next step's classification /
-// prologue rewrites cells of the pressure they read.
 // True when no listener stencil (the cells its MLS may read, two cells around
 // them) meets a classification box: the classification of the next step writes
 // flags and pressures only inside its boxes, its fresh cells lie in the boxes of
 // this step.
+}  // namespace
+namespace fdtd {
 bool listeners_clear_of(const fdtd_solver* s, const ClsBoxes& B) {
     for (int l = 0; l < s->L; ++l) {
         int lo[3], hi[3];
@@ -108,16 +107,19 @@ bool listeners_clear_of(const fdtd_solver* s, const ClsBoxes& B) {
     }
     return true;
 }
+}  // namespace fdtd
+namespace {
 
-// The listener rows of a step run on stream4 beside the next step: static
-// scenes after their first step, moving scenes while every listener stencil is
-// clear of this step's classification boxes (the next step waits for them if
-// its own boxes reach a stencil).  Not with Engquist cells (the step after
-// writes the exterior cells of the pressure they read) or solids in the PML
-// (re-zeroed at the start of every step).
+// The listener rows of a step run on stream4 beside the next step while every
+// listener stencil is clear of this step's classification boxes (static scenes
+// after their first step; for moving bodies the next step waits for the rows if
+// its own boxes reach a stencil).  A stencil that holds a ghost cell is not: its
+// rows also read p^n beside the solid, in the buffer the next step writes.  Not
+// with Engquist cells either (the step after writes the exterior cells of the
+// pressure they read) or solids in the PML (re-zeroed at the start of every step).
 bool listeners_aside(const fdtd_solver* s, bool classify) {
     if (!s->stream4 || s->n_solid_pml != 0 || !s->eng.empty()) return false;
-    return s->moving ? listeners_clear_of(s, s->hP.boxes) : !classify;
+    return s->moving ? listeners_clear_of(s, s->hP.boxes) : (!classify && s->lis_clear);
 }
 
 // Make the solver stream wait for every listener launch on stream4.
