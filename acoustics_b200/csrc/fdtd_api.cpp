@@ -878,6 +878,11 @@ static void carve_arena(fdtd_solver* s, const fdtd_scene_desc* sc, const fdtd_op
         s->region.ghost_cap = (int)std::min<double>(cells, (double)n);
         cv.add((void**)&s->d_ghost_list, (size_t)s->region.ghost_cap * 4);
         cv.add((void**)&s->d_ghost_count, 16);
+        // plans of its cells: static scenes with rasterized ghost pressures
+        P.plan_cap = (s->moving || sc->boundary_handling != FDTD_BOUNDARY_RASTERIZE || o.kernel != FDTD_KERNEL_FUSED)
+                         ? 0
+                         : std::min(s->region.ghost_cap, GHOST_PLAN_MAX);
+        if (P.plan_cap > 0) cv.add((void**)&P.ghost_plan, (size_t)P.plan_cap * sizeof(GhostPlan));
         // fresh cells were solid the step before: fewer than the solid cells of the boxes
         P.fresh_cap = s->moving ? s->region.ghost_cap : 0;
         cv.add((void**)&P.fresh_list, (size_t)std::max(1, P.fresh_cap) * 4);
@@ -1280,7 +1285,10 @@ fdtd_status fdtd_solver_reset(fdtd_solver* s, double t0) {
     s->n_solid_pml = 0;
     P.solid_pml = nullptr;
     P.n_solid_pml = 0;
-    P.lis_ready = 0;  // the first step classifies and rebuilds the listener fits
+    P.lis_ready = 0;  // the first step classifies and rebuilds the listener fits and ghost plans
+    P.plan_ready = 0;
+    s->lag_row = nullptr;
+    s->n_ghost = -1;
     fdtd_status st = upload_params(s);
     if (st != FDTD_OK) return st;
     CUDA_TRY(s, launch_consts_init(s->dP, t0, s->stream));
@@ -1333,6 +1341,14 @@ fdtd_status fdtd_solver_reset(fdtd_solver* s, double t0) {
         if (s->shell.xs != xs) build_shell_boxes(s, xs);
         s->region.shell = s->shell;
     }
+    // the whole step in one launch: static scenes with a PML on every side, up to
+    // one_launch_cells() (fdtd_one_launch.cuh); explicit tile shapes or staging ask
+    // for the region-split kernels
+    s->region.one = (!s->moving && s->opt.kernel == FDTD_KERNEL_FUSED && s->eng.empty() && !s->region.fc &&
+                     s->n_solid_pml == 0 && P.plan_cap == P.ghost_cap && s->opt.tile_y == 0 && s->opt.x_chunk == 0 && s->opt.shell_staging == 0 &&
+                     s->ncell <= one_launch_cells(s->precision))
+                        ? 1
+                        : 0;
     st = upload_params(s);
     if (st != FDTD_OK) return st;
     CUDA_TRY(s, cudaStreamSynchronize(s->stream));

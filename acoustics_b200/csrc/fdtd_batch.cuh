@@ -224,7 +224,7 @@ cudaError_t launch_batch(const BatchLaunch& L, const StepStreams& S, int* launch
     return cudaGetLastError();
 }
 
-// Last kernel of a batched step, one thread per member: write the member's
+// Last kernel of a batched step, one warp per member: write the member's
 // constants of the next step (consts[cur ^ 1]) and, after its last step, mark
 // it halted, so its kernels leave at once from the next step on (the tables
 // alternate every step, a halted member's state no longer does).  The flag goes
@@ -236,17 +236,17 @@ cudaError_t launch_batch(const BatchLaunch& L, const StepStreams& S, int* launch
 template <typename T>
 __global__ void __launch_bounds__(128) k_batch_advance(BatchDesc<T>* __restrict__ D, BatchDesc<T>* __restrict__ D2,
                                                        int n) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= n) return;
+    const int m = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (m >= n) return;  // whole warps
     const BatchDesc<T>& d = D[m];
     if (!d.active) return;
     if (d.halted) {
-        D2[m].halted = 1;
+        if (lane == 0) D2[m].halted = 1;
         return;
     }
     const long long step = d.P->consts[d.cur].step;
-    advance_consts(*d.P, d.cur);
-    if (step + 1 >= d.total) D2[m].halted = 1;
+    advance_consts(*d.P, d.cur, lane);
+    if (lane == 0 && step + 1 >= d.total) D2[m].halted = 1;
 }
 
 // Listener rows of a batched step.  Instantiated in the FP64 translation unit
@@ -267,7 +267,7 @@ template <typename T>
 cudaError_t launch_batch_advance(const BatchLaunch& L, cudaStream_t s, int* launches) {
     BatchDesc<T>* D = static_cast<BatchDesc<T>*>(L.descs);
     if (L.n_members > 0) {
-        k_batch_advance<T><<<(L.n_members + 127) / 128, 128, 0, s>>>(D, static_cast<BatchDesc<T>*>(L.descs_other),
+        k_batch_advance<T><<<(L.n_members + 3) / 4, 128, 0, s>>>(D, static_cast<BatchDesc<T>*>(L.descs_other),
                                                                       L.n_members);
         if (launches) *launches += 1;
     }

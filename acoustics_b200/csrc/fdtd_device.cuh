@@ -194,6 +194,7 @@ struct RegionLaunch {
     int skip;          // kernels left out (timing of single kernels): 1 interior, 2 shell, 4 ghost list
     int red;           // FP32: the shell keeps the reduced PML state (k_pml_shell_red)
     int fc;            // FULLY_COUPLED ghost cells: solve their system before the ghost list
+    int one;           // the whole step in one launch (k_step_one)
     const TmaStep* tma;  // reduced state: the TMA-staged shell (k_pml_shell_tma) when not null (host memory)
 };
 
@@ -202,7 +203,38 @@ struct RegionLaunch {
 struct StepConsts {
     double t;                       // simulation time at the start of the step
     double src_tf[FDTD_MAX_SOURCES];  // exp(-((t+k/2 - t0)/wt)^2/2)
+    double obj_g[FDTD_MAX_OBJECTS];   // amp exp(-((t - t0)/tau)^2/2): the body's acceleration (boundary_accel)
     int64_t step;
+};
+
+// One cell of the ghost-neighbour list of a static scene with what its update
+// needs besides pressures and the step's factors: its flags, place, and per
+// direction f = 2 axis + (sign > 0) with a solid neighbour the body whose
+// acceleration moves that face (GHOST_STILL: none) and the component along the axis
+// of that acceleration per unit of obj_g.  The general path finds all this again
+// every step by a chain of dependent loads (list, flags, object, table entries)
+// with a division and an exponential per face.
+constexpr uint8_t GHOST_STILL = 0xFF;
+constexpr int GHOST_PLAN_MAX = 1 << 17;  // planned cells (10 MB); a longer list ends in the general path
+struct alignas(16) GhostPlan {
+    int c;
+    uint32_t code;       // the cell's flag byte
+    uint8_t obj[6], pad[2];
+    uint16_t ijk[3], pad1;
+    int pad2[2];
+    double u[3][2];      // by axis: toward -, toward +
+};
+static_assert(sizeof(GhostPlan) == 80, "loaded as 16-byte words");
+
+// The Gaussian sources as the kernels that add them to their own cells read
+// them (by value; the factors of source_term).
+struct SourceArgs {
+    Box3 region;              // bounding box of the supports, inside the interior kernel's box
+    int n;
+    int N[3];
+    const double* ax[3];
+    const StepConsts* consts; // of this step
+    double k;
 };
 
 // Iteration boxes of one classification (MAC_Grid::classifyCells_FAST,
@@ -308,6 +340,9 @@ struct SolveParams {
     int* ghost_list;              // non-PML bulk cells with a solid neighbour
     int* ghost_count;
     int ghost_cap;
+    GhostPlan* ghost_plan;        // [plan_cap] the list's cells prepared (static scenes)
+    int plan_cap;
+    int plan_ready;               // ghost_plan valid for the current classification
     ClsBoxes boxes;               // iteration boxes of the latest classification
     int* fresh_list;              // bulk cells without a valid history (found by the classification sweep)
     int* fresh_count;             // may exceed fresh_cap: the fresh-cell kernel then sweeps every cell
@@ -533,23 +568,40 @@ __device__ __forceinline__ double source_term(const SolveParams& P, int cur, int
     return src;
 }
 
+// Factors of a step into *n, by the lanes of one warp (a factor per lane: an
+// exponential and a division each, which one thread would take in turn): the
+// source time factors at ts = t + k/2 and the bodies' accelerations at t.
+__device__ __forceinline__ void step_factors(const SolveParams& P, StepConsts& n, double ts, double t, int lane) {
+    static_assert(FDTD_MAX_SOURCES + FDTD_MAX_OBJECTS <= 32, "one factor per lane");
+    if (lane < FDTD_MAX_SOURCES) {
+        double tf = 0.0;
+        if (lane < P.n_src) {
+            const double u = (ts - P.src[lane].t0) / P.src[lane].wt;
+            tf = exp(-(u * u) / 2.0);
+        }
+        n.src_tf[lane] = tf;
+    } else if (lane < FDTD_MAX_SOURCES + FDTD_MAX_OBJECTS) {
+        const int o = lane - FDTD_MAX_SOURCES;
+        double g = 0.0;
+        if (o < P.n_obj && P.obj[o].accel_kind != 0) {
+            const double u = (t - P.obj[o].t0) / P.obj[o].tau;
+            g = P.obj[o].amp * exp(-(u * u) / 2.0);  // as boundary_accel
+        }
+        n.obj_g[o] = g;
+    }
+}
+
 // consts[cur^1] <- the next step's constants (PML_WaveSolver.cpp:825,
-// _currentTime += _timeStep; source time factors at t + k/2).
-__device__ inline void advance_consts(const SolveParams& P, int cur) {
+// _currentTime += _timeStep); called by one warp.
+__device__ __forceinline__ void advance_consts(const SolveParams& P, int cur, int lane) {
     const StepConsts& c = P.consts[cur];
     StepConsts& n = P.consts[cur ^ 1];
     const double t = c.t + P.k;
-    n.t = t;
-    const double ts = t + 0.5 * P.k;
-    for (int s = 0; s < FDTD_MAX_SOURCES; ++s) {
-        double tf = 0.0;
-        if (s < P.n_src) {
-            const double u = (ts - P.src[s].t0) / P.src[s].wt;
-            tf = exp(-(u * u) / 2.0);
-        }
-        n.src_tf[s] = tf;
+    step_factors(P, n, t + 0.5 * P.k, t, lane);
+    if (lane == 31) {
+        n.t = t;
+        n.step = c.step + 1;
     }
-    n.step = c.step + 1;
 }
 
 // Szudzik pairing of two cell indices (MAC_Grid.h:108-116)

@@ -27,6 +27,14 @@ cudaError_t launch_step_regions_fp32(const SolveParams* dP, const SolveParams& h
 }
 }  // namespace fdtd
 
+#include "fdtd_one_launch.cuh"
+namespace fdtd {
+cudaError_t launch_one_fp32(const SolveParams* dP, const SolveParams& hP, const RegionLaunch& R, int cur, bool src,
+                            int n_ghost, double* lis_row, cudaStream_t s) {
+    return launch_one<float>(dP, hP, R, cur, src, n_ghost, lis_row, s);
+}
+}  // namespace fdtd
+
 #include "fdtd_batch.cuh"
 namespace fdtd {
 // The reduced-state shell kernels stage their loads in more than the default

@@ -13,6 +13,7 @@
 #include "fdtd_geometry.cuh"
 #include "fdtd_launch.hpp"
 #include "fdtd_listeners.cuh"
+#include "fdtd_region.cuh"
 #include "fdtd_stencil.cuh"
 
 namespace fdtd {
@@ -1047,15 +1048,18 @@ cudaError_t launch_listeners(const SolveParams* dP, int precision, int newp, int
     return cudaGetLastError();
 }
 
-// listener fit plans from the current classification (static scenes, once)
-__global__ void k_set_lis_ready(SolveParams* __restrict__ Pp) { Pp->lis_ready = 1; }
+// listener fits and ghost-cell plans from the current classification (static scenes, once)
+__global__ void k_set_ready(SolveParams* __restrict__ Pp, int plan) {
+    Pp->lis_ready = 1;
+    Pp->plan_ready = plan;
+}
 
-cudaError_t launch_listener_prep(SolveParams* dP, int precision, int newp, int n_lis, cudaStream_t s) {
-    if (n_lis <= 0) return cudaSuccess;
+cudaError_t launch_static_prep(SolveParams* dP, int precision, int newp, int n_lis, int plan_cap, cudaStream_t s) {
     const int grid = (n_lis + 3) / 4;
-    if (precision == 0) k_listener_prep<double><<<grid, 128, 0, s>>>(dP, newp);
-    else k_listener_prep<float><<<grid, 128, 0, s>>>(dP, newp);
-    k_set_lis_ready<<<1, 1, 0, s>>>(dP);
+    if (grid > 0 && precision == 0) k_listener_prep<double><<<grid, 128, 0, s>>>(dP, newp);
+    if (grid > 0 && precision != 0) k_listener_prep<float><<<grid, 128, 0, s>>>(dP, newp);
+    if (plan_cap > 0) k_ghost_prep<<<grid_for(plan_cap, 128), 128, 0, s>>>(dP);
+    k_set_ready<<<1, 1, 0, s>>>(dP, plan_cap > 0);
     return cudaGetLastError();
 }
 
@@ -1140,6 +1144,15 @@ cudaError_t launch_step_regions_fp64(const SolveParams* dP, const SolveParams& h
                                      const StepStreams& S, int* launches) {
     return launch_regions<double>(dP, hP, R, cur, S, launches);
 }
+}  // namespace fdtd
+
+#include "fdtd_one_launch.cuh"
+namespace fdtd {
+cudaError_t launch_one_fp64(const SolveParams* dP, const SolveParams& hP, const RegionLaunch& R, int cur, bool src,
+                            int n_ghost, double* lis_row, cudaStream_t s) {
+    return launch_one<double>(dP, hP, R, cur, src, n_ghost, lis_row, s);
+}
+long long one_launch_cells(int precision) { return precision == 0 ? FDTD_ONE_LAUNCH_CELLS_F64 : FDTD_ONE_LAUNCH_CELLS_F32; }
 }  // namespace fdtd
 
 // ---------------------------------------------------------------------------

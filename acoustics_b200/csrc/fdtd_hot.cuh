@@ -67,6 +67,10 @@ __device__ __forceinline__ void stv(T* p, const Vec<T, V>& v) {
     *reinterpret_cast<Vec<T, V>*>(p) = v;
 }
 
+// Of a kernel launched as a programmatic dependent of the step before: what
+// follows sees that step's results.  (Everything before it may run beside that step.)
+__device__ __forceinline__ void step_before_done() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // One interior tile: 256 consecutive (row, z-group) units of the box (one per
 // thread; a z group is a 16-byte vector of V = 4 FP32 / 2 FP64 cells starting
 // at a multiple of V) x XB x planes, at unit tile tu and plane tile tx.  Units
@@ -76,8 +80,12 @@ __device__ __forceinline__ void stv(T* p, const Vec<T, V>& v) {
 // shuffle when that lane holds the neighbouring group of the same row, else
 // from memory.  Cells of a group outside the box or not plain bulk are masked
 // (scalar stores for partial groups).  Every thread of the CTA must call it.
-template <typename T, int XB, bool VISC = false, typename AT = KArgs<T>>
-__device__ __forceinline__ void interior_tile(const AT& A, const Box3& box, int tu, int tx) {
+// SRC (the one-launch step): the sources of S are added to the tile's cells here
+// instead of by k_sources afterwards (the same sums in the same order), and what
+// the step before makes is read after step_before_done().
+template <typename T, int XB, bool VISC = false, typename AT = KArgs<T>, bool SRC = false>
+__device__ __forceinline__ void interior_tile(const AT& A, const Box3& box, int tu, int tx,
+                                              const SourceArgs* S = nullptr) {
     constexpr bool COMP = sizeof(T) == 4;
     constexpr int V = 16 / (int)sizeof(T);
     using VT = Vec16<T>;
@@ -109,6 +117,31 @@ __device__ __forceinline__ void interior_tile(const AT& A, const Box3& box, int 
 
     VT pcol[XB + 2], ym[XB], yp[XB], prev[XB], lapl[XB];
     uint32_t code[XB];
+    auto load_code = [&](int i) {
+        if constexpr (V == 4) code[i] = *reinterpret_cast<const uint32_t*>(cls + i * sx);
+        else code[i] = *reinterpret_cast<const uint16_t*>(cls + i * sx);
+    };
+    // the row's cells may lie in a source's support: their spatial factors
+    // (zero outside it) where there is one source, read with the flags
+    bool src_row = false;
+    double src_xy[XB], src_z[V], src_tf = 0.0;
+    if constexpr (SRC) {
+        // the flags and factors of a static scene are no results of the step before
+#pragma unroll
+        for (int i = 0; i < XB; ++i)
+            if (i < nx) load_code(i);
+        src_row = S->n > 0 && x0 < S->region.hi[0] && x0 + XB > S->region.lo[0] && yc >= S->region.lo[1] &&
+                  yc < S->region.hi[1] && zc < S->region.hi[2] && zc + V > S->region.lo[2];
+        if (src_row && S->n == 1) {
+            const double fy = S->ax[1][yc];
+#pragma unroll
+            for (int i = 0; i < XB; ++i) src_xy[i] = i < nx ? S->ax[0][x0 + i] * fy : 0.0;
+#pragma unroll
+            for (int e = 0; e < V; ++e) src_z[e] = zc + e < S->N[2] ? S->ax[2][zc + e] : 0.0;
+        }
+        step_before_done();
+        if (src_row && S->n == 1) src_tf = S->consts->src_tf[0];
+    }
     T zme[XB], zpe[XB];
     pcol[0] = ldv(pc - sx);
 #pragma unroll
@@ -126,8 +159,7 @@ __device__ __forceinline__ void interior_tile(const AT& A, const Box3& box, int 
             } else {
                 prev[i] = ldv(pn + i * sx);
             }
-            if constexpr (V == 4) code[i] = *reinterpret_cast<const uint32_t*>(cls + i * sx);
-            else code[i] = *reinterpret_cast<const uint16_t*>(cls + i * sx);
+            if constexpr (!SRC) load_code(i);
             if constexpr (VISC) lapl[i] = ldv(A.lapl + off + i * sx);
             zme[i] = zm_mem ? pc[i * sx - 1] : (T)0;
             zpe[i] = zp_mem ? pc[i * sx + V] : (T)0;
@@ -170,6 +202,23 @@ __device__ __forceinline__ void interior_tile(const AT& A, const Box3& box, int 
                 outp.e[e] = p0 + d;
             }
             outl.e[e] = lap;
+        }
+        if constexpr (SRC) {
+            // cells outside the support, and sources that are off, add zero
+            if (src_row && (S->n > 1 || src_tf != 0.0)) {
+#pragma unroll
+                for (int e = 0; e < V; ++e) {
+                    const double src = S->n == 1 ? (src_xy[i] * src_z[e]) * src_tf
+                                       : ((act >> e) & 1u) ? source_at(*S, x0 + i, yc, zc + e) : 0.0;
+                    const double add = src * S->k;
+                    if constexpr (!COMP) {
+                        outp.e[e] += add;
+                    } else {
+                        outd.e[e] = outd.e[e] + (float)add;
+                        outp.e[e] = c0.e[e] + outd.e[e];
+                    }
+                }
+            }
         }
         if (act == (1u << V) - 1u) {
             stv(pn + i * sx, outp);
@@ -578,7 +627,7 @@ __device__ __forceinline__ void shell_decode(const ShellBoxes& B, int blk, int& 
 
 template <typename T>
 __global__ void __launch_bounds__(256, shell_min_blocks(sizeof(T))) k_pml_shell(const KArgs<T> A, const ShellBoxes B) {
-    if (A.advance && blockIdx.x == 0 && threadIdx.x == 0 && threadIdx.y == 0) advance_consts(*A.P, A.cur);
+    if (A.advance && blockIdx.x == 0 && threadIdx.y == 0) advance_consts(*A.P, A.cur, threadIdx.x);
     int b, tu, tx;
     shell_decode(B, blockIdx.x, b, tu, tx);
     shell_tile<T>(A, B, b, tu, tx);

@@ -118,6 +118,10 @@ struct fdtd_solver {
     fdtd::Box3 interior{};            // non-PML box
     fdtd::ShellBoxes shell{};         // PML shell boxes
     fdtd::RegionLaunch region{};      // launch description of the region-split step
+    // one-launch steps: the listener row of the last step, written by the next
+    // step's launch (or by flush_lag), and the cells of the ghost list once known
+    double* lag_row = nullptr;
+    int n_ghost = -1;
     int* d_ghost_list = nullptr;
     int* d_ghost_count = nullptr;
     // stepping state

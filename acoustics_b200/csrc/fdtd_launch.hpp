@@ -21,6 +21,16 @@ cudaError_t launch_step_regions_fp64(const SolveParams* dP, const SolveParams& h
 cudaError_t launch_step_regions_fp32(const SolveParams* dP, const SolveParams& hP, const RegionLaunch& R, int cur,
                                      const StepStreams& S, int* launches);
 
+// a static solve's step in one launch (fdtd_one_launch.cuh): n_ghost cells of the
+// ghost-neighbour list (< 0: not known on the host), the listener row of the step
+// before to lis_row (null: none)
+cudaError_t launch_one_fp64(const SolveParams* dP, const SolveParams& hP, const RegionLaunch& R, int cur, bool src,
+                            int n_ghost, double* lis_row, cudaStream_t s);
+cudaError_t launch_one_fp32(const SolveParams* dP, const SolveParams& hP, const RegionLaunch& R, int cur, bool src,
+                            int n_ghost, double* lis_row, cudaStream_t s);
+// grid cells up to which a static solve steps that way
+long long one_launch_cells(int precision);
+
 // batched step of many members (fdtd_batch.cuh)
 cudaError_t launch_batch_fp64(const BatchLaunch& L, const StepStreams& S, int* launches);
 cudaError_t launch_batch_fp32(const BatchLaunch& L, const StepStreams& S, int* launches);
@@ -30,7 +40,8 @@ cudaError_t launch_batch_advance_any(int precision, const BatchLaunch& L, cudaSt
 
 // fdtd_fp64.cu (compiled with -fmad=false)
 cudaError_t launch_prologue_fp64(const SolveParams* dP, int cur, int advance, int n_solid_pml, cudaStream_t s);
-cudaError_t launch_listener_prep(SolveParams* dP, int precision, int newp, int n_lis, cudaStream_t s);
+// listener fits and ghost-cell plans of a static scene's classification (once)
+cudaError_t launch_static_prep(SolveParams* dP, int precision, int newp, int n_lis, int plan_cap, cudaStream_t s);
 cudaError_t launch_consts_init(const SolveParams* dP, double t0, cudaStream_t s);
 cudaError_t launch_listeners(const SolveParams* dP, int precision, int newp, int n_lis, double* out_row,
                              cudaStream_t s);

@@ -71,47 +71,236 @@ __device__ __noinline__ T ghost_laplacian(const SolveParams& P, long long c, con
     return lap;
 }
 
-// Full update of one non-PML bulk cell next to a solid (ghost-aware Laplacian,
+// Full update of non-PML bulk cell c next to a solid (ghost-aware Laplacian,
 // cavity freeze), everything re-read from memory.  Sources are added by
 // k_sources afterwards, as the reference adds them after the update
 // (MAC_Grid.cpp:938-944).
 template <typename T>
-__device__ __forceinline__ void ghost_cells_body(const SolveParams& P, int cur, int bid, int nblocks) {
-    const int n = *P.ghost_count;
+__device__ __forceinline__ void ghost_cell(const SolveParams& P, int cur, long long c) {
     const long long sx = P.SX, sy = P.SY;
     const T* __restrict__ pc = (const T*)P.p[cur];
     T* __restrict__ pn = (T*)P.p[cur ^ 1];
     const double t = P.consts[cur].t;
-    for (int g = bid * blockDim.x + threadIdx.x; g < n && g < P.ghost_cap; g += nblocks * blockDim.x) {
-        const long long c = P.ghost_list[g];
-        int x, y, z;
-        cell_ijk(P, c, x, y, z);
-        const uint8_t code = P.cls[c];
-        const T p0 = pc[c];
-        const T nbp[3] = {pc[c + sx], pc[c + sy], pc[c + 1]};
-        const T nbm[3] = {pc[c - sx], pc[c - sy], pc[c - 1]};
-        const int idx[3] = {x, y, z};
-        int surrounded = 0;
-        T lap = ghost_laplacian<T>(P, c, idx, code & CLS_MASK, p0, nbp, nbm, t, cur, &surrounded);
-        lap = lap * (T)P.lap_scale;
-        const bool cavity = (surrounded > 1) && (code & CLS_VALID);
-        // air viscosity on cells with a valid history (MAC_Grid.cpp:926-930)
-        const bool visc = P.visc && (code & CLS_VALID);
-        T lapl = 0;
-        if (P.visc) {
-            lapl = ((const T*)P.lapv[cur ^ 1])[c];
-            ((T*)P.lapv[cur])[c] = lap;
+    int x, y, z;
+    cell_ijk(P, c, x, y, z);
+    const uint8_t code = P.cls[c];
+    const T p0 = pc[c];
+    const T nbp[3] = {pc[c + sx], pc[c + sy], pc[c + 1]};
+    const T nbm[3] = {pc[c - sx], pc[c - sy], pc[c - 1]};
+    const int idx[3] = {x, y, z};
+    int surrounded = 0;
+    T lap = ghost_laplacian<T>(P, c, idx, code & CLS_MASK, p0, nbp, nbm, t, cur, &surrounded);
+    lap = lap * (T)P.lap_scale;
+    const bool cavity = (surrounded > 1) && (code & CLS_VALID);
+    // air viscosity on cells with a valid history (MAC_Grid.cpp:926-930)
+    const bool visc = P.visc && (code & CLS_VALID);
+    T lapl = 0;
+    if (P.visc) {
+        lapl = ((const T*)P.lapv[cur ^ 1])[c];
+        ((T*)P.lapv[cur])[c] = lap;
+    }
+    if constexpr (sizeof(T) == 8) {
+        if (cavity) pn[c] = p0;
+        else if (visc) pn[c] = (T)2.0 * p0 - pn[c] - lapl * (T)P.kcalp + lap * (T)(P.c2k2 + P.kcalp);
+        else pn[c] = (T)2.0 * p0 - pn[c] + lap * (T)P.c2k2;
+    } else {
+        float d = cavity ? 0.0f : P.dinc[c] + (float)(lap * (T)P.c2k2);
+        if (!cavity && visc) d = fmaf((float)P.kcalp, (float)(lap - lapl), d);
+        P.dinc[c] = d;
+        pn[c] = p0 + d;
+    }
+}
+
+// Pointers and scalars of the planned update, by value or read from the
+// solve's parameters once.
+template <typename T>
+struct GhostArgs {
+    const T* pc;
+    T* pn;
+    float* dinc;
+    const T* lapl;  // air viscosity, else null
+    T* lapc;
+    unsigned sx, sy;
+    T c2k2, lap_scale, kcalp;
+    double h75, rho;              // 0.75 h, rho
+    const StepConsts* consts;     // of this step
+};
+
+template <typename T>
+__device__ __forceinline__ GhostArgs<T> ghost_args(const SolveParams& P, int cur) {
+    return GhostArgs<T>{(const T*)P.p[cur], (T*)P.p[cur ^ 1], P.dinc, P.visc ? (const T*)P.lapv[cur ^ 1] : nullptr,
+                        (T*)P.lapv[cur], (unsigned)P.SX, (unsigned)P.SY, (T)P.c2k2, (T)P.lap_scale, (T)P.kcalp,
+                        0.75 * P.h, P.rho, P.consts + cur};
+}
+
+// ghost_cell from the cells' plans, four lanes a cell: an axis of the Laplacian
+// each (its two faces and its division) and, in the last, what the cell keeps of
+// p^{n-1} and the sources.  One lane alone would take the axes' divisions in turn
+// at the end of every small step.  The terms are summed in axis order, and every
+// expression is ghost_cell's (boundary_accel, ghost_pressure, ghost_laplacian), so
+// the bits are the same.
+struct GhostLoad {
+    uint4 h0, h1;  // words 0-7 of the plan
+    double2 u;     // this lane's axis
+};
+__device__ __forceinline__ GhostLoad ghost_load(const GhostPlan* plan, int g, int q) {
+    const uint4* w = reinterpret_cast<const uint4*>(plan + g);
+    GhostLoad r;
+    r.h0 = w[0];
+    r.h1 = w[1];
+    r.u = *reinterpret_cast<const double2*>(&w[2 + (q < 3 ? q : 0)]);
+    return r;
+}
+
+// sum_s G_s(x, t + k/2) at cell (x, y, z), as source_term (the factors' loads do
+// not wait for the time factor)
+__device__ __forceinline__ double source_at(const SourceArgs& S, int x, int y, int z) {
+    double src = 0.0;
+    for (int s = 0; s < S.n; ++s) {
+        const double f = (S.ax[0][s * S.N[0] + x] * S.ax[1][s * S.N[1] + y]) * S.ax[2][s * S.N[2] + z];
+        const double tf = S.consts->src_tf[s];
+        if (tf != 0.0) src += f * tf;
+    }
+    return src;
+}
+
+// Called by whole warps; lanes with on = false work on some plan and store nothing.
+// S: the sources to add (null: k_sources does).
+template <typename T>
+__device__ __forceinline__ void ghost_cell_planned(const GhostArgs<T>& A, const GhostLoad& G, bool on,
+                                                   const SourceArgs* S) {
+    const int q = threadIdx.x & 3;
+    const unsigned c = G.h0.x;
+    const uint32_t code = G.h0.y;
+    const T* __restrict__ pc = A.pc + c;
+    const unsigned st = q == 0 ? A.sx : q == 1 ? A.sy : 1u;
+    const T p0 = pc[0];
+    // lanes 0-2: the neighbours along the axis; lane 3: p^{n-1} or the increment, the last Laplacian
+    const T pp = q < 3 ? pc[st] : sizeof(T) == 8 ? A.pn[c] : (T)A.dinc[c];
+    const T pm = q < 3 ? *(pc - st) : A.lapl ? A.lapl[c] : (T)0;
+    const bool gn = q < 3 && ((code >> (2 * q)) & 1u), gp = q < 3 && ((code >> (2 * q + 1)) & 1u);
+    // bodies of the axis' two faces: bytes 8-13 of the plan
+    const uint32_t bodies = q == 0 ? G.h0.z : q == 1 ? G.h0.z >> 16 : G.h0.w;
+    const unsigned on_n = bodies & 0xFFu, on_p = (bodies >> 8) & 0xFFu;
+    const double gt_n = gn && on_n != GHOST_STILL ? A.consts->obj_g[on_n] : 0.0;
+    const double gt_p = gp && on_p != GHOST_STILL ? A.consts->obj_g[on_p] : 0.0;
+    double add = 0.0;
+    bool add_src = false;
+    if (S && S->n > 0 && q == 3) {
+        const int x = (int)(G.h1.x & 0xFFFFu), y = (int)(G.h1.x >> 16), z = (int)(G.h1.y & 0xFFFFu);
+        const Box3& r = S->region;
+        add_src = x >= r.lo[0] && x < r.hi[0] && y >= r.lo[1] && y < r.hi[1] && z >= r.lo[2] && z < r.hi[2];
+        if (add_src) add = source_at(*S, x, y, z) * S->k;
+    }
+    double vn = (double)p0, vp = (double)p0;
+    if (gn && on_n != GHOST_STILL) vn = vn - A.h75 * (G.u.x * gt_n * (-A.rho));
+    // the face toward + has its normal toward this cell, along -
+    if (gp && on_p != GHOST_STILL) vp = vp - A.h75 * (G.u.y * gt_p * (-A.rho) * -1.0);
+    const T pgn = (T)vn, pgp = (T)vp;
+    T num, den;
+    if (gp && gn) {
+        num = pgp + pgn - (T)2.0 * p0;
+        den = (T)(9.0 / 16.0);
+    } else if (gp) {
+        num = pgp + (T)0.75 * pm - (T)(7.0 / 4.0) * p0;
+        den = (T)(21.0 / 32.0);
+    } else if (gn) {
+        num = (T)0.75 * pp + pgn - (T)(7.0 / 4.0) * p0;
+        den = (T)(21.0 / 32.0);
+    } else {
+        num = pp + pm - (T)2.0 * p0;
+        den = (T)1.0;
+    }
+    const T term = gp || gn ? num / den : num;
+    const unsigned both = __ballot_sync(0xffffffffu, gp && gn);
+    const int base = threadIdx.x & 28;
+    T lap = 0.0;
+    lap = lap + __shfl_sync(0xffffffffu, term, base);
+    lap = lap + __shfl_sync(0xffffffffu, term, base + 1);
+    lap = lap + __shfl_sync(0xffffffffu, term, base + 2);
+    if (q != 3 || !on) return;
+    const T prev = pp, lapl = pm;
+    lap = lap * A.lap_scale;
+    const bool valid = code & CLS_VALID;
+    const bool cavity = __popc((both >> base) & 7u) > 1 && valid;
+    const bool visc = A.lapl && valid;
+    if (A.lapl) A.lapc[c] = lap;
+    if constexpr (sizeof(T) == 8) {
+        T v;
+        if (cavity) v = p0;
+        else if (visc) v = (T)2.0 * p0 - prev - lapl * A.kcalp + lap * (A.c2k2 + A.kcalp);
+        else v = (T)2.0 * p0 - prev + lap * A.c2k2;
+        if (add_src) v += add;
+        A.pn[c] = v;
+    } else {
+        float d = cavity ? 0.0f : prev + (float)(lap * A.c2k2);
+        if (!cavity && visc) d = fmaf((float)A.kcalp, (float)(lap - lapl), d);
+        if (add_src) d = d + (float)add;
+        A.dinc[c] = d;
+        A.pn[c] = p0 + d;
+    }
+}
+
+// The cells of the ghost-neighbour list, by plan where there is one.
+template <typename T>
+__device__ __forceinline__ void ghost_cells_body(const SolveParams& P, int cur, int bid, int nblocks) {
+    const int n = min(*P.ghost_count, P.ghost_cap);
+    const int planned = P.plan_ready ? min(n, P.plan_cap) : 0;
+    const int first = bid * blockDim.x + threadIdx.x, stride = nblocks * blockDim.x;
+    if (planned > 0) {
+        const GhostArgs<T> A = ghost_args<T>(P, cur);
+        // whole warps, eight cells each
+        for (int w = first & ~31; w < 4 * planned; w += stride) {
+            const int g = (w + (int)(threadIdx.x & 31)) >> 2;
+            ghost_cell_planned<T>(A, ghost_load(P.ghost_plan, min(g, planned - 1), threadIdx.x & 3), g < planned,
+                                  nullptr);
         }
-        if constexpr (sizeof(T) == 8) {
-            if (cavity) pn[c] = p0;
-            else if (visc) pn[c] = (T)2.0 * p0 - pn[c] - lapl * (T)P.kcalp + lap * (T)(P.c2k2 + P.kcalp);
-            else pn[c] = (T)2.0 * p0 - pn[c] + lap * (T)P.c2k2;
-        } else {
-            float d = cavity ? 0.0f : P.dinc[c] + (float)(lap * (T)P.c2k2);
-            if (!cavity && visc) d = fmaf((float)P.kcalp, (float)(lap - lapl), d);
-            P.dinc[c] = d;
-            pn[c] = p0 + d;
+    }
+    for (int g = planned + first; g < n; g += stride) ghost_cell<T>(P, cur, P.ghost_list[g]);
+}
+
+// Plans of the ghost-neighbour list of the current classification (static scenes).
+static __global__ void __launch_bounds__(128) k_ghost_prep(const SolveParams* __restrict__ Pp) {
+    const SolveParams& P = *Pp;
+    const int n = min(min(*P.ghost_count, P.ghost_cap), P.plan_cap);
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+        GhostPlan G;
+        G.c = P.ghost_list[q];
+        int idx[3];
+        cell_ijk(P, G.c, idx[0], idx[1], idx[2]);
+        G.code = P.cls[G.c];
+        G.pad[0] = G.pad[1] = 0;
+        G.pad1 = 0;
+        G.pad2[0] = G.pad2[1] = 0;
+        const long long strides[3] = {P.SX, P.SY, 1};
+        for (int d = 0; d < 3; ++d) {
+            G.ijk[d] = (uint16_t)idx[d];
+            for (int s = 0; s < 2; ++s) {
+                const int f = 2 * d + s;
+                G.obj[f] = GHOST_STILL;
+                G.u[d][s] = 0.0;
+                if (!((G.code >> f) & 1u)) continue;
+                const int sgn = s ? 1 : -1;
+                const unsigned gobj = P.gobj[G.c + sgn * strides[d]];
+                const unsigned o = gobj & 0x7F;
+                if ((gobj & GOBJ_CONSTRAINT) || o >= (unsigned)P.n_obj || P.obj[o].accel_kind == 0) continue;
+                // the face a quarter cell from the solid cell's centre (ghost_pressure)
+                double pos[3] = {P.cpos[0][idx[0]], P.cpos[1][idx[1]], P.cpos[2][idx[2]]};
+                pos[d] = P.cpos[d][idx[d] + sgn];
+                pos[d] += (sgn > 0 ? -1.0 : 1.0) * 0.25 * P.h;
+                const DevObject& O = P.obj[o];
+                if (O.accel_kind == 1) {
+                    G.u[d][s] = O.dir[d];
+                } else {
+                    const double r0 = pos[0] - O.c[0], r1 = pos[1] - O.c[1], r2 = pos[2] - O.c[2];
+                    const double len = sqrt(r0 * r0 + r1 * r1 + r2 * r2);
+                    const double r[3] = {r0, r1, r2};
+                    G.u[d][s] = len > 0.0 ? r[d] / len : 0.0;
+                }
+                G.obj[f] = (uint8_t)o;
+            }
         }
+        P.ghost_plan[q] = G;
     }
 }
 

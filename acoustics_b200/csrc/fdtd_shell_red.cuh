@@ -413,7 +413,7 @@ __device__ __forceinline__ void shell_tile_red(const KArgs<float>& A, const Shel
 template <typename T>
 __global__ void __launch_bounds__(256, FDTD_SHELL_RED_MINB) k_pml_shell_red(const KArgs<T> A, const ShellBoxes B) {
     static_assert(sizeof(T) == 4, "the reduced PML state is an FP32 path");
-    if (A.advance && blockIdx.x == 0 && threadIdx.x == 0 && threadIdx.y == 0) advance_consts(*A.P, A.cur);
+    if (A.advance && blockIdx.x == 0 && threadIdx.y == 0) advance_consts(*A.P, A.cur, threadIdx.x);
     int b, tu, tx;
     shell_decode(B, blockIdx.x, b, tu, tx);
     shell_tile_red(A, B, b, tu, tx);

@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(TMA_BLOCK, 3)
     extern __shared__ __align__(128) unsigned char tma_ring[];
     uint64_t* full = reinterpret_cast<uint64_t*>(tma_ring + TMA_STAGES * Lc.stage_bytes);
     uint64_t* empty = full + TMA_STAGES;
-    if (A.advance && blockIdx.x == 0 && threadIdx.x == 0) advance_consts(*A.P, A.cur);
+    if (A.advance && blockIdx.x == 0 && threadIdx.x < 32) advance_consts(*A.P, A.cur, threadIdx.x);
     const int tid = threadIdx.x;
     const uint32_t ring = smem_u32(tma_ring);
     // tensor copies land on 128-byte boundaries (every buffer size is a multiple of 128)

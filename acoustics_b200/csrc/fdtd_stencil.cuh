@@ -90,7 +90,7 @@ static __device__ __noinline__ double source_sum(const SolveParams& P, const Ste
 template <typename T>
 __global__ void k_prologue(const SolveParams* __restrict__ Pp, int cur, int advance) {
     const SolveParams& P = *Pp;
-    if (advance && blockIdx.x == 0 && threadIdx.x == 0) advance_consts(P, cur);
+    if (advance && blockIdx.x == 0 && threadIdx.x < 32) advance_consts(P, cur, threadIdx.x);
     T* p0 = (T*)P.p[0];
     T* p1 = (T*)P.p[1];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < P.n_solid_pml; i += gridDim.x * blockDim.x) {
@@ -104,10 +104,12 @@ __global__ void k_prologue(const SolveParams* __restrict__ Pp, int cur, int adva
 // consts[0] <- the constants of the first step at time t0.
 static __global__ void k_consts_init(const SolveParams* __restrict__ Pp, double t0) {
     const SolveParams& P = *Pp;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (blockIdx.x != 0 || threadIdx.x >= 32) return;
+    const double t = (t0 - P.k) + P.k;  // the sources' clock advances to the first step
+    step_factors(P, P.consts[0], t + 0.5 * P.k, t0, threadIdx.x);
+    if (threadIdx.x == 31) {
         P.consts[1].t = t0 - P.k;
         P.consts[1].step = -1;
-        advance_consts(P, 1);
         P.consts[0].t = t0;
         P.consts[0].step = 0;
     }

@@ -131,6 +131,26 @@ fdtd_status join_listeners(fdtd_solver* s) {
     return FDTD_OK;
 }
 
+// The row a one-launch step left to its successor; newp: the parity of the
+// current pressure.
+fdtd_status flush_lag(fdtd_solver* s, int newp) {
+    if (!s->lag_row) return FDTD_OK;
+    CUDA_TRY(s, launch_listeners(s->dP, s->precision, newp, s->L, s->lag_row, s->stream));
+    s->launches++;
+    s->lag_row = nullptr;
+    return FDTD_OK;
+}
+
+// Listener fits and ghost-cell plans of a static scene's classification.
+fdtd_status static_prep(fdtd_solver* s, int newp) {
+    CUDA_TRY(s, launch_static_prep(s->dP, s->precision, newp, s->L, s->hP.plan_cap, s->stream));
+    s->launches += 1 + (s->L > 0) + (s->hP.plan_cap > 0);
+    // host mirrors of the flags the prep sets (later uploads keep them)
+    s->hP.lis_ready = 1;
+    s->hP.plan_ready = s->hP.plan_cap > 0;
+    return FDTD_OK;
+}
+
 // Enqueue one time step with the pressure parity `cur`; listener row to dev_row.
 fdtd_status enqueue_step(fdtd_solver* s, int cur, double* dev_row, bool classify, bool src) {
     s->region.sources = src ? 1 : 0;
@@ -197,12 +217,29 @@ fdtd_status enqueue_step(fdtd_solver* s, int cur, double* dev_row, bool classify
                                                     s->stream));
             }
         }
-        if (!s->moving && s->L > 0) {
-            // static classification: the listener fits become fixed weights
-            CUDA_TRY(s, launch_listener_prep(s->dP, s->precision, cur ^ 1, s->L, s->stream));
-            s->launches += 2;
-            s->hP.lis_ready = 1;  // host mirror of the flag the prep sets (later uploads keep it)
+        if (!s->moving) {
+            // static classification: the listener fits become fixed weights, the
+            // ghost list's cells plans
+            const fdtd_status pst = static_prep(s, cur ^ 1);
+            if (pst != FDTD_OK) return pst;
         }
+    }
+    if (s->region.one) {
+        cudaError_t e = s->precision == FDTD_PRECISION_FP64
+                            ? launch_one_fp64(s->dP, s->hP, s->region, cur, src, s->n_ghost, s->lag_row, s->stream)
+                            : launch_one_fp32(s->dP, s->hP, s->region, cur, src, s->n_ghost, s->lag_row, s->stream);
+        CUDA_TRY(s, e);
+        s->launches++;
+        s->lag_row = nullptr;
+        if (s->L > 0 && dev_row) {
+            if (s->lis_clear) {
+                s->lag_row = dev_row;  // by the next step's launch, or flush_lag
+            } else {
+                CUDA_TRY(s, launch_listeners(s->dP, s->precision, cur ^ 1, s->L, dev_row, s->stream));
+                s->launches++;
+            }
+        }
+        return FDTD_OK;
     }
     // the region-split path advances the step constants inside its shell kernel;
     // the prologue then only runs to re-zero solid cells inside the PML, or to
@@ -278,6 +315,7 @@ fdtd_status check_device_errors(fdtd_solver* s) {
     CUDA_TRY(s, cudaStreamSynchronize(s->stream));
     int ghosts = 0;
     CUDA_TRY(s, fdtd::counted_copy(s, &ghosts, s->d_ghost_count, sizeof(int), cudaMemcpyDeviceToHost));
+    if (!s->moving) s->n_ghost = ghosts;
     if (ghosts > s->region.ghost_cap) {
         set_error(s, "ghost-neighbour list overflow (" + std::to_string(ghosts) + " > " +
                          std::to_string(s->region.ghost_cap) + ")");
@@ -314,6 +352,7 @@ fdtd_status capture_graph(fdtd_solver* s, int cur, int n, bool src, cudaGraphExe
         st = enqueue_step(s, c, s->d_lis + (size_t)i * s->L, false, src);
         c ^= 1;
     }
+    if (st == FDTD_OK) st = flush_lag(s, c);
     if (st == FDTD_OK) st = join_listeners(s);  // the graph ends with every row written
     s->lis_pending[0] = s->lis_pending[1] = false;
     cudaError_t e = cudaStreamEndCapture(s->stream, &g);
@@ -379,7 +418,8 @@ fdtd_status run_steps(fdtd_solver* s, int n, Sink sink) {
             st = after_step(s);
             if (st != FDTD_OK) return st;
         }
-        fdtd_status st = join_listeners(s);
+        fdtd_status st = flush_lag(s, s->cur);
+        if (st == FDTD_OK) st = join_listeners(s);
         if (st != FDTD_OK) return st;
         st = sink(done, m);
         if (st != FDTD_OK) return st;
@@ -1037,13 +1077,13 @@ bool moving_clear_of_pml(fdtd_solver* s) {
     return clear;
 }
 
-// Listener plans (fixed MLS weights) of a static solve from its current
-// classification, as its first step builds them; used after a restore.
+// Listener plans (fixed MLS weights) and ghost-cell plans of a static solve from
+// its current classification, as its first step builds them; used after a restore.
 fdtd_status rebuild_listener_plans(fdtd_solver* s) {
-    if (s->moving || s->L <= 0) return FDTD_OK;
+    if (s->moving) return FDTD_OK;
     CUDA_TRY(s, cudaSetDevice(s->opt.device));
-    CUDA_TRY(s, launch_listener_prep(s->dP, s->precision, s->cur, s->L, s->stream));
-    s->hP.lis_ready = 1;
+    const fdtd_status st = static_prep(s, s->cur);
+    if (st != FDTD_OK) return st;
     CUDA_TRY(s, cudaStreamSynchronize(s->stream));
     return FDTD_OK;
 }
