@@ -878,8 +878,8 @@ static void carve_arena(fdtd_solver* s, const fdtd_scene_desc* sc, const fdtd_op
         s->region.ghost_cap = (int)std::min<double>(cells, (double)n);
         cv.add((void**)&s->d_ghost_list, (size_t)s->region.ghost_cap * 4);
         cv.add((void**)&s->d_ghost_count, 16);
-        // plans of its cells: static scenes with rasterized ghost pressures
-        P.plan_cap = (s->moving || sc->boundary_handling != FDTD_BOUNDARY_RASTERIZE || o.kernel != FDTD_KERNEL_FUSED)
+        // plans of its cells: static scenes
+        P.plan_cap = (s->moving || o.kernel != FDTD_KERNEL_FUSED)
                          ? 0
                          : std::min(s->region.ghost_cap, GHOST_PLAN_MAX);
         if (P.plan_cap > 0) cv.add((void**)&P.ghost_plan, (size_t)P.plan_cap * sizeof(GhostPlan));
@@ -1344,7 +1344,7 @@ fdtd_status fdtd_solver_reset(fdtd_solver* s, double t0) {
     // the whole step in one launch: static scenes with a PML on every side, up to
     // one_launch_cells() (fdtd_one_launch.cuh); explicit tile shapes or staging ask
     // for the region-split kernels
-    s->region.one = (!s->moving && s->opt.kernel == FDTD_KERNEL_FUSED && s->eng.empty() && !s->region.fc &&
+    s->region.one = (!s->moving && s->opt.kernel == FDTD_KERNEL_FUSED && s->eng.empty() &&
                      s->n_solid_pml == 0 && P.plan_cap == P.ghost_cap && s->opt.tile_y == 0 && s->opt.x_chunk == 0 && s->opt.shell_staging == 0 &&
                      s->ncell <= one_launch_cells(s->precision))
                         ? 1

@@ -170,6 +170,8 @@ void free_fully_coupled(fdtd_solver* s) {
     P.fc_idx = nullptr;
     P.fc_b = P.fc_x = P.fc_work = nullptr;
     P.fc_status = nullptr;
+    P.fc_w = nullptr;
+    P.fc_u = nullptr;
     P.fc_n = 0;
 }
 
@@ -327,7 +329,28 @@ fdtd_status build_fully_coupled(fdtd_solver* s) {
         }
     }
     if (nrow == 0) return FDTD_OK;
+    // off-diagonal entries by entry, then by row, for the cluster solve
+    int width = 1;
+    for (const FcRow& r : rows) {
+        int m = 0;
+        for (int q = 0; q < 8; ++q) m += r.kind == 2 && r.unk[q] >= 0;
+        width = std::max(width, m);
+    }
+    std::vector<double> ew((size_t)width * nrow, 0.0);
+    std::vector<int> eu((size_t)width * nrow, -1);
+    for (long long ri = 0; ri < nrow; ++ri) {
+        const FcRow& r = rows[ri];
+        int m = 0;
+        for (int q = 0; q < 8; ++q) {
+            if (r.kind != 2 || r.unk[q] < 0) continue;
+            ew[(size_t)m * nrow + ri] = rows[r.unk[q]].kind <= 1 ? r.w[q] : -r.w[q];
+            eu[(size_t)m * nrow + ri] = r.unk[q];
+            ++m;
+        }
+    }
     void* d_rows = nullptr;
+    void* d_ew = nullptr;
+    void* d_eu = nullptr;
     void* d_idx = nullptr;
     void* d_vec = nullptr;
     void* d_st = nullptr;
@@ -339,6 +362,12 @@ fdtd_status build_fully_coupled(fdtd_solver* s) {
     s->fc_alloc.push_back(d_vec);
     CUDA_TRY(s, cudaMalloc(&d_st, 4 * sizeof(int)));
     s->fc_alloc.push_back(d_st);
+    CUDA_TRY(s, cudaMalloc(&d_ew, ew.size() * sizeof(double)));
+    s->fc_alloc.push_back(d_ew);
+    CUDA_TRY(s, cudaMalloc(&d_eu, eu.size() * sizeof(int)));
+    s->fc_alloc.push_back(d_eu);
+    CUDA_TRY(s, cudaMemcpy(d_ew, ew.data(), ew.size() * sizeof(double), cudaMemcpyHostToDevice));
+    CUDA_TRY(s, cudaMemcpy(d_eu, eu.data(), eu.size() * sizeof(int), cudaMemcpyHostToDevice));
     CUDA_TRY(s, cudaMemcpy(d_rows, rows.data(), nrow * sizeof(FcRow), cudaMemcpyHostToDevice));
     CUDA_TRY(s, cudaMemcpy(d_idx, idx.data(), np * sizeof(int), cudaMemcpyHostToDevice));
     CUDA_TRY(s, cudaMemset(d_vec, 0, 9 * nrow * sizeof(double)));
@@ -349,6 +378,9 @@ fdtd_status build_fully_coupled(fdtd_solver* s) {
     P.fc_x = P.fc_b + nrow;
     P.fc_work = P.fc_x + 2 * nrow;
     P.fc_status = (int*)d_st;
+    P.fc_w = (const double*)d_ew;
+    P.fc_u = (const int*)d_eu;
+    P.fc_width = width;
     P.fc_n = (int)nrow;
     P.fc_maxit = (int)std::min<long long>(2 * nrow, 1000);
     s->fc_immersed = s->fc_fallback = 0;

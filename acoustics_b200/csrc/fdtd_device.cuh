@@ -215,6 +215,7 @@ struct StepConsts {
 // every step by a chain of dependent loads (list, flags, object, table entries)
 // with a division and an exponential per face.
 constexpr uint8_t GHOST_STILL = 0xFF;
+constexpr uint8_t GHOST_COUPLED = 0xFE;  // FULLY_COUPLED: u is the face's row of the system
 constexpr int GHOST_PLAN_MAX = 1 << 17;  // planned cells (10 MB); a longer list ends in the general path
 struct alignas(16) GhostPlan {
     int c;
@@ -354,6 +355,9 @@ struct SolveParams {
     double* fc_b;                 // [fc_n] right-hand side of the step
     double* fc_x;                 // [2][fc_n] ghost pressures by step parity
     double* fc_work;              // [6][fc_n] BiCGSTAB vectors
+    const double* fc_w;           // [fc_width][fc_n] off-diagonal entries (times the column's diagonal), and
+    const int* fc_u;              // their columns; a row's end in -1
+    int fc_width;
     int fc_n;
     int fc_maxit;
     int* fc_status;               // iterations of the last solve (negative: not converged)

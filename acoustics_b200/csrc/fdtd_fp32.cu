@@ -30,8 +30,8 @@ cudaError_t launch_step_regions_fp32(const SolveParams* dP, const SolveParams& h
 #include "fdtd_one_launch.cuh"
 namespace fdtd {
 cudaError_t launch_one_fp32(const SolveParams* dP, const SolveParams& hP, const RegionLaunch& R, int cur, bool src,
-                            int n_ghost, double* lis_row, cudaStream_t s) {
-    return launch_one<float>(dP, hP, R, cur, src, n_ghost, lis_row, s);
+                            int n_ghost, double* lis_row, cudaStream_t s, int* launches) {
+    return launch_one<float>(dP, hP, R, cur, src, n_ghost, lis_row, s, launches);
 }
 }  // namespace fdtd
 
@@ -43,6 +43,7 @@ cudaError_t prepare_fp32_kernels() {
     // the TMA-staged shell: a ring of up to 24 KB stages
     cudaError_t e = cudaFuncSetAttribute(k_pml_shell_tma<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          TMA_STAGES * 24 * 1024 + 16 * TMA_STAGES);
+    if (e == cudaSuccess) e = prepare_fc<float>();
     if (e != cudaSuccess) return e;
     if (shell_smem_bytes<float>() > 0) {
         e = cudaFuncSetAttribute(k_pml_shell<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -1149,8 +1149,8 @@ cudaError_t launch_step_regions_fp64(const SolveParams* dP, const SolveParams& h
 #include "fdtd_one_launch.cuh"
 namespace fdtd {
 cudaError_t launch_one_fp64(const SolveParams* dP, const SolveParams& hP, const RegionLaunch& R, int cur, bool src,
-                            int n_ghost, double* lis_row, cudaStream_t s) {
-    return launch_one<double>(dP, hP, R, cur, src, n_ghost, lis_row, s);
+                            int n_ghost, double* lis_row, cudaStream_t s, int* launches) {
+    return launch_one<double>(dP, hP, R, cur, src, n_ghost, lis_row, s, launches);
 }
 long long one_launch_cells(int precision) { return precision == 0 ? FDTD_ONE_LAUNCH_CELLS_F64 : FDTD_ONE_LAUNCH_CELLS_F32; }
 }  // namespace fdtd
@@ -1164,9 +1164,9 @@ cudaError_t launch_batch_fp64(const BatchLaunch& L, const StepStreams& S, int* l
     return launch_batch<double>(L, S, launches);
 }
 cudaError_t prepare_fp64_kernels() {
+    cudaError_t e = prepare_fc<double>();
     // the full-state shell's ring of staged loads
-    cudaError_t e = cudaSuccess;
-    if (shell_smem_bytes<double>() > 0) {
+    if (e == cudaSuccess && shell_smem_bytes<double>() > 0) {
         e = cudaFuncSetAttribute(k_pml_shell<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  shell_smem_bytes<double>());
         if (e == cudaSuccess)

@@ -262,12 +262,11 @@ FDTD_HD int enclosing_neighbours(const SolveParams& P, const double x[3], int ou
     return n;
 }
 
-// Boundary acceleration vector of object o at a boundary sample point.
-FDTD_HD void boundary_accel(const DevObject& o, const double at[3], double t, double a[3]) {
+// Boundary acceleration vector of object o at a boundary sample point, with
+// g = amp exp(-((t - t0)/tau)^2/2) given.
+FDTD_HD void boundary_accel_g(const DevObject& o, const double at[3], double g, double a[3]) {
     a[0] = a[1] = a[2] = 0.0;
     if (o.accel_kind == 0) return;
-    const double u = (t - o.t0) / o.tau;
-    const double g = o.amp * exp(-(u * u) / 2.0);
     if (o.accel_kind == 1) {
         for (int i = 0; i < 3; ++i) a[i] = o.dir[i] * g;
     } else {
@@ -276,6 +275,16 @@ FDTD_HD void boundary_accel(const DevObject& o, const double at[3], double t, do
         const double r[3] = {r0, r1, r2};
         for (int i = 0; i < 3; ++i) a[i] = (n > 0.0 ? r[i] / n : 0.0) * g;
     }
+}
+
+// The same at time t.
+FDTD_HD void boundary_accel(const DevObject& o, const double at[3], double t, double a[3]) {
+    double g = 0.0;
+    if (o.accel_kind != 0) {
+        const double u = (t - o.t0) / o.tau;
+        g = o.amp * exp(-(u * u) / 2.0);
+    }
+    boundary_accel_g(o, at, g, a);
 }
 
 // RASTERIZE ghost-face pressure (MAC_Grid.cpp:1188-1281):

@@ -675,9 +675,7 @@ cudaError_t launch_regions(const SolveParams* dP, const SolveParams& hP, const R
     }
     if (R.fc) {
         // FULLY_COUPLED: this step's ghost pressures, before the cells that read them
-        k_fc_rhs<T><<<64, 256, 0, gside ? S.s3 : si>>>(dP, cur);
-        k_fc_solve<<<1, 1024, 0, gside ? S.s3 : si>>>(dP, cur);
-        l += 2;
+        if ((e = launch_fc<T>(dP, hP, cur, gside ? S.s3 : si, false, &l)) != cudaSuccess) return e;
     }
     if (has_ghost) {
         // cells next to a solid: disjoint from the interior and shell cells

@@ -45,6 +45,7 @@ struct OneLaunch {
     const int* ghost_count;
     int plan_cap;
     double h75, rho;
+    const double* fc_x;
     int n_lis;
     const LisPlan* lis_plan;
     const LisRow* lis_rows;
@@ -224,7 +225,7 @@ __device__ __noinline__ void one_listener_unplanned(const SolveParams* P, int ne
 template <typename T, bool VISC>
 __device__ __forceinline__ void one_ghost_cells(const KArgs<T>& A, const OneLaunch& L, int first) {
     const GhostArgs<T> G{A.pc, A.pn, A.dinc, VISC ? A.lapl : nullptr, A.lapc, A.sx, A.sy, A.c2k2, A.lap_scale, A.kcalp,
-                         L.h75, L.rho, L.src.consts};
+                         L.h75, L.rho, L.src.consts, L.fc_x};
     // the list is no result of the step before; its first plans are read beside the count
     const int stride = L.ghost_blocks * 256, q = threadIdx.x & 3;
     GhostLoad p{};
@@ -304,7 +305,12 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FDTD_ONE_MINB_F32 : FDTD
 
 template <typename T>
 cudaError_t launch_one(const SolveParams* dP, const SolveParams& hP, const RegionLaunch& R, int cur, bool src, int n_ghost,
-                       double* lis_row, cudaStream_t s) {
+                       double* lis_row, cudaStream_t s, int* launches) {
+    if (R.fc) {
+        const cudaError_t e = launch_fc<T>(dP, hP, cur, s, true, launches);
+        if (e != cudaSuccess) return e;
+    }
+    if (launches) *launches += 1;
     KArgs<T> A = make_kargs<T>(const_cast<SolveParams*>(dP), hP, cur);
     OneLaunch L{};
     L.interior = R.interior;
@@ -339,6 +345,7 @@ cudaError_t launch_one(const SolveParams* dP, const SolveParams& hP, const Regio
     L.plan_cap = hP.plan_ready ? hP.plan_cap : 0;
     L.h75 = 0.75 * hP.h;
     L.rho = hP.rho;
+    L.fc_x = R.fc ? hP.fc_x + (size_t)cur * hP.fc_n : nullptr;
     L.n_lis = hP.n_lis;
     L.lis_plan = hP.lis_plan;
     L.lis_rows = hP.lis_rows;

@@ -124,13 +124,14 @@ struct GhostArgs {
     T c2k2, lap_scale, kcalp;
     double h75, rho;              // 0.75 h, rho
     const StepConsts* consts;     // of this step
+    const double* fc_x;           // FULLY_COUPLED: this step's ghost pressures by row
 };
 
 template <typename T>
 __device__ __forceinline__ GhostArgs<T> ghost_args(const SolveParams& P, int cur) {
     return GhostArgs<T>{(const T*)P.p[cur], (T*)P.p[cur ^ 1], P.dinc, P.visc ? (const T*)P.lapv[cur ^ 1] : nullptr,
                         (T*)P.lapv[cur], (unsigned)P.SX, (unsigned)P.SY, (T)P.c2k2, (T)P.lap_scale, (T)P.kcalp,
-                        0.75 * P.h, P.rho, P.consts + cur};
+                        0.75 * P.h, P.rho, P.consts + cur, P.fc_rows ? P.fc_x + (size_t)cur * P.fc_n : nullptr};
 }
 
 // ghost_cell from the cells' plans, four lanes a cell: an axis of the Laplacian
@@ -182,8 +183,12 @@ __device__ __forceinline__ void ghost_cell_planned(const GhostArgs<T>& A, const 
     // bodies of the axis' two faces: bytes 8-13 of the plan
     const uint32_t bodies = q == 0 ? G.h0.z : q == 1 ? G.h0.z >> 16 : G.h0.w;
     const unsigned on_n = bodies & 0xFFu, on_p = (bodies >> 8) & 0xFFu;
-    const double gt_n = gn && on_n != GHOST_STILL ? A.consts->obj_g[on_n] : 0.0;
-    const double gt_p = gp && on_p != GHOST_STILL ? A.consts->obj_g[on_p] : 0.0;
+    // a face's body's acceleration, or its solved pressure
+    auto face = [&](bool here, unsigned o, double u) {
+        if (!here || o == GHOST_STILL) return 0.0;
+        return o == GHOST_COUPLED ? A.fc_x[(int)u] : A.consts->obj_g[o];
+    };
+    const double gt_n = face(gn, on_n, G.u.x), gt_p = face(gp, on_p, G.u.y);
     double add = 0.0;
     bool add_src = false;
     if (S && S->n > 0 && q == 3) {
@@ -193,9 +198,9 @@ __device__ __forceinline__ void ghost_cell_planned(const GhostArgs<T>& A, const 
         if (add_src) add = source_at(*S, x, y, z) * S->k;
     }
     double vn = (double)p0, vp = (double)p0;
-    if (gn && on_n != GHOST_STILL) vn = vn - A.h75 * (G.u.x * gt_n * (-A.rho));
+    if (gn && on_n != GHOST_STILL) vn = on_n == GHOST_COUPLED ? gt_n : vn - A.h75 * (G.u.x * gt_n * (-A.rho));
     // the face toward + has its normal toward this cell, along -
-    if (gp && on_p != GHOST_STILL) vp = vp - A.h75 * (G.u.y * gt_p * (-A.rho) * -1.0);
+    if (gp && on_p != GHOST_STILL) vp = on_p == GHOST_COUPLED ? gt_p : vp - A.h75 * (G.u.y * gt_p * (-A.rho) * -1.0);
     const T pgn = (T)vn, pgp = (T)vp;
     T num, den;
     if (gp && gn) {
@@ -281,6 +286,14 @@ static __global__ void __launch_bounds__(128) k_ghost_prep(const SolveParams* __
                 G.u[d][s] = 0.0;
                 if (!((G.code >> f) & 1u)) continue;
                 const int sgn = s ? 1 : -1;
+                if (P.fc_rows) {
+                    const int row = fc_row(P, G.c + sgn * strides[d], 2 * d + (s ? 0 : 1));
+                    if (row >= 0) {  // (else, which classification rules out, the cell's own pressure)
+                        G.obj[f] = GHOST_COUPLED;
+                        G.u[d][s] = (double)row;
+                    }
+                    continue;
+                }
                 const unsigned gobj = P.gobj[G.c + sgn * strides[d]];
                 const unsigned o = gobj & 0x7F;
                 if ((gobj & GOBJ_CONSTRAINT) || o >= (unsigned)P.n_obj || P.obj[o].accel_kind == 0) continue;
