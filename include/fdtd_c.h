@@ -451,14 +451,15 @@ fdtd_status fdtd_solver_time_kernel(fdtd_solver* s, int32_t which, int32_t n_lau
  *   p_next = 2 p_curr - p_prev + c2k2 * lap_scale * sum_d (p_+ + p_- - 2 p_curr)
  * p_next may equal p_prev (in place); cells outside the box are not written.
  * Requires 1 <= lo < hi <= dims-1 per axis and at most FDTD_NOALLOC_MAX_CELLS
- * box cells (FDTD_ERR_INVALID_ARG otherwise).  The Laplacian scratch is one
- * static device array of FDTD_NOALLOC_MAX_CELLS doubles (8 MiB) that every GPU
- * loading the library keeps until exit.  The first call on a device (and the
- * first after a device reset gave it a new context) looks up that array's
- * device address (cudaGetSymbolAddress) with the device current; make that
- * first call before any stream capture.  Calls share the array, so calls that
- * overlap on the GPU race; serialise them on one stream.  `stream` is a
- * cudaStream_t (NULL: the legacy default stream); the call only enqueues work. */
+ * box cells (FDTD_ERR_INVALID_ARG otherwise).  A call whose p_next shares no
+ * memory with p_curr is one launch that needs no scratch.  Where it does
+ * (stepping over p_curr), the Laplacian scratch is one static device array of
+ * FDTD_NOALLOC_MAX_CELLS doubles (8 MiB) that every GPU loading the library
+ * keeps until exit: the first such call on a device (and the first after a
+ * device reset gave it a new context) looks up that array's device address
+ * (cudaGetSymbolAddress) with the device current, so make it before any stream
+ * capture, and such calls share the array, so those that overlap on the GPU
+ * race; serialise them on one stream.  `stream` is a cudaStream_t (NULL: the legacy default stream); the call only enqueues work. */
 #define FDTD_NOALLOC_MAX_CELLS (1 << 20)
 fdtd_status fdtd_interior_step_noalloc(const double* p_curr, const double* p_prev, double* p_next,
                                        const int32_t dims[3], const int32_t lo[3], const int32_t hi[3],
