@@ -851,6 +851,7 @@ static void carve_arena(fdtd_solver* s, const fdtd_scene_desc* sc, const fdtd_op
         cv.add((void**)&P.pdiv_f[d], N[d] * 4);
         cv.add((void**)&P.vupd_f[d], (N[d] + 1) * 4);
         cv.add((void**)&P.vgrad_f[d], (N[d] + 1) * 4);
+        cv.add((void**)&s->d_csig[d], N[d] * 8);
         // N+8 entries: z-vector groups of the shell kernel read up to 7 past N (zeros)
         cv.add((void**)&P.axflag[d], N[d] + 8);
         cv.add((void**)&P.coef_d[d], (N[d] + 8) * sizeof(AxisCoef<double>));
@@ -1172,6 +1173,7 @@ fdtd_status fdtd_solver_create(const fdtd_scene_desc* sc, const fdtd_options* op
         CUDA_TRY(s.get(), fdtd::counted_copy(s.get(), (void*)P.pdiv_f[d], f2.data(), N[d] * 4, cudaMemcpyHostToDevice));
         CUDA_TRY(s.get(), fdtd::counted_copy(s.get(), (void*)P.vupd_f[d], f3.data(), (N[d] + 1) * 4, cudaMemcpyHostToDevice));
         CUDA_TRY(s.get(), fdtd::counted_copy(s.get(), (void*)P.vgrad_f[d], f4.data(), (N[d] + 1) * 4, cudaMemcpyHostToDevice));
+        CUDA_TRY(s.get(), fdtd::counted_copy(s.get(), (void*)s->d_csig[d], T.csig.data(), N[d] * 8, cudaMemcpyHostToDevice));
         // packed flags and coefficient quads of the shell kernel
         std::vector<uint8_t> fl(N[d] + 8, 0);
         std::vector<AxisCoef<double>> cd(N[d] + 8, AxisCoef<double>{0.0, 0.0, 0.0, 0.0});
@@ -1232,6 +1234,9 @@ fdtd_status fdtd_solver_destroy(fdtd_solver* s) {
     if (s->d_solid_pml) cudaFree(s->d_solid_pml);
     if (s->arena) arena_release(s->opt.device, s->arena, s->arena_block);
     if (s->h_lis_stage) cudaFreeHost(s->h_lis_stage);
+    if (s->rb_host) cudaFreeHost(s->rb_host);
+    for (cudaEvent_t ev : s->rb_done)
+        if (ev) cudaEventDestroy(ev);
     for (cudaEvent_t ev : {s->ev_fork, s->ev_join, s->ev_ghost, s->ev_step, s->ev_lis[0], s->ev_lis[1], s->ev_lis_join,
                            s->ev_sfork, s->ev_sdone})
         if (ev) cudaEventDestroy(ev);

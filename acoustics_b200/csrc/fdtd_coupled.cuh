@@ -4,7 +4,7 @@
 // fdtd_coupled.cpp) and its solution by BiCGSTAB with the diagonal
 // preconditioner and a tolerance of one machine epsilon relative to the
 // right-hand side, the reference's solver and settings (MAC_Grid.cpp:1409-1412),
-// in one CTA.  The ghost pressures of a step land in fc_x[parity]; the
+// in a cluster of eight CTAs (one CTA for more rows than it holds).  The ghost pressures of a step land in fc_x[parity]; the
 // ghost-cell Laplacian and the listeners of that step read them there.
 #pragma once
 #include "fdtd_device.cuh"

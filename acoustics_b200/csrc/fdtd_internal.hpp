@@ -12,6 +12,9 @@
 
 namespace fdtd {
 
+constexpr size_t READBACK_BYTES = (size_t)512 << 10;
+constexpr int READBACK_WORKERS = 8;
+
 struct HostObject {
     fdtd_object_desc d;
     double c[3] = {0, 0, 0};
@@ -135,6 +138,11 @@ struct fdtd_solver {
     long long last_launches = 0;
     long long graph_launches_per_exec = 0;
     fdtd::TmaStep* tma = nullptr;     // tiles and tensor maps of the TMA-staged shell (reduced state)
+    // read-backs (fields, cells): mapped host staging made on first use, a part and
+    // an event per worker
+    void* rb_host = nullptr;
+    cudaEvent_t rb_done[fdtd::READBACK_WORKERS] = {};
+    const double* d_csig[3] = {nullptr, nullptr, nullptr};  // absorption at the cell centres
     // bytes this handle copied between host and device memory since creation
     long long bytes_h2d = 0, bytes_d2h = 0;
     std::string err;

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "../../include/fdtd_c.h"
 #include "fdtd_device.cuh"
 
 namespace fdtd {
@@ -61,24 +62,33 @@ cudaError_t launch_fresh_cells(const SolveParams* dP, int precision, int cur, lo
 cudaError_t launch_phased_fp64(const SolveParams* dP, const int N[3], int cur, double* lap, cudaStream_t s,
                                int* launches);
 
-// fdtd_fetch.cu: cell read-back (FetchCell / SampleAxisAlignedSlice).  A request
-// is a padded cell index and the element addresses of its split pressures
-// (a[0..2]) and of its lower (a[3+2d]) and upper (a[4+2d]) face velocities,
-// null where the solve does not hold them.
-struct FetchReq {
-    long long c;
-    const void* a[9];
+// fdtd_fetch.cu: read-back of cells (FetchCell / SampleAxisAlignedSlice) and fields.
+// Cells first, first + 1, ... of a request: the cell `cell` (dim < 0), or the plane
+// k of axis dim with i over N[(dim+1)%3] outer, j over N[(dim+2)%3] inner.
+struct FetchArgs {
+    int dim, k;
+    long long cell;
+    long long step_index;
+    double pml_strength;
+    bool reduced, phased, moving;
+    int vbuf;                 // face-velocity buffer of the current state
+    const double* csig[3];    // absorption at the cell centres
+    ShellBoxes shell;
 };
-struct FetchVal {
-    double p, p_prev;   // p^{n+1} (current) and p^n
-    double pdir[3];
-    double v[6];        // lower / upper face along x, y, z
-    double gc[6];       // ghost-face pressures of the last step toward -x,+x,-y,+y,-z,+z; -1: none
-    double lap;         // the Laplacian kept for the next step (air viscosity), else NaN
-    int cls, gobj;      // classification byte and ghost-object byte
+cudaError_t launch_fetch_cells(const SolveParams* dP, bool fp64, int cur, const FetchArgs& F, long long first, int n,
+                               fdtd_cell* out, cudaStream_t s);  // out may be mapped host memory
+// Elements first .. first + n of a dense field (extents ext) as doubles to out:
+// src (and, where the PML state is compact, zsrc) hold it; inc: subtracted (FP32
+// p^{n-1}); dface: the faces' axis, -1 for cells.  out may be mapped host memory.
+struct FieldArgs {
+    const void* src;
+    const float* inc;
+    const void* zsrc;
+    int ext[3], N[3], dface;
+    long long SX, SY;
+    ShellBoxes shell;
 };
-cudaError_t launch_fetch_cells(const SolveParams* dP, bool fp64, int cur, const FetchReq* req, FetchVal* out, int n,
-                               cudaStream_t s);
+cudaError_t launch_field_dense(const FieldArgs& F, bool fp64, long long first, long long n, double* out, cudaStream_t s);
 
 // fdtd_fp32.cu
 cudaError_t prepare_fp32_kernels();

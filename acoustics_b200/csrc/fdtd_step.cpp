@@ -4,10 +4,12 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
-#include <limits>
+#include <exception>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/fdtd_c.h"
@@ -717,26 +719,28 @@ long long zslab_index(const fdtd_solver* s, int dface, int x, int y, int z) {
     return ((long long)(x - B.x0[b]) * B.ny[b] + (y - B.y0[b])) * B.zrw + q;
 }
 
-// Field `which` between the device layout (padded arrays, the compact z-slab
-// arrays of the PML state) and a dense host array in the reference's flat order
-// (cells, or faces of one orientation).  to_device: dense -> device.  FP32
-// PRESSURE_PREV is p^n - d (d the compensated increment); writing it sets d from
-// the p^n already on the device, so write PRESSURE first.
-fdtd_status field_transfer(fdtd_solver* s, int32_t which, double* dense, int64_t count, bool to_device) {
-    if (!s || !dense) return FDTD_ERR_INVALID_ARG;
-    CUDA_TRY(s, cudaSetDevice(s->opt.device));
+// Where field `which` lies on the device: padded array, the compact z-slab array
+// of the PML state (or null) and the extents of its dense form.  FP32 PRESSURE_PREV
+// is p^n - d (d the compensated increment).
+struct FieldPlace {
+    void* src = nullptr;
+    void* zsrc = nullptr;
+    int ext[3] = {0, 0, 0};
+    int dface = -1;
+    bool fp32_prev = false;
+};
+
+fdtd_status field_place(fdtd_solver* s, int32_t which, int64_t count, FieldPlace& f) {
     const SolveParams& P = s->hP;
     const bool f64 = s->precision == FDTD_PRECISION_FP64;
-    const size_t w = f64 ? 8 : 4;
-    void* src = nullptr;
     long long n = s->ncell;
-    int vbuf = s->opt.kernel == FDTD_KERNEL_PHASED ? 0 : s->cur;
+    const int vbuf = s->opt.kernel == FDTD_KERNEL_PHASED ? 0 : s->cur;
     switch (which) {
-        case FDTD_FIELD_PRESSURE: src = P.p[s->cur]; break;
-        case FDTD_FIELD_PRESSURE_PREV: src = f64 ? P.p[s->cur ^ 1] : P.p[s->cur]; break;
-        case FDTD_FIELD_PML_PX: case FDTD_FIELD_PML_PY: case FDTD_FIELD_PML_PZ: src = P.pd[which - FDTD_FIELD_PML_PX]; break;
+        case FDTD_FIELD_PRESSURE: f.src = P.p[s->cur]; break;
+        case FDTD_FIELD_PRESSURE_PREV: f.src = f64 ? P.p[s->cur ^ 1] : P.p[s->cur]; break;
+        case FDTD_FIELD_PML_PX: case FDTD_FIELD_PML_PY: case FDTD_FIELD_PML_PZ: f.src = P.pd[which - FDTD_FIELD_PML_PX]; break;
         case FDTD_FIELD_VX: case FDTD_FIELD_VY: case FDTD_FIELD_VZ:
-            src = P.v[vbuf][which - FDTD_FIELD_VX];
+            f.src = P.v[vbuf][which - FDTD_FIELD_VX];
             n = s->vcount[which - FDTD_FIELD_VX];
             break;
         default: return (set_error(s, "unknown field"), FDTD_ERR_INVALID_ARG);
@@ -747,197 +751,166 @@ fdtd_status field_transfer(fdtd_solver* s, int32_t which, double* dense, int64_t
                              "along axes without absorption); create it with pml_state = FDTD_PML_STATE_FULL to "
                              "access them"),
                 FDTD_ERR_UNSUPPORTED);
-    // extent of the requested grid (cells, or faces of one orientation)
-    int ext[3] = {s->N[0], s->N[1], s->N[2]};
-    if (which >= FDTD_FIELD_VX) ext[which - FDTD_FIELD_VX] += 1;
+    for (int d = 0; d < 3; ++d) f.ext[d] = s->N[d];
+    if (which >= FDTD_FIELD_VX) {
+        f.dface = which - FDTD_FIELD_VX;
+        f.ext[f.dface] += 1;
+    }
+    f.fp32_prev = !f64 && which == FDTD_FIELD_PRESSURE_PREV;
+    if (P.zcount > 0 && which >= FDTD_FIELD_PML_PX)
+        f.zsrc = which <= FDTD_FIELD_PML_PZ ? P.zpd[which - FDTD_FIELD_PML_PX] : P.zv[vbuf][which - FDTD_FIELD_VX];
+    return FDTD_OK;
+}
+
+// A dense host array into a field (fdtd_solver_set_field).  Writing FP32
+// PRESSURE_PREV sets d from the p^n already on the device, so write PRESSURE first.
+fdtd_status field_write(fdtd_solver* s, int32_t which, const double* dense, int64_t count) {
+    if (!s || !dense) return FDTD_ERR_INVALID_ARG;
+    CUDA_TRY(s, cudaSetDevice(s->opt.device));
+    const SolveParams& P = s->hP;
+    FieldPlace f;
+    const fdtd_status st = field_place(s, which, count, f);
+    if (st != FDTD_OK) return st;
+    const bool f64 = s->precision == FDTD_PRECISION_FP64;
+    const size_t w = f64 ? 8 : 4;
     const long long np = s->np;
-    std::vector<char> raw(np * w);
+    std::vector<char> raw(np * w), zraw;
     std::vector<float> inc;
-    CUDA_TRY(s, fdtd::counted_copyAsync(s, raw.data(), src, np * w, cudaMemcpyDeviceToHost, s->stream));
-    const bool fp32_prev = !f64 && which == FDTD_FIELD_PRESSURE_PREV;
-    if (fp32_prev) {
+    CUDA_TRY(s, fdtd::counted_copyAsync(s, raw.data(), f.src, np * w, cudaMemcpyDeviceToHost, s->stream));
+    if (f.fp32_prev) {
         inc.resize(np);
         CUDA_TRY(s, fdtd::counted_copyAsync(s, inc.data(), P.dinc, np * 4, cudaMemcpyDeviceToHost, s->stream));
     }
     // the z-slab box keeps its PML state in compact arrays (ShellBoxes)
     const ShellBoxes& B = s->shell;
-    const bool zc = P.zcount > 0 && which >= FDTD_FIELD_PML_PX;
-    std::vector<char> zraw;
-    void* zsrc = nullptr;
-    if (zc) {
-        zsrc = which <= FDTD_FIELD_PML_PZ ? P.zpd[which - FDTD_FIELD_PML_PX] : P.zv[vbuf][which - FDTD_FIELD_VX];
+    if (f.zsrc) {
         zraw.resize(P.zcount * w);
-        CUDA_TRY(s, fdtd::counted_copyAsync(s, zraw.data(), zsrc, P.zcount * w, cudaMemcpyDeviceToHost, s->stream));
+        CUDA_TRY(s, fdtd::counted_copyAsync(s, zraw.data(), f.zsrc, P.zcount * w, cudaMemcpyDeviceToHost, s->stream));
     }
     CUDA_TRY(s, cudaStreamSynchronize(s->stream));
-    // every (padded grid index, compact index) pair of the z-slab box
-    auto for_compact = [&](auto&& fn) {
-        const int b = B.zbox;
-        const int dface = which >= FDTD_FIELD_VX ? which - FDTD_FIELD_VX : -1;
-        for (int x = B.x0[b]; x < B.x0[b] + B.nx[b]; ++x)
-            for (int y = B.y0[b]; y < B.y0[b] + B.ny[b]; ++y)
-                for (int z = 0; z <= s->N[2]; ++z) {
-                    const long long q = zslab_index(s, dface, x, y, z);
-                    if (q >= 0) fn(x * s->SX + y * s->SY + z, q);
-                }
-    };
     double* r64 = (double*)raw.data();
     float* r32 = (float*)raw.data();
-    if (!to_device) {
-        if (zc) for_compact([&](long long c, long long q) { std::memcpy(raw.data() + c * w, zraw.data() + q * w, w); });
-        long long o = 0;
-        for (int i = 0; i < ext[0]; ++i)
-            for (int j = 0; j < ext[1]; ++j)
-                for (int k = 0; k < ext[2]; ++k, ++o) {
-                    const long long c = i * s->SX + j * s->SY + k;
-                    if (f64) dense[o] = r64[c];
-                    else dense[o] = fp32_prev ? (double)r32[c] - (double)inc[c] : (double)r32[c];
-                }
-        return FDTD_OK;
-    }
     long long o = 0;
-    for (int i = 0; i < ext[0]; ++i)
-        for (int j = 0; j < ext[1]; ++j)
-            for (int k = 0; k < ext[2]; ++k, ++o) {
+    for (int i = 0; i < f.ext[0]; ++i)
+        for (int j = 0; j < f.ext[1]; ++j)
+            for (int k = 0; k < f.ext[2]; ++k, ++o) {
                 const long long c = i * s->SX + j * s->SY + k;
                 if (f64) r64[c] = dense[o];
-                else if (fp32_prev) inc[c] = (float)((double)r32[c] - dense[o]);
+                else if (f.fp32_prev) inc[c] = (float)((double)r32[c] - dense[o]);
                 else r32[c] = (float)dense[o];
             }
-    if (fp32_prev) {
+    if (f.fp32_prev) {
         CUDA_TRY(s, fdtd::counted_copyAsync(s, P.dinc, inc.data(), np * 4, cudaMemcpyHostToDevice, s->stream));
     } else {
-        if (zc) for_compact([&](long long c, long long q) { std::memcpy(zraw.data() + q * w, raw.data() + c * w, w); });
-        CUDA_TRY(s, fdtd::counted_copyAsync(s, src, raw.data(), np * w, cudaMemcpyHostToDevice, s->stream));
-        if (zc) CUDA_TRY(s, fdtd::counted_copyAsync(s, zsrc, zraw.data(), P.zcount * w, cudaMemcpyHostToDevice, s->stream));
+        if (f.zsrc) {
+            // every (padded grid index, compact index) pair of the z-slab box
+            const int b = B.zbox;
+            for (int x = B.x0[b]; x < B.x0[b] + B.nx[b]; ++x)
+                for (int y = B.y0[b]; y < B.y0[b] + B.ny[b]; ++y)
+                    for (int z = 0; z <= s->N[2]; ++z) {
+                        const long long q = zslab_index(s, f.dface, x, y, z);
+                        if (q >= 0) std::memcpy(zraw.data() + q * w, raw.data() + (x * s->SX + y * s->SY + z) * w, w);
+                    }
+        }
+        CUDA_TRY(s, fdtd::counted_copyAsync(s, f.src, raw.data(), np * w, cudaMemcpyHostToDevice, s->stream));
+        if (f.zsrc)
+            CUDA_TRY(s, fdtd::counted_copyAsync(s, f.zsrc, zraw.data(), P.zcount * w, cudaMemcpyHostToDevice, s->stream));
     }
     CUDA_TRY(s, cudaStreamSynchronize(s->stream));
     return FDTD_OK;
 }
 
-// Device address of element (x, y, z) of a split pressure or face-velocity
-// field, where field_transfer finds it; null when the solve does not hold it
-// (the reduced PML state).
-const void* field_element(const fdtd_solver* s, int which, int x, int y, int z) {
-    const SolveParams& P = s->hP;
-    if (s->region.red) return nullptr;
-    const size_t w = s->precision == FDTD_PRECISION_FP64 ? 8 : 4;
-    const int vbuf = s->opt.kernel == FDTD_KERNEL_PHASED ? 0 : s->cur;
-    const int dface = which >= FDTD_FIELD_VX ? which - FDTD_FIELD_VX : -1;
-    const void* base = dface < 0 ? P.pd[which - FDTD_FIELD_PML_PX] : P.v[vbuf][dface];
-    if (!base) return nullptr;
-    const long long q = zslab_index(s, dface, x, y, z);
-    if (q >= 0) {
-        const void* zb = dface < 0 ? P.zpd[which - FDTD_FIELD_PML_PX] : P.zv[vbuf][dface];
-        return (const char*)zb + q * (long long)w;
+// total items of item_bytes to out: launch(first, n, buffer) makes a chunk of them
+// in the mapped host buffer given (enqueued on the solver stream), which is then
+// copied out.  The device makes the chunks at the bus's rate; what takes long is
+// the first touch of the caller's fresh memory (35 MB: 7.5 ms with one thread, 1.3
+// with eight), so several threads take chunks in turn, each with its own buffer.
+template <typename Launch>
+fdtd_status read_back(fdtd_solver* s, long long total, size_t item_bytes, void* out, Launch launch) {
+    const long long chunk = (long long)(fdtd::READBACK_BYTES / item_bytes);
+    const long long chunks = (total + chunk - 1) / chunk;
+    if (!s->rb_host)
+        CUDA_TRY(s, cudaHostAlloc(&s->rb_host, fdtd::READBACK_WORKERS * fdtd::READBACK_BYTES, cudaHostAllocMapped));
+    const unsigned cores = std::thread::hardware_concurrency();
+    const int workers = (int)std::min<long long>({chunks, (long long)fdtd::READBACK_WORKERS, cores ? (long long)cores : 1});
+    for (int w = 0; w < workers; ++w)
+        if (!s->rb_done[w]) CUDA_TRY(s, cudaEventCreateWithFlags(&s->rb_done[w], cudaEventDisableTiming));
+    std::atomic<long long> next{0};
+    std::atomic<int> failed{(int)cudaSuccess};
+    auto work = [&](int w) {
+        char* buf = (char*)s->rb_host + (size_t)w * fdtd::READBACK_BYTES;
+        cudaError_t e = w > 0 ? cudaSetDevice(s->opt.device) : cudaSuccess;
+        for (long long c; e == cudaSuccess && failed.load() == (int)cudaSuccess && (c = next.fetch_add(1)) < chunks;) {
+            const long long first = c * chunk, n = std::min(chunk, total - first);
+            e = launch(first, n, buf);
+            if (e == cudaSuccess) e = cudaEventRecord(s->rb_done[w], s->stream);
+            if (e == cudaSuccess) e = cudaEventSynchronize(s->rb_done[w]);
+            if (e == cudaSuccess) std::memcpy((char*)out + (size_t)first * item_bytes, buf, (size_t)n * item_bytes);
+        }
+        int none = (int)cudaSuccess;
+        if (e != cudaSuccess) failed.compare_exchange_strong(none, (int)e);
+    };
+    std::vector<std::thread> others;
+    try {
+        for (int w = 1; w < workers; ++w) others.emplace_back(work, w);
+    } catch (const std::exception&) {
+        // no thread to be had: the ones there are take all chunks
     }
-    return (const char*)base + (x * s->SX + y * s->SY + z) * (long long)w;
+    work(0);
+    for (auto& t : others) t.join();
+    CUDA_TRY(s, (cudaError_t)failed.load());
+    fdtd::count_transfer(s, (size_t)total * item_bytes, cudaMemcpyDeviceToHost);
+    return FDTD_OK;
+}
+
+// A field as a dense host array of doubles (fdtd_solver_get_field).
+fdtd_status field_read(fdtd_solver* s, int32_t which, double* dense, int64_t count) {
+    if (!s || !dense) return FDTD_ERR_INVALID_ARG;
+    CUDA_TRY(s, cudaSetDevice(s->opt.device));
+    FieldPlace f;
+    const fdtd_status st = field_place(s, which, count, f);
+    if (st != FDTD_OK) return st;
+    const SolveParams& P = s->hP;
+    FieldArgs F{};
+    F.src = f.src;
+    F.inc = f.fp32_prev ? P.dinc : nullptr;
+    F.zsrc = f.zsrc;
+    F.dface = f.dface;
+    for (int d = 0; d < 3; ++d) {
+        F.ext[d] = f.ext[d];
+        F.N[d] = s->N[d];
+    }
+    F.SX = s->SX;
+    F.SY = s->SY;
+    F.shell = s->shell;
+    return read_back(s, count, sizeof(double), dense, [&](long long first, long long n, void* buf) {
+        return launch_field_dense(F, s->precision == FDTD_PRECISION_FP64, first, n, (double*)buf, s->stream);
+    });
 }
 
 // MAC_Grid::GetCell (MAC_Grid.cpp:4182-4258) + the stored Laplacian of
-// PML_WaveSolver::FetchCell (PML_WaveSolver.cpp:439-447) for the cells of
-// dense indices `cells`: the device gathers (k_fetch_cells), the host fills
-// the geometry and PressureCellType (MAC_Grid.cpp:3977-3997).
-fdtd_status fetch_cells(fdtd_solver* s, const std::vector<long long>& cells, fdtd_cell* out) {
+// PML_WaveSolver::FetchCell (PML_WaveSolver.cpp:439-447): cell `cell` (dim < 0)
+// or the `total` cells of plane k of axis dim, made by the device (k_fetch_cells).
+fdtd_status fetch_cells(fdtd_solver* s, int dim, int k, long long cell, long long total, fdtd_cell* out) {
     CUDA_TRY(s, cudaSetDevice(s->opt.device));
-    const int n = (int)cells.size();
-    if (n == 0) return FDTD_OK;
-    std::vector<FetchReq> req(n);
-    for (int q = 0; q < n; ++q) {
-        int ijk[3];
-        const long long t = cells[q];
-        ijk[0] = (int)(t / ((long long)s->N[1] * s->N[2]));
-        ijk[1] = (int)((t / s->N[2]) % s->N[1]);
-        ijk[2] = (int)(t % s->N[2]);
-        FetchReq& R = req[q];
-        R.c = ijk[0] * s->SX + ijk[1] * s->SY + ijk[2];
-        for (int d = 0; d < 3; ++d) {
-            int up[3] = {ijk[0], ijk[1], ijk[2]};
-            up[d] += 1;  // the upper face index never exceeds N[d] (MAC_Grid.cpp:4247-4249)
-            R.a[d] = field_element(s, FDTD_FIELD_PML_PX + d, ijk[0], ijk[1], ijk[2]);
-            R.a[3 + 2 * d] = field_element(s, FDTD_FIELD_VX + d, ijk[0], ijk[1], ijk[2]);
-            R.a[4 + 2 * d] = field_element(s, FDTD_FIELD_VX + d, up[0], up[1], up[2]);
-        }
-    }
-    const size_t req_bytes = (size_t)n * sizeof(FetchReq), val_bytes = (size_t)n * sizeof(FetchVal);
-    std::vector<FetchVal> vals(n);
-    void* dbuf = nullptr;
-    CUDA_TRY(s, cudaMallocAsync(&dbuf, req_bytes + val_bytes, s->stream));
-    FetchReq* dreq = (FetchReq*)dbuf;
-    FetchVal* dval = (FetchVal*)((char*)dbuf + req_bytes);
-    cudaError_t e = fdtd::counted_copyAsync(s, dreq, req.data(), req_bytes, cudaMemcpyHostToDevice, s->stream);
-    if (e == cudaSuccess)
-        e = launch_fetch_cells(s->dP, s->precision == FDTD_PRECISION_FP64, s->cur, dreq, dval, n, s->stream);
-    if (e == cudaSuccess) {
-        ++s->launches;
-        e = fdtd::counted_copyAsync(s, vals.data(), dval, val_bytes, cudaMemcpyDeviceToHost, s->stream);
-    }
-    const cudaError_t ef = cudaFreeAsync(dbuf, s->stream);
-    if (e == cudaSuccess) e = ef;
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
-    CUDA_TRY(s, e);
-    // the Laplacian kept for the next step: the phased path keeps the reference's
-    // (every cell, every step); the fused kernels keep it on the non-PML cells of
-    // a static scene (its other cells stay zero)
-    const bool visc = s->hP.visc != 0;
-    const bool phased = s->opt.kernel == FDTD_KERNEL_PHASED;
-    const double nan = std::numeric_limits<double>::quiet_NaN();
-    for (int q = 0; q < n; ++q) {
-        const long long t = cells[q];
-        const FetchVal& v = vals[q];
-        fdtd_cell& C = out[q];
-        std::memset(&C, 0, sizeof(C));
-        C.index = (int32_t)t;
-        C.indices[0] = (int32_t)(t / ((long long)s->N[1] * s->N[2]));
-        C.indices[1] = (int32_t)((t / s->N[2]) % s->N[1]);
-        C.indices[2] = (int32_t)(t % s->N[2]);
-        const int i = C.indices[0], j = C.indices[1], k = C.indices[2];
-        const uint8_t f = cell_flags(s, (uint8_t)v.cls, (uint8_t)v.gobj, i, j, k);
-        int32_t flags = f;
-        const bool pml = f & FDTD_CELL_PML;
-        if (pml) {
-            double m = std::numeric_limits<double>::min();
-            m = std::max(m, s->tab[0].csig[i]);
-            m = std::max(m, s->tab[1].csig[j]);
-            m = std::max(m, s->tab[2].csig[k]);
-            C.r_identity = -0.5 * m / s->pml_strength;
-        } else if (f & FDTD_CELL_BULK) {
-            C.r_identity = 0.5;
-        } else if (!(f & FDTD_CELL_GHOST)) {
-            C.r_identity = 1.0;
-        } else {
-            C.r_identity = -1.0;
-            C.n_gc_value = 6;
-        }
-        const double cp[3] = {s->tab[0].cpos[i], s->tab[1].cpos[j], s->tab[2].cpos[k]};
-        for (int d = 0; d < 3; ++d) {
-            C.centroid[d] = cp[d];
-            C.lower_corner[d] = cp[d] - s->h / 2.0;
-            C.upper_corner[d] = cp[d] + s->h / 2.0;
-        }
-        // ghost faces toward bulk neighbours; they hold zero until the first step computes them
-        const unsigned faces = C.n_gc_value ? (unsigned)(v.cls & CLS_MASK) : 0u;
-        for (int g = 0; g < 6; ++g)
-            C.gc_value[g] = ((faces >> g) & 1u) ? (s->step_index == 0 ? 0.0 : v.gc[g]) : -1.0;
-        for (int d = 0; d < 3; ++d) C.p_directional[d] = v.pdir[d];
-        C.p_full = v.p;
-        C.vx[0] = v.v[0], C.vx[1] = v.v[1];
-        C.vy[0] = v.v[2], C.vy[1] = v.v[3];
-        C.vz[0] = v.v[4], C.vz[1] = v.v[5];
-        if (!s->region.red) flags |= FDTD_CELLINFO_PML_STATE;
-        C.h = s->h;
-        if (s->step_index == 0) {
-            C.laplacian = 0.0;
-            flags |= FDTD_CELLINFO_LAPLACIAN;
-        } else if (visc && (phased || (!s->moving && !pml))) {
-            C.laplacian = v.lap;
-            flags |= FDTD_CELLINFO_LAPLACIAN;
-        } else {
-            C.laplacian = nan;
-        }
-        C.flags = flags;
-    }
-    return FDTD_OK;
+    FetchArgs F{};
+    F.dim = dim;
+    F.k = k;
+    F.cell = cell;
+    F.step_index = s->step_index;
+    F.pml_strength = s->pml_strength;
+    F.reduced = s->region.red != 0;
+    F.phased = s->opt.kernel == FDTD_KERNEL_PHASED;
+    F.moving = s->moving;
+    F.vbuf = F.phased ? 0 : s->cur;
+    for (int d = 0; d < 3; ++d) F.csig[d] = s->d_csig[d];
+    F.shell = s->shell;
+    s->launches += (total + (long long)(fdtd::READBACK_BYTES / sizeof(fdtd_cell)) - 1) /
+                   (long long)(fdtd::READBACK_BYTES / sizeof(fdtd_cell));
+    return read_back(s, total, sizeof(fdtd_cell), out, [&](long long first, long long n, void* buf) {
+        return launch_fetch_cells(s->dP, s->precision == FDTD_PRECISION_FP64, s->cur, F, first, (int)n, (fdtd_cell*)buf,
+                                  s->stream);
+    });
 }
 
 }  // namespace
@@ -948,11 +921,11 @@ fdtd_status fdtd_solver_get_field(fdtd_solver* s, int32_t which, double* out, in
     // the read-back stages the field in host memory
     if (s && fdtd::inject_failure(FDTD_INJECT_HOST_ALLOC))
         return (set_error(s, "host staging buffer of the field read-back: allocation failed"), FDTD_ERR_OOM);
-    return field_transfer(s, which, out, count, false);
+    return field_read(s, which, out, count);
 }
 
 fdtd_status fdtd_solver_set_field(fdtd_solver* s, int32_t which, const double* in, int64_t count) {
-    return field_transfer(s, which, const_cast<double*>(in), count, true);
+    return field_write(s, which, in, count);
 }
 
 fdtd_status fdtd_solver_domain(fdtd_solver* s, double min_bound[3], double max_bound[3]) {
@@ -968,7 +941,7 @@ fdtd_status fdtd_solver_fetch_cell(fdtd_solver* s, int64_t cell_index, fdtd_cell
     if (!s || !out) return FDTD_ERR_INVALID_ARG;
     if (cell_index < 0 || cell_index >= s->ncell)
         return (set_error(s, "cell_index out of range"), FDTD_ERR_INVALID_ARG);
-    return fetch_cells(s, std::vector<long long>{cell_index}, out);
+    return fetch_cells(s, -1, 0, cell_index, 1, out);
 }
 
 fdtd_status fdtd_solver_sample_slice(fdtd_solver* s, int32_t dim, double offset, fdtd_cell* out, int64_t capacity,
@@ -986,17 +959,7 @@ fdtd_status fdtd_solver_sample_slice(fdtd_solver* s, int32_t dim, double offset,
     if (!(r > -1.0) || !(r < 2147483647.0))
         return (set_error(s, "offset outside the grid along dim"), FDTD_ERR_INVALID_ARG);
     const int k = std::min((int)r, s->N[dim] - 1);
-    std::vector<long long> cells((size_t)n);
-    size_t c = 0;
-    for (int a = 0; a < s->N[d1]; ++a)
-        for (int b = 0; b < s->N[d2]; ++b) {
-            int idx[3];
-            idx[dim] = k;
-            idx[d1] = a;
-            idx[d2] = b;
-            cells[c++] = ((long long)idx[0] * s->N[1] + idx[1]) * s->N[2] + idx[2];
-        }
-    return fetch_cells(s, cells, out);
+    return fetch_cells(s, dim, k, 0, n, out);
 }
 
 // ---------------------------------------------------------------------------
