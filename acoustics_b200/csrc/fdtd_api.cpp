@@ -413,8 +413,8 @@ bool use_reduced_pml(const fdtd_solver* s, bool no_solid_pml) {
     return true;
 }
 
-// x planes per PML-shell thread: tile_y when given, else the default of the
-// solve's PML state.
+// x planes per PML-shell thread of a batch member: tile_y when given, else the
+// default of its PML state (the members fill the GPU together).
 int shell_planes(const fdtd_solver* s, int tile_y) {
     if (tile_y > 0) return std::min(tile_y, 256);
     return s->region.red ? FDTD_SHELL_RED_PLANES : FDTD_SHELL_PLANES;
@@ -477,6 +477,26 @@ void build_shell_boxes(fdtd_solver* s, int xs) {
     if (B.n > 0 && B.x0[B.n - 1] == lo[0] && B.y0[B.n - 1] == lo[1] && B.zb[B.n - 1] == hi[2]) {
         B.zbox = B.n - 1;
         B.zrw = (B.ng[B.zbox] + 1) * V;
+    }
+}
+
+// x planes per shell thread of a solve on its own, by how its CTAs fill the GPU (two per SM in
+// FP32, one in FP64).  A longer march reads less twice (the planes at its ends)
+// and a shorter one spreads over more SMs: FP32 takes 4 planes where 8 make
+// fewer than 1.6 waves of CTAs (us a step, 4 / 8: 144x120x112 17.0 / 21.3, 160^3
+// 25.5 / 30.4, 192x160x144 with 1.7 waves 30.9 / 29.5), FP64 16 where they still
+// make 3 waves (8 / 16: 192x160x144 58.2 / 59.6, 224^3 116.5 / 113.6, 256^3
+// 175.9 / 171.2).
+void choose_shell_planes(fdtd_solver* s) {
+    const bool f64 = s->precision == FDTD_PRECISION_FP64;
+    const int xs = shell_planes(s, s->opt.tile_y);
+    if (s->shell.xs != xs) build_shell_boxes(s, xs);
+    if (s->opt.tile_y > 0) return;
+    if (!f64) {
+        if (10 * s->shell.block_first[s->shell.n] < 16 * 2 * 148) build_shell_boxes(s, xs / 2);
+    } else {
+        build_shell_boxes(s, 2 * xs);
+        if (s->shell.block_first[s->shell.n] < 3 * 148) build_shell_boxes(s, xs);
     }
 }
 
@@ -1342,8 +1362,7 @@ fdtd_status fdtd_solver_reset(fdtd_solver* s, double t0) {
     }
     // default x planes per shell thread of the state in effect (tile_y overrides)
     if (s->opt.kernel == FDTD_KERNEL_FUSED) {
-        const int xs = shell_planes(s, s->opt.tile_y);
-        if (s->shell.xs != xs) build_shell_boxes(s, xs);
+        choose_shell_planes(s);
         s->region.shell = s->shell;
     }
     // the whole step in one launch: static scenes with a PML on every side, up to

@@ -29,9 +29,9 @@ cudaError_t launch_step_regions_fp32(const SolveParams* dP, const SolveParams& h
 
 #include "fdtd_one_launch.cuh"
 namespace fdtd {
-cudaError_t launch_one_fp32(const SolveParams* dP, const SolveParams& hP, const RegionLaunch& R, int cur, bool src,
+cudaError_t launch_one_fp32(const SolveParams* dP, const SolveParams& hP, const RegionLaunch& R, int cur,
                             int n_ghost, double* lis_row, cudaStream_t s, int* launches) {
-    return launch_one<float>(dP, hP, R, cur, src, n_ghost, lis_row, s, launches);
+    return launch_one<float>(dP, hP, R, cur, n_ghost, lis_row, s, launches);
 }
 }  // namespace fdtd
 

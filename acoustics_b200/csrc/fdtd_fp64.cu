@@ -1148,9 +1148,9 @@ cudaError_t launch_step_regions_fp64(const SolveParams* dP, const SolveParams& h
 
 #include "fdtd_one_launch.cuh"
 namespace fdtd {
-cudaError_t launch_one_fp64(const SolveParams* dP, const SolveParams& hP, const RegionLaunch& R, int cur, bool src,
+cudaError_t launch_one_fp64(const SolveParams* dP, const SolveParams& hP, const RegionLaunch& R, int cur,
                             int n_ghost, double* lis_row, cudaStream_t s, int* launches) {
-    return launch_one<double>(dP, hP, R, cur, src, n_ghost, lis_row, s, launches);
+    return launch_one<double>(dP, hP, R, cur, n_ghost, lis_row, s, launches);
 }
 long long one_launch_cells(int precision) { return precision == 0 ? FDTD_ONE_LAUNCH_CELLS_F64 : FDTD_ONE_LAUNCH_CELLS_F32; }
 }  // namespace fdtd

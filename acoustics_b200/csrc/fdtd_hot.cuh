@@ -241,6 +241,51 @@ __global__ void __launch_bounds__(256) k_interior(const KArgs<T> A, Box3 box) {
     interior_tile<T, XB, VISC>(A, box, blockIdx.x, blockIdx.y);
 }
 
+// While a source is active: the interior adds the sources to its own cells (and
+// k_ghost_cells to its own), instead of a kernel that waits for both (4-7 us at
+// the end of every step).  The thread goes over its cells in the supports' box
+// again once they are stored, as k_sources would: factors held beside the
+// stencil's registers spilled at four CTAs per SM.
+template <typename T>
+__device__ __forceinline__ void interior_sources(const KArgs<T>& A, const Box3& box, int tu, int tx, int xb,
+                                                 const SourceArgs& S) {
+    constexpr int V = 16 / (int)sizeof(T);
+    const Box3& r = S.region;
+    const int x0 = max(box.lo[0] + tx * xb, r.lo[0]), x1 = min(min(box.lo[0] + (tx + 1) * xb, box.hi[0]), r.hi[0]);
+    if (x0 >= x1) return;
+    const int ng = interior_groups_z(box, V);
+    const int u = tu * 256 + threadIdx.x + 32 * threadIdx.y;
+    const int row = u / ng, g = u - row * ng;
+    const int y = box.lo[1] + row;
+    if (y >= box.hi[1] || y < r.lo[1] || y >= r.hi[1]) return;
+    const int zc = box.lo[2] / V * V + g * V;
+    const int z0 = max(zc, r.lo[2]), z1 = min(zc + V, r.hi[2]);  // the region lies inside the box
+    if (z0 >= z1) return;
+    bool any = false;
+    for (int s = 0; s < S.n; ++s) any |= S.consts->src_tf[s] != 0.0;
+    if (!any) return;
+    for (int x = x0; x < x1; ++x)
+        for (int z = z0; z < z1; ++z) {
+            const unsigned c = (unsigned)x * A.sx + (unsigned)y * A.sy + z;
+            if ((A.cls[c] & (CLS_BULK | CLS_MASK)) != CLS_BULK) continue;
+            const double add = source_at(S, x, y, z) * S.k;
+            if constexpr (sizeof(T) == 8) {
+                A.pn[c] += add;
+            } else {
+                const float d = A.dinc[c] + (float)add;
+                A.dinc[c] = d;
+                A.pn[c] = A.pc[c] + d;
+            }
+        }
+}
+
+template <typename T, bool VISC = false>
+__global__ void __launch_bounds__(256) k_interior_src(const KArgs<T> A, const Box3 box,
+                                                      const __grid_constant__ SourceArgs S) {
+    interior_tile<T, 2, VISC>(A, box, blockIdx.x, blockIdx.y);
+    interior_sources<T>(A, box, blockIdx.x, blockIdx.y, 2, S);
+}
+
 // Masked store of a z vector: one vector store when every cell is selected,
 // else the selected cells one by one.
 template <typename T, int V>
@@ -641,6 +686,19 @@ __global__ void __launch_bounds__(256, shell_min_blocks(sizeof(T))) k_pml_shell(
 
 namespace fdtd {
 
+inline SourceArgs source_args(const SolveParams& hP, const RegionLaunch& R, int cur) {
+    SourceArgs S{};
+    S.region = R.src_region;
+    S.n = R.sources ? hP.n_src : 0;
+    for (int d = 0; d < 3; ++d) {
+        S.N[d] = hP.N[d];
+        S.ax[d] = hP.src_ax[d];
+    }
+    S.consts = hP.consts + cur;
+    S.k = hP.k;
+    return S;
+}
+
 // Host side: one region-split step (streams: StepStreams).  Launch order: the
 // ghost-cell list (s3), the interior (s2), the shell (s) (FP64: the shell before
 // the interior), then the sources (s2, after the interior and the ghost list,
@@ -673,6 +731,9 @@ cudaError_t launch_regions(const SolveParams* dP, const SolveParams& hP, const R
         if (e == cudaSuccess && gside) e = cudaStreamWaitEvent(S.s3, S.fork, 0);
         if (e != cudaSuccess) return e;
     }
+    // sources in the interior and ghost kernels (explicit x chunks keep k_sources)
+    const bool fuse_src = R.sources && has_interior && R.xb == 2;
+    const SourceArgs src = source_args(hP, R, cur);
     if (R.fc) {
         // FULLY_COUPLED: this step's ghost pressures, before the cells that read them
         if ((e = launch_fc<T>(dP, hP, cur, gside ? S.s3 : si, false, &l)) != cudaSuccess) return e;
@@ -680,7 +741,7 @@ cudaError_t launch_regions(const SolveParams* dP, const SolveParams& hP, const R
     if (has_ghost) {
         // cells next to a solid: disjoint from the interior and shell cells
         const int blocks = (R.ghost_cap + 127) / 128 < 1184 ? (R.ghost_cap + 127) / 128 : 1184;
-        k_ghost_cells<T><<<blocks, 128, 0, gside ? S.s3 : si>>>(dP, cur);
+        k_ghost_cells<T><<<blocks, 128, 0, gside ? S.s3 : si>>>(dP, cur, fuse_src ? src : SourceArgs{});
         ++l;
     }
     if (gside && (e = cudaEventRecord(S.ghost, S.s3)) != cudaSuccess) return e;
@@ -694,7 +755,9 @@ cudaError_t launch_regions(const SolveParams* dP, const SolveParams& hP, const R
             dim3 block(32, 8);
             const int xb = (!hP.visc && (R.xb == 4 || R.xb == 8)) ? R.xb : 2;
             dim3 grid(interior_unit_tiles(b, 16 / (int)sizeof(T)), (nx + xb - 1) / xb);
-            if (hP.visc) k_interior<T, 2, true><<<grid, block, 0, si>>>(A, b);
+            if (fuse_src && hP.visc) k_interior_src<T, true><<<grid, block, 0, si>>>(A, b, src);
+            else if (fuse_src) k_interior_src<T><<<grid, block, 0, si>>>(A, b, src);
+            else if (hP.visc) k_interior<T, 2, true><<<grid, block, 0, si>>>(A, b);
             else if (xb == 2) k_interior<T, 2><<<grid, block, 0, si>>>(A, b);
             else if (xb == 8) k_interior<T, 8><<<grid, block, 0, si>>>(A, b);
             else k_interior<T, 4><<<grid, block, 0, si>>>(A, b);
@@ -717,7 +780,7 @@ cudaError_t launch_regions(const SolveParams* dP, const SolveParams& hP, const R
     }
     if (shell_first) launch_interior();
     if (gside && (e = cudaStreamWaitEvent(S.s2, S.ghost, 0)) != cudaSuccess) return e;
-    if (R.sources) {
+    if (R.sources && !fuse_src) {
         // source cells are non-PML cells: after the interior and ghost updates of
         // their cells, concurrent with the shell
         const Box3& r = R.src_region;

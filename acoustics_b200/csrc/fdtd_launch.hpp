@@ -25,9 +25,9 @@ cudaError_t launch_step_regions_fp32(const SolveParams* dP, const SolveParams& h
 // a static solve's step in one launch (fdtd_one_launch.cuh): n_ghost cells of the
 // ghost-neighbour list (< 0: not known on the host), the listener row of the step
 // before to lis_row (null: none)
-cudaError_t launch_one_fp64(const SolveParams* dP, const SolveParams& hP, const RegionLaunch& R, int cur, bool src,
+cudaError_t launch_one_fp64(const SolveParams* dP, const SolveParams& hP, const RegionLaunch& R, int cur,
                             int n_ghost, double* lis_row, cudaStream_t s, int* launches);
-cudaError_t launch_one_fp32(const SolveParams* dP, const SolveParams& hP, const RegionLaunch& R, int cur, bool src,
+cudaError_t launch_one_fp32(const SolveParams* dP, const SolveParams& hP, const RegionLaunch& R, int cur,
                             int n_ghost, double* lis_row, cudaStream_t s, int* launches);
 // grid cells up to which a static solve steps that way
 long long one_launch_cells(int precision);

@@ -292,19 +292,19 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? FDTD_ONE_MINB_F32 : FDTD
 // Grid cells up to which a static solve steps by one launch: where the region-split
 // step with 16-step graphs takes as long (us a step, one launch / split; a sphere
 // and a box, one active source, 8 listeners, PML 8-10):
-//   FP32  64^3 5.8 / 13.8, 112^3 13.3 / 15.2, 144x120x112 17.9 / 20.9, 160^3 29.6 / 29.5
-//   FP64  64^3 8.0 / 14.0, 96^3 14.2 / 14.8, 112^3 20.3 / 17.5, 160^3 70.8 / 54.9
+//   FP32  64^3 5.8 / 13.8, 112^3 13.3 / 14.5, 144x120x112 17.9 / 17.0, 160^3 29.6 / 25.5
+//   FP64  64^3 8.0 / 14.0, 96^3 14.2 / 14.8, 112^3 20.3 / 17.4, 160^3 70.8 / 51.4
 // Past it a thread per PML cell moves more bytes than the marching shell, which
 // carries p and the low x face along.
 #ifndef FDTD_ONE_LAUNCH_CELLS_F32
-#define FDTD_ONE_LAUNCH_CELLS_F32 2500000
+#define FDTD_ONE_LAUNCH_CELLS_F32 1600000
 #endif
 #ifndef FDTD_ONE_LAUNCH_CELLS_F64
 #define FDTD_ONE_LAUNCH_CELLS_F64 1000000
 #endif
 
 template <typename T>
-cudaError_t launch_one(const SolveParams* dP, const SolveParams& hP, const RegionLaunch& R, int cur, bool src, int n_ghost,
+cudaError_t launch_one(const SolveParams* dP, const SolveParams& hP, const RegionLaunch& R, int cur, int n_ghost,
                        double* lis_row, cudaStream_t s, int* launches) {
     if (R.fc) {
         const cudaError_t e = launch_fc<T>(dP, hP, cur, s, true, launches);
@@ -332,14 +332,7 @@ cudaError_t launch_one(const SolveParams* dP, const SolveParams& hP, const Regio
     if (nx > 0 && L.int_tu > 0) blocks += L.int_tu * ((nx + 1) / 2);
     L.lis_first = blocks;
     if (lis_row && hP.n_lis > 0) blocks += (hP.n_lis + 7) / 8;
-    L.src.region = R.src_region;
-    L.src.n = src ? hP.n_src : 0;
-    for (int d = 0; d < 3; ++d) {
-        L.src.N[d] = hP.N[d];
-        L.src.ax[d] = hP.src_ax[d];
-    }
-    L.src.consts = hP.consts + cur;
-    L.src.k = hP.k;
+    L.src = source_args(hP, R, cur);
     L.plan = hP.ghost_plan;
     L.ghost_count = hP.ghost_count;
     L.plan_cap = hP.plan_ready ? hP.plan_cap : 0;

@@ -248,7 +248,8 @@ __device__ __forceinline__ void ghost_cell_planned(const GhostArgs<T>& A, const 
 
 // The cells of the ghost-neighbour list, by plan where there is one.
 template <typename T>
-__device__ __forceinline__ void ghost_cells_body(const SolveParams& P, int cur, int bid, int nblocks) {
+__device__ __forceinline__ void ghost_cells_body(const SolveParams& P, int cur, int bid, int nblocks,
+                                                 const SourceArgs* S = nullptr) {
     const int n = min(*P.ghost_count, P.ghost_cap);
     const int planned = P.plan_ready ? min(n, P.plan_cap) : 0;
     const int first = bid * blockDim.x + threadIdx.x, stride = nblocks * blockDim.x;
@@ -258,10 +259,26 @@ __device__ __forceinline__ void ghost_cells_body(const SolveParams& P, int cur, 
         for (int w = first & ~31; w < 4 * planned; w += stride) {
             const int g = (w + (int)(threadIdx.x & 31)) >> 2;
             ghost_cell_planned<T>(A, ghost_load(P.ghost_plan, min(g, planned - 1), threadIdx.x & 3), g < planned,
-                                  nullptr);
+                                  S);
         }
     }
-    for (int g = planned + first; g < n; g += stride) ghost_cell<T>(P, cur, P.ghost_list[g]);
+    for (int g = planned + first; g < n; g += stride) {
+        const long long c = P.ghost_list[g];
+        ghost_cell<T>(P, cur, c);
+        if (!S || S->n == 0) continue;
+        // (outside the supports' bounding box a source's factors are zero)
+        int x, y, z;
+        cell_ijk(P, c, x, y, z);
+        const double src = source_at(*S, x, y, z);
+        T* __restrict__ pn = (T*)P.p[cur ^ 1];
+        if constexpr (sizeof(T) == 8) {
+            pn[c] += src * S->k;
+        } else {
+            const float d = P.dinc[c] + (float)(src * S->k);
+            P.dinc[c] = d;
+            pn[c] = ((const T*)P.p[cur])[c] + d;
+        }
+    }
 }
 
 // Plans of the ghost-neighbour list of the current classification (static scenes).
@@ -348,8 +365,9 @@ __device__ __forceinline__ void sources_body(const SolveParams& P, int cur, cons
 }
 
 template <typename T>
-__global__ void __launch_bounds__(128) k_ghost_cells(const SolveParams* __restrict__ Pp, int cur) {
-    ghost_cells_body<T>(*Pp, cur, blockIdx.x, gridDim.x);
+__global__ void __launch_bounds__(128) k_ghost_cells(const SolveParams* __restrict__ Pp, int cur,
+                                                     const __grid_constant__ SourceArgs S) {
+    ghost_cells_body<T>(*Pp, cur, blockIdx.x, gridDim.x, &S);
 }
 
 template <typename T>

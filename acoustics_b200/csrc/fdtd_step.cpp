@@ -229,8 +229,8 @@ fdtd_status enqueue_step(fdtd_solver* s, int cur, double* dev_row, bool classify
     if (s->region.one) {
         int l = 0;
         cudaError_t e = s->precision == FDTD_PRECISION_FP64
-                            ? launch_one_fp64(s->dP, s->hP, s->region, cur, src, s->n_ghost, s->lag_row, s->stream, &l)
-                            : launch_one_fp32(s->dP, s->hP, s->region, cur, src, s->n_ghost, s->lag_row, s->stream, &l);
+                            ? launch_one_fp64(s->dP, s->hP, s->region, cur, s->n_ghost, s->lag_row, s->stream, &l)
+                            : launch_one_fp32(s->dP, s->hP, s->region, cur, s->n_ghost, s->lag_row, s->stream, &l);
         CUDA_TRY(s, e);
         s->launches += l;
         s->lag_row = nullptr;

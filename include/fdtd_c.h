@@ -176,7 +176,7 @@ typedef struct {
     int32_t device;           /* CUDA ordinal                                            */
     int32_t kernel;           /* FDTD_KERNEL_*                                           */
     int32_t graph_steps;      /* >0: capture this many steps per CUDA graph launch       */
-    int32_t tile_y;           /* fused path: x planes a PML-shell thread marches over; 0: 8   */
+    int32_t tile_y;           /* fused path: x planes a PML-shell thread marches over; 0: by size */
     int32_t x_chunk;          /* fused path: interior x planes per thread (2, 4, 8); 0: 2        */
     int32_t pml_state;        /* FDTD_PML_STATE_*                                        */
     int32_t shell_staging;    /* FDTD_SHELL_STAGING_*                                    */
