@@ -376,9 +376,10 @@ fdtd_status run_classification(fdtd_solver* s) {
     ClsBoxes& B = s->hP.boxes;
     classification_boxes(s, B);
     CUDA_TRY(s, fdtd::counted_copyAsync(s, &s->dP->boxes, &B, sizeof(ClsBoxes), cudaMemcpyHostToDevice, s->stream));
-    CUDA_TRY(s, launch_classify(s->dP, s->N, B, false, !s->mesh_alloc.empty(), s->stream));
+    int l = 0;  // (as by the step before the first one, whose parity is 0)
+    CUDA_TRY(s, launch_classify(s->dP, s->N, B, false, !s->mesh_alloc.empty(), 1, s->stream, &l));
     s->cls_boxes_current = true;
-    s->launches += B.ufirst[B.n] > 0 ? 3 : 2;
+    s->launches += l;
     return FDTD_OK;
 }
 
@@ -899,8 +900,11 @@ static void carve_arena(fdtd_solver* s, const fdtd_scene_desc* sc, const fdtd_op
         s->region.ghost_cap = (int)std::min<double>(cells, (double)n);
         cv.add((void**)&s->d_ghost_list, (size_t)s->region.ghost_cap * 4);
         cv.add((void**)&s->d_ghost_count, 16);
-        // plans of its cells: static scenes
-        P.plan_cap = (s->moving || o.kernel != FDTD_KERNEL_FUSED)
+        // plans of its cells: static scenes, and moving analytic bodies (k_cls_tiles)
+        bool mesh = false;
+        for (int i = 0; i < sc->n_objects; ++i) mesh = mesh || sc->objects[i].shape == FDTD_SHAPE_MESH;
+        P.plan_cap = (o.kernel != FDTD_KERNEL_FUSED ||
+                      (s->moving && (mesh || sc->boundary_handling != FDTD_BOUNDARY_RASTERIZE)))
                          ? 0
                          : std::min(s->region.ghost_cap, GHOST_PLAN_MAX);
         if (P.plan_cap > 0) cv.add((void**)&P.ghost_plan, (size_t)P.plan_cap * sizeof(GhostPlan));
@@ -1008,6 +1012,10 @@ fdtd_status fdtd_solver_create(const fdtd_scene_desc* sc, const fdtd_options* op
     CUDA_TRY(nullptr, cudaEventCreateWithFlags(&s->ev_lis[1], cudaEventDisableTiming));
     CUDA_TRY(nullptr, cudaEventCreateWithFlags(&s->ev_lis_join, cudaEventDisableTiming));
     CUDA_TRY(nullptr, cudaStreamCreateWithFlags(&s->stream5, cudaStreamNonBlocking));
+    if (any_moving) {
+        CUDA_TRY(nullptr, cudaStreamCreateWithFlags(&s->stream6, cudaStreamNonBlocking));
+        CUDA_TRY(nullptr, cudaEventCreateWithFlags(&s->ev_fdone, cudaEventDisableTiming));
+    }
     CUDA_TRY(nullptr, cudaEventCreateWithFlags(&s->ev_sfork, cudaEventDisableTiming));
     CUDA_TRY(nullptr, cudaEventCreateWithFlags(&s->ev_sdone, cudaEventDisableTiming));
     if (s->precision == FDTD_PRECISION_FP32_COMPENSATED) CUDA_TRY(nullptr, prepare_fp32_kernels());
@@ -1130,7 +1138,7 @@ fdtd_status fdtd_solver_create(const fdtd_scene_desc* sc, const fdtd_options* op
     P.ghost_list = s->d_ghost_list;
     P.ghost_count = s->d_ghost_count;
     P.ghost_cap = s->region.ghost_cap;
-    P.fresh_count = s->d_ghost_count + 1;
+    P.moving = s->moving ? 1 : 0;
     s->region.interior = update_box(s.get());
     P.eng_n = (int)s->eng.size();
     P.eng_lambda = s->c * s->k / s->h;  // MAC_Grid.cpp:488
@@ -1244,7 +1252,7 @@ fdtd_status fdtd_solver_destroy(fdtd_solver* s) {
     if (!s) return FDTD_OK;
     cudaSetDevice(s->opt.device);
     // (also releases a solver whose creation failed part way: null handles are skipped)
-    for (cudaStream_t st : {s->stream, s->stream2, s->stream3, s->stream4, s->stream5})
+    for (cudaStream_t st : {s->stream, s->stream2, s->stream3, s->stream4, s->stream5, s->stream6})
         if (st) cudaStreamSynchronize(st);
     for (int i = 0; i < 4; ++i)
         if (s->graph_exec[i]) cudaGraphExecDestroy(s->graph_exec[i]);
@@ -1258,9 +1266,9 @@ fdtd_status fdtd_solver_destroy(fdtd_solver* s) {
     for (cudaEvent_t ev : s->rb_done)
         if (ev) cudaEventDestroy(ev);
     for (cudaEvent_t ev : {s->ev_fork, s->ev_join, s->ev_ghost, s->ev_step, s->ev_lis[0], s->ev_lis[1], s->ev_lis_join,
-                           s->ev_sfork, s->ev_sdone})
+                           s->ev_sfork, s->ev_sdone, s->ev_fdone})
         if (ev) cudaEventDestroy(ev);
-    for (cudaStream_t st : {s->stream2, s->stream3, s->stream4, s->stream5, s->stream})
+    for (cudaStream_t st : {s->stream2, s->stream3, s->stream4, s->stream5, s->stream6, s->stream})
         if (st) cudaStreamDestroy(st);
     delete s;
     return FDTD_OK;

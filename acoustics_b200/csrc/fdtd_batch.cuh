@@ -131,7 +131,7 @@ template <typename T>
 __global__ void __launch_bounds__(128) k_batch_ghost(const BatchDesc<T>* __restrict__ D) {
     const BatchDesc<T>& d = D[blockIdx.y];
     if (!d.active || d.halted || d.ghost_cap == 0) return;
-    ghost_cells_body<T>(*d.P, d.cur, blockIdx.x, gridDim.x);
+    ghost_cells_body<T>(*d.P, d.cur, blockIdx.x, gridDim.x, d.P->plan_ready != 0);
 }
 
 // grid (src_blocks, members)

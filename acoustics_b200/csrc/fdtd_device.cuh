@@ -73,6 +73,8 @@ struct DevSource {
     double scale;        // (1/3.6836) * normalize constant
 };
 
+constexpr int CLS_MAX_BOXES_X = FDTD_MAX_OBJECTS + 4;  // CLS_MAX_BOXES
+
 // Non-PML box [lo, hi) of the grid.
 struct Box3 {
     int lo[3];
@@ -183,6 +185,13 @@ struct KArgs {
     int advance;                  // the shell kernel advances consts[cur^1]
 };
 
+// Ranges of x planes the interior kernel is restricted to.
+constexpr int MAX_X_RANGES = CLS_MAX_BOXES_X + 1;
+struct XRanges {
+    int n;                        // 0: the whole box
+    int lo[MAX_X_RANGES], hi[MAX_X_RANGES];
+};
+
 // Launch description of one region-split step.
 struct RegionLaunch {
     Box3 interior;
@@ -195,6 +204,7 @@ struct RegionLaunch {
     int red;           // FP32: the shell keeps the reduced PML state (k_pml_shell_red)
     int fc;            // FULLY_COUPLED ghost cells: solve their system before the ghost list
     int one;           // the whole step in one launch (k_step_one)
+    XRanges x;         // planes of the interior kernel
     const TmaStep* tma;  // reduced state: the TMA-staged shell (k_pml_shell_tma) when not null (host memory)
 };
 
@@ -339,14 +349,14 @@ struct SolveParams {
                                   // exp(-(x_d - c_d)^2 / 2w^2) inside the source box (the
                                   // x factor times the source scale), 0 outside
     int* ghost_list;              // non-PML bulk cells with a solid neighbour
-    int* ghost_count;
+    int* ghost_count;             // its cells and, next to it, the fresh cells (list_counts)
     int ghost_cap;
+    int moving;                   // some body moves
     GhostPlan* ghost_plan;        // [plan_cap] the list's cells prepared (static scenes)
     int plan_cap;
     int plan_ready;               // ghost_plan valid for the current classification
     ClsBoxes boxes;               // iteration boxes of the latest classification
     int* fresh_list;              // bulk cells without a valid history (found by the classification sweep)
-    int* fresh_count;             // may exceed fresh_cap: the fresh-cell kernel then sweeps every cell
     int fresh_cap;
     int precision;                // 0 fp64, 1 fp32 compensated
     // FULLY_COUPLED ghost cells (static scenes; null under RASTERIZE)
@@ -550,6 +560,15 @@ __host__ __device__ __forceinline__ void dense_ijk(const SolveParams& P, long lo
     const long long r = t - i * yz;
     j = (int)(r / P.N[2]);
     k = (int)(r - (long long)j * P.N[2]);
+}
+
+// Lengths of the ghost-neighbour list [0] and of the fresh-cell list [1] (which may
+// exceed fresh_cap: the fresh-cell kernel then sweeps every cell) of the
+// classification made in a step of parity cur.  Moving bodies: a pair per parity,
+// so that the classification of a step finds its own pair empty (the step before
+// emptied it) and empties the other.
+__device__ __forceinline__ int* list_counts(const SolveParams& P, int cur) {
+    return P.ghost_count + (P.moving ? 2 * cur : 0);
 }
 
 // Some Gaussian source contributes at the step of parity `cur` (its time

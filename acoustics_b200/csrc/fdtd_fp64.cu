@@ -90,10 +90,7 @@ __device__ __forceinline__ void cls_box_cell(const SolveParams& P, long long c, 
 __global__ void __launch_bounds__(128) k_cls_boxes(const SolveParams* __restrict__ Pp) {
     const SolveParams& P = *Pp;
     const ClsBoxes& B = P.boxes;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        *P.ghost_count = 0;
-        *P.fresh_count = 0;
-    }
+    if (blockIdx.x == 0 && threadIdx.x < 4) P.ghost_count[threadIdx.x] = 0;
     const long long total = B.first[B.n];
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
          t += (long long)gridDim.x * blockDim.x) {
@@ -141,10 +138,7 @@ __global__ void __launch_bounds__(32 * CLS_MESH_WARPS, 3) k_cls_boxes_mesh(const
     __shared__ double near_d[32], centre_d;
     const SolveParams& P = *Pp;
     const ClsBoxes& B = P.boxes;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        *P.ghost_count = 0;
-        *P.fresh_count = 0;
-    }
+    if (blockIdx.x == 0 && threadIdx.x < 4) P.ghost_count[threadIdx.x] = 0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int* stack = stacks[warp];
     const double h = P.h, reach = sample_reach(P);
@@ -264,7 +258,7 @@ __global__ void __launch_bounds__(32 * CLS_MESH_WARPS, 3) k_cls_boxes_mesh(const
 // call it together are taken with one atomic per list (an atomic per cell on
 // one counter serialises thousands of cells a step); the lists are unordered.
 __device__ __noinline__ void cls_cells(const SolveParams& P, const ClsQuad q, uint32_t sel, uint32_t code,
-                                       uint32_t listed, uint32_t fresh) {
+                                       uint32_t listed, uint32_t fresh, int cur) {
     namespace cg = cooperative_groups;
     uint32_t to_list = 0, to_fresh = 0;  // bytes (bulk bit) of this quad's cells for each list
     while (sel) {
@@ -289,8 +283,9 @@ __device__ __noinline__ void cls_cells(const SolveParams& P, const ClsQuad q, ui
     const int tl = g.shfl(pl + nl, g.size() - 1), tf = g.shfl(pf + nf, g.size() - 1);
     int bl = 0, bf = 0;
     if (g.thread_rank() == 0) {
-        if (tl) bl = atomicAdd(P.ghost_count, tl);
-        if (tf) bf = atomicAdd(P.fresh_count, tf);
+        int* counts = list_counts(P, cur);
+        if (tl) bl = atomicAdd(counts, tl);
+        if (tf) bf = atomicAdd(counts + 1, tf);
     }
     int sl = g.shfl(bl, 0) + pl, sf = g.shfl(bf, 0) + pf;
     while (to_list) {
@@ -323,7 +318,8 @@ __device__ __forceinline__ uint32_t quad_bulk(const SolveParams& P, const ClsBox
 // Laplacian.  Mask bit 2d + (s > 0) is set where the
 // neighbour in direction s along axis d exists and differs in bulk-ness; the
 // four cells are compared at once, byte by byte of the words.
-__device__ __noinline__ void cls_sweep_near(const SolveParams& P, const ClsQuad q, uint32_t own, int collect_fresh) {
+__device__ __noinline__ void cls_sweep_near(const SolveParams& P, const ClsQuad q, uint32_t own, int collect_fresh,
+                                            int cur) {
     const ClsBoxes& B = P.boxes;
     const uint32_t cells = quad_cells(q.nk);
     const uint32_t inb = box_bytes(B, q.i, q.j, q.k0);
@@ -361,15 +357,16 @@ __device__ __noinline__ void cls_sweep_near(const SolveParams& P, const ClsQuad 
     const uint32_t listed = bulk & masked;
     const uint32_t fresh = collect_fresh ? bulk & ~((base & QUAD_VALID) << 1) : 0u;
     const uint32_t sel = ghost | listed | fresh;
-    if (sel) cls_cells(P, q, sel, base, listed, fresh);
+    if (sel) cls_cells(P, q, sel, base, listed, fresh, cur);
     const uint32_t out = ((base | mask) & cells) | (own & ~cells);
     if (out != own) *(uint32_t*)(P.cls + q.c0) = out;
 }
 
 // One quad of the sweep with its word `own`.
-__device__ __forceinline__ void cls_sweep_quad(const SolveParams& P, const ClsQuad& q, uint32_t own, int collect_fresh) {
+__device__ __forceinline__ void cls_sweep_quad(const SolveParams& P, const ClsQuad& q, uint32_t own, int collect_fresh,
+                                               int cur) {
     if (quad_near(P.boxes, q)) {
-        cls_sweep_near(P, q, own, collect_fresh);
+        cls_sweep_near(P, q, own, collect_fresh, cur);
         return;
     }
     // no solid cell within one cell: bulk, history from the last step, no mask
@@ -378,7 +375,7 @@ __device__ __forceinline__ void cls_sweep_quad(const SolveParams& P, const ClsQu
     if (out != own) {
         *(uint32_t*)(P.cls + q.c0) = out;
         const uint32_t fresh = collect_fresh ? ~own & QUAD_BULK & cells : 0u;
-        if (fresh) cls_cells(P, q, fresh, out, 0u, fresh);
+        if (fresh) cls_cells(P, q, fresh, out, 0u, fresh, cur);
     }
 }
 
@@ -396,7 +393,7 @@ __device__ __forceinline__ bool unit_in(const ClsBoxes& B, int b, int i, int j, 
 constexpr int CLS_UNITS = 8;
 
 __global__ void __launch_bounds__(256) k_cls_sweep(const SolveParams* __restrict__ Pp, int nunits, int chunks,
-                                                   int collect_fresh) {
+                                                   int collect_fresh, int cur) {
     const SolveParams& P = *Pp;
     const ClsBoxes& B = P.boxes;
     const int lane = threadIdx.x & 31;
@@ -460,7 +457,7 @@ __global__ void __launch_bounds__(256) k_cls_sweep(const SolveParams* __restrict
         while (fresh) {
             const int m = (__ffsll((long long)fresh) - 1) >> 3;
             fresh &= ~(0xFFull << (8 * m));
-            const int slot = atomicAdd(P.fresh_count, 1);
+            const int slot = atomicAdd(list_counts(P, cur) + 1, 1);
             if (slot < P.fresh_cap) P.fresh_list[slot] = (int)(c + m);
         }
     }
@@ -473,7 +470,7 @@ __global__ void __launch_bounds__(256) k_cls_sweep(const SolveParams* __restrict
 // reach), so the full sweep would write nothing there.  One warp per unit,
 // every unit once; units a box of this step reaches are left to k_cls_near.
 __global__ void __launch_bounds__(256) k_cls_sweep_prev(const SolveParams* __restrict__ Pp, const ClsBoxes prev,
-                                                        int collect_fresh) {
+                                                        int collect_fresh, int cur) {
     const SolveParams& P = *Pp;
     const ClsBoxes& B = P.boxes;
     const int lane = threadIdx.x & 31;
@@ -506,7 +503,7 @@ __global__ void __launch_bounds__(256) k_cls_sweep_prev(const SolveParams* __res
         while (fresh) {
             const int m = (__ffsll((long long)fresh) - 1) >> 3;
             fresh &= ~(0xFFull << (8 * m));
-            const int slot = atomicAdd(P.fresh_count, 1);
+            const int slot = atomicAdd(list_counts(P, cur) + 1, 1);
             if (slot < P.fresh_cap) P.fresh_list[slot] = (int)(c + m);
         }
     }
@@ -514,7 +511,7 @@ __global__ void __launch_bounds__(256) k_cls_sweep_prev(const SolveParams* __res
 
 // Units some box reaches, one warp each, every unit once (in the first box
 // that reaches it); a lane takes two quads.
-__global__ void __launch_bounds__(256) k_cls_near(const SolveParams* __restrict__ Pp, int collect_fresh) {
+__global__ void __launch_bounds__(256) k_cls_near(const SolveParams* __restrict__ Pp, int collect_fresh, int cur) {
     const SolveParams& P = *Pp;
     const ClsBoxes& B = P.boxes;
     const int lane = threadIdx.x & 31;
@@ -543,7 +540,164 @@ __global__ void __launch_bounds__(256) k_cls_near(const SolveParams* __restrict_
         q.k0 = k0;
         q.nk = min(4, P.N[2] - k0);
         q.c0 = (long long)i * P.SX + (long long)j * P.SY + k0;
-        cls_sweep_quad(P, q, *(const uint32_t*)(P.cls + q.c0), collect_fresh);
+        cls_sweep_quad(P, q, *(const uint32_t*)(P.cls + q.c0), collect_fresh, cur);
+    }
+}
+
+// A moving-body step's classification of analytic bodies in one launch.  The
+// kernels above meet twice (the sweep reads the boxes' new flags), each a chain of
+// its own of a few hundred cells' work: 12 + 4 + 22 us of a step in front of the
+// fresh cells.  Here a CTA takes a tile of 2 x 4 x 32 cells of the region a body's
+// boxes of this step and the one before reach (outside it every cell keeps the
+// default flags) and makes the new bulk bits of the tile and of one cell around it
+// itself, in shared memory: an analytic distance costs less than a launch.  Flags,
+// objects and lists are those of the kernels above; the listed cells get their
+// plans here too (GhostPlan).  384x384x256, two spheres of 25 cells: 28 us
+// (4 x 8 x 32 tiles, 56 CTAs: 47 us).
+constexpr int CLS_T0 = 2, CLS_T1 = 4, CLS_T2 = 32;
+struct ClsTiles {
+    int n;
+    int lo[CLS_MAX_BOXES][3], hi[CLS_MAX_BOXES][3];  // region of each box, clipped to the grid
+    int nt[CLS_MAX_BOXES][3];
+    int first[CLS_MAX_BOXES + 1];
+};
+
+// The regions: hull of a box and the same body's box of the step before, and the
+// cells around it (whose masks the box's cells decide).
+static ClsTiles cls_tiles(const int N[3], const ClsBoxes& B, const ClsBoxes& prev) {
+    static const int T[3] = {CLS_T0, CLS_T1, CLS_T2};
+    ClsTiles R{};
+    R.n = B.n;
+    for (int b = 0; b < B.n; ++b) {
+        const bool now = B.first[b + 1] > B.first[b], before = b < prev.n && prev.first[b + 1] > prev.first[b];
+        int tiles = 1;
+        for (int d = 0; d < 3; ++d) {
+            int lo = now ? B.lo[b][d] : prev.lo[b][d], hi = now ? lo + B.rg[b][d] : lo + prev.rg[b][d];
+            if (now && before) {
+                lo = std::min(lo, prev.lo[b][d]);
+                hi = std::max(hi, prev.lo[b][d] + prev.rg[b][d]);
+            }
+            R.lo[b][d] = std::max(0, lo - 1);
+            R.hi[b][d] = now || before ? std::min(N[d], hi + 1) : R.lo[b][d];
+            R.nt[b][d] = (std::max(0, R.hi[b][d] - R.lo[b][d]) + T[d] - 1) / T[d];
+            tiles *= R.nt[b][d];
+        }
+        R.first[b + 1] = R.first[b] + tiles;
+    }
+    return R;
+}
+
+__global__ void __launch_bounds__(256) k_cls_tiles(const SolveParams* __restrict__ Pp, const __grid_constant__ ClsTiles R,
+                                                   int cur) {
+    constexpr int H1 = CLS_T1 + 2, H2 = CLS_T2 + 2, CELLS = (CLS_T0 + 2) * H1 * H2;
+    enum : uint8_t { SOLID = 0, BULK = 1, NONE = 2, CONSTRAINT = 4 };
+    __shared__ uint8_t made[CELLS];
+    const SolveParams& P = *Pp;
+    const ClsBoxes& B = P.boxes;
+    if (blockIdx.x == 0 && threadIdx.x < 2) list_counts(P, cur ^ 1)[threadIdx.x] = 0;
+    const int t = (int)blockIdx.x;
+    int b = 0;
+    while (b < R.n && t >= R.first[b + 1]) ++b;
+    if (b >= R.n) return;
+    const int r = t - R.first[b];
+    const int i0 = R.lo[b][0] + CLS_T0 * (r / (R.nt[b][1] * R.nt[b][2]));
+    const int j0 = R.lo[b][1] + CLS_T1 * ((r / R.nt[b][2]) % R.nt[b][1]);
+    const int k0 = R.lo[b][2] + CLS_T2 * (r % R.nt[b][2]);
+    for (int q = threadIdx.x; q < CELLS; q += 256) {
+        const int i = i0 - 1 + q / (H1 * H2), j = j0 - 1 + (q / H2) % H1, k = k0 - 1 + q % H2;
+        uint8_t m = NONE;
+        if (i >= 0 && i < P.N[0] && j >= 0 && j < P.N[1] && k >= 0 && k < P.N[2]) {
+            bool in = false;
+            for (int e = 0; e < B.n && !in; ++e) in = in_box(B, e, i, j, k);
+            m = BULK;
+            if (in) {
+                const double pos[3] = {P.cpos[0][i], P.cpos[1][j], P.cpos[2][k]};
+                int type = 0;
+                if (!is_fluid(P, pos, type)) m = (uint8_t)(SOLID | (type ? CONSTRAINT : 0));
+            }
+        }
+        made[q] = m;
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    int* counts = list_counts(P, cur);
+    for (int q = threadIdx.x; q < CLS_T0 * CLS_T1 * CLS_T2; q += 256) {  // whole warps
+        const int di = q / (CLS_T1 * CLS_T2), dj = (q / CLS_T2) % CLS_T1, dk = q % CLS_T2;
+        const int i = i0 + di, j = j0 + dj, k = k0 + dk;
+        bool on = i < R.hi[b][0] && j < R.hi[b][1] && k < R.hi[b][2];
+        // each cell in the first region that holds it
+        for (int e = 0; e < b && on; ++e)
+            on = !(i >= R.lo[e][0] && i < R.hi[e][0] && j >= R.lo[e][1] && j < R.hi[e][1] && k >= R.lo[e][2] &&
+                   k < R.hi[e][2]);
+        bool to_list = false, to_fresh = false;
+        long long c = 0;
+        unsigned mask = 0;
+        uint8_t out = 0;
+        if (on) {
+            c = cidx(P, i, j, k);
+            const int a = ((di + 1) * H1 + dj + 1) * H2 + dk + 1;
+            const uint8_t own = made[a];
+            const bool bulk = own & BULK;
+            // directions whose neighbour exists and differs
+            auto differs = [&](int n) { return made[n] != NONE && ((made[n] ^ own) & BULK) ? 1u : 0u; };
+            mask = differs(a - H1 * H2) | differs(a + H1 * H2) << 1 | differs(a - H2) << 2 |
+                                  differs(a + H2) << 3 | differs(a - 1) << 4 | differs(a + 1) << 5;
+            const uint8_t old = P.cls[c];
+            const bool valid = old & CLS_BULK;
+            out = (uint8_t)((bulk ? CLS_BULK : 0) | (valid ? CLS_VALID : 0) | mask);
+            if (out != old) P.cls[c] = out;
+            if (!bulk) {
+                uint8_t g = (own & CONSTRAINT) ? GOBJ_CONSTRAINT : 0;
+                if (mask) {  // a ghost cell: its closest object
+                    const double pos[3] = {P.cpos[0][i], P.cpos[1][j], P.cpos[2][k]};
+                    const int o = lowest_object(P, pos);
+                    g = g | (uint8_t)(o < 0 ? GOBJ_NONE : o);
+                }
+                P.gobj[c] = g;
+                if (P.precision == 0) {
+                    ((double*)P.p[0])[c] = 0.0;
+                    ((double*)P.p[1])[c] = 0.0;
+                } else {
+                    ((float*)P.p[0])[c] = 0.0f;
+                    ((float*)P.p[1])[c] = 0.0f;
+                    P.dinc[c] = 0.0f;
+                }
+            } else {
+                to_list = mask && !(P.pml_cell[0][i] || P.pml_cell[1][j] || P.pml_cell[2][k]);
+                to_fresh = !valid;
+            }
+        }
+        // the lists (unordered): an atomic per warp
+        const unsigned ml = __ballot_sync(0xffffffffu, to_list), mf = __ballot_sync(0xffffffffu, to_fresh);
+        const unsigned below = (1u << lane) - 1u;
+        int bl = 0, bf = 0;
+        if (lane == 0) {
+            if (ml) bl = atomicAdd(counts, __popc(ml));
+            if (mf) bf = atomicAdd(counts + 1, __popc(mf));
+        }
+        bl = __shfl_sync(0xffffffffu, bl, 0) + __popc(ml & below);
+        bf = __shfl_sync(0xffffffffu, bf, 0) + __popc(mf & below);
+        if (to_list && bl < P.ghost_cap) {
+            P.ghost_list[bl] = (int)c;
+            if (bl < P.plan_cap) {
+                const int idx[3] = {i, j, k};
+                GhostPlan G = empty_plan((int)c, out, idx);
+                const int a = ((di + 1) * H1 + dj + 1) * H2 + dk + 1;
+                const int step[3] = {H1 * H2, H2, 1};
+                for (int f = 0; f < 6; ++f) {
+                    if (!((mask >> f) & 1u)) continue;
+                    const int d = f >> 1, s = f & 1;
+                    if (made[a + (s ? step[d] : -step[d])] & CONSTRAINT) continue;
+                    // the solid neighbour's closest object
+                    double pos[3] = {P.cpos[0][i], P.cpos[1][j], P.cpos[2][k]};
+                    pos[d] = P.cpos[d][idx[d] + (s ? 1 : -1)];
+                    const int o = lowest_object(P, pos);
+                    if (o >= 0) plan_face(P, G, idx, d, s, (unsigned)o);
+                }
+                P.ghost_plan[bl] = G;
+            }
+        }
+        if (to_fresh && bf < P.fresh_cap) P.fresh_list[bf] = (int)c;
     }
 }
 
@@ -853,7 +1007,7 @@ __global__ void __launch_bounds__(128) k_fresh_cells(const SolveParams* __restri
                                                      int* status) {
     const SolveParams& P = *Pp;
     const double t = P.consts[cur].t;
-    const int count = *P.fresh_count;
+    const int count = list_counts(P, cur)[1];
     int st = 0;
     if (count > P.fresh_cap) {
         for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n;
@@ -1064,7 +1218,15 @@ cudaError_t launch_static_prep(SolveParams* dP, int precision, int newp, int n_l
 }
 
 cudaError_t launch_classify(const SolveParams* dP, const int N[3], const ClsBoxes& B, bool collect_fresh, bool meshes,
-                            cudaStream_t s, const ClsBoxes* prev) {
+                            int cur, cudaStream_t s, int* launches, const ClsBoxes* prev) {
+    const int fresh = collect_fresh ? 1 : 0;
+    if (prev && !meshes) {
+        const ClsTiles T = cls_tiles(N, B, *prev);
+        if (launches) *launches += 1;
+        k_cls_tiles<<<(unsigned)std::max(T.first[T.n], 1), 256, 0, s>>>(dP, T, cur);
+        return cudaGetLastError();
+    }
+    if (launches) *launches += B.ufirst[B.n] > 0 ? 3 : 2;
     if (meshes) {
         long long bricks = 1;  // (one CTA at least: it empties the lists)
         for (int b = 0; b < B.n; ++b) bricks += cls_bricks(B, b);
@@ -1075,15 +1237,15 @@ cudaError_t launch_classify(const SolveParams* dP, const int N[3], const ClsBoxe
     if (prev) {
         const long long units = prev->ufirst[prev->n];
         if (units > 0)
-            k_cls_sweep_prev<<<(unsigned)std::min<long long>((units + 7) / 8, 148 * 16), 256, 0, s>>>(
-                dP, *prev, collect_fresh ? 1 : 0);
+            k_cls_sweep_prev<<<(unsigned)std::min<long long>((units + 7) / 8, 148 * 16), 256, 0, s>>>(dP, *prev, fresh,
+                                                                                                     cur);
     } else {
         const int chunks = (N[2] + CLS_CHUNK - 1) / CLS_CHUNK;
         const int nunits = N[0] * N[1] * chunks;
         const int warps = (nunits + CLS_UNITS - 1) / CLS_UNITS;
-        k_cls_sweep<<<(warps + 7) / 8, 256, 0, s>>>(dP, nunits, chunks, collect_fresh ? 1 : 0);
+        k_cls_sweep<<<(warps + 7) / 8, 256, 0, s>>>(dP, nunits, chunks, fresh, cur);
     }
-    if (B.ufirst[B.n] > 0) k_cls_near<<<grid_for((2 * B.ufirst[B.n] + 7) / 8, 1), 256, 0, s>>>(dP, collect_fresh ? 1 : 0);
+    if (B.ufirst[B.n] > 0) k_cls_near<<<grid_for((2 * B.ufirst[B.n] + 7) / 8, 1), 256, 0, s>>>(dP, fresh, cur);
     return cudaGetLastError();
 }
 

@@ -686,6 +686,20 @@ __global__ void __launch_bounds__(256, shell_min_blocks(sizeof(T))) k_pml_shell(
 
 namespace fdtd {
 
+// The interior of some x planes only (XRanges): x tiles count through the ranges.
+template <typename T, bool SRC>
+__global__ void __launch_bounds__(256) k_interior_planes(const KArgs<T> A, const Box3 box,
+                                                         const __grid_constant__ XRanges X,
+                                                         const __grid_constant__ SourceArgs S) {
+    int tx = blockIdx.y, q = 0;
+    while (q + 1 < X.n && tx >= (X.hi[q] - X.lo[q] + 1) / 2) tx -= (X.hi[q] - X.lo[q] + 1) / 2, ++q;
+    Box3 b = box;
+    b.lo[0] = X.lo[q];
+    b.hi[0] = X.hi[q];
+    interior_tile<T, 2>(A, b, blockIdx.x, tx);
+    if constexpr (SRC) interior_sources<T>(A, b, blockIdx.x, tx, 2, S);
+}
+
 inline SourceArgs source_args(const SolveParams& hP, const RegionLaunch& R, int cur) {
     SourceArgs S{};
     S.region = R.src_region;
@@ -741,7 +755,7 @@ cudaError_t launch_regions(const SolveParams* dP, const SolveParams& hP, const R
     if (has_ghost) {
         // cells next to a solid: disjoint from the interior and shell cells
         const int blocks = (R.ghost_cap + 127) / 128 < 1184 ? (R.ghost_cap + 127) / 128 : 1184;
-        k_ghost_cells<T><<<blocks, 128, 0, gside ? S.s3 : si>>>(dP, cur, fuse_src ? src : SourceArgs{});
+        k_ghost_cells<T><<<blocks, 128, 0, gside ? S.s3 : si>>>(dP, cur, hP.plan_ready != 0, fuse_src ? src : SourceArgs{});
         ++l;
     }
     if (gside && (e = cudaEventRecord(S.ghost, S.s3)) != cudaSuccess) return e;
@@ -755,7 +769,14 @@ cudaError_t launch_regions(const SolveParams* dP, const SolveParams& hP, const R
             dim3 block(32, 8);
             const int xb = (!hP.visc && (R.xb == 4 || R.xb == 8)) ? R.xb : 2;
             dim3 grid(interior_unit_tiles(b, 16 / (int)sizeof(T)), (nx + xb - 1) / xb);
-            if (fuse_src && hP.visc) k_interior_src<T, true><<<grid, block, 0, si>>>(A, b, src);
+            if (R.x.n > 0) {
+                // (x ranges come with the default planes per thread and no viscosity)
+                unsigned tiles = 0;
+                for (int q = 0; q < R.x.n; ++q) tiles += (unsigned)(R.x.hi[q] - R.x.lo[q] + 1) / 2;
+                grid.y = tiles;
+                if (fuse_src) k_interior_planes<T, true><<<grid, block, 0, si>>>(A, b, R.x, src);
+                else k_interior_planes<T, false><<<grid, block, 0, si>>>(A, b, R.x, src);
+            } else if (fuse_src && hP.visc) k_interior_src<T, true><<<grid, block, 0, si>>>(A, b, src);
             else if (fuse_src) k_interior_src<T><<<grid, block, 0, si>>>(A, b, src);
             else if (hP.visc) k_interior<T, 2, true><<<grid, block, 0, si>>>(A, b);
             else if (xb == 2) k_interior<T, 2><<<grid, block, 0, si>>>(A, b);

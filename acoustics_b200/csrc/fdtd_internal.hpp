@@ -76,6 +76,9 @@ struct fdtd_solver {
     // beside that step's classification
     cudaStream_t stream5 = nullptr;
     cudaEvent_t ev_sfork = nullptr, ev_sdone = nullptr;
+    // and the interior planes out of the bodies' reach on stream6 (planes_ahead)
+    cudaStream_t stream6 = nullptr;
+    cudaEvent_t ev_fdone = nullptr;
     // hP.boxes are the boxes of the classification the cell flags hold (the
     // solid cells lie in them); cleared when the flags are loaded from elsewhere
     bool cls_boxes_current = false;

@@ -248,10 +248,10 @@ __device__ __forceinline__ void ghost_cell_planned(const GhostArgs<T>& A, const 
 
 // The cells of the ghost-neighbour list, by plan where there is one.
 template <typename T>
-__device__ __forceinline__ void ghost_cells_body(const SolveParams& P, int cur, int bid, int nblocks,
+__device__ __forceinline__ void ghost_cells_body(const SolveParams& P, int cur, int bid, int nblocks, bool plans,
                                                  const SourceArgs* S = nullptr) {
-    const int n = min(*P.ghost_count, P.ghost_cap);
-    const int planned = P.plan_ready ? min(n, P.plan_cap) : 0;
+    const int n = min(list_counts(P, cur)[0], P.ghost_cap);
+    const int planned = plans ? min(n, P.plan_cap) : 0;
     const int first = bid * blockDim.x + threadIdx.x, stride = nblocks * blockDim.x;
     if (planned > 0) {
         const GhostArgs<T> A = ghost_args<T>(P, cur);
@@ -281,54 +281,59 @@ __device__ __forceinline__ void ghost_cells_body(const SolveParams& P, int cur, 
     }
 }
 
+// Face (d, s) of a plan: toward the solid cell idx + (s ? 1 : -1) e_d, whose
+// closest object is o (GHOST_STILL: none, or a constraint).
+__device__ __forceinline__ void plan_face(const SolveParams& P, GhostPlan& G, const int idx[3], int d, int s, unsigned o) {
+    if (o >= (unsigned)P.n_obj || P.obj[o].accel_kind == 0) return;
+    const int sgn = s ? 1 : -1;
+    // the face a quarter cell from the solid cell's centre (ghost_pressure)
+    double pos[3] = {P.cpos[0][idx[0]], P.cpos[1][idx[1]], P.cpos[2][idx[2]]};
+    pos[d] = P.cpos[d][idx[d] + sgn];
+    pos[d] += (sgn > 0 ? -1.0 : 1.0) * 0.25 * P.h;
+    const DevObject& O = P.obj[o];
+    if (O.accel_kind == 1) {
+        G.u[d][s] = O.dir[d];
+    } else {
+        const double r0 = pos[0] - O.c[0], r1 = pos[1] - O.c[1], r2 = pos[2] - O.c[2];
+        const double len = sqrt(r0 * r0 + r1 * r1 + r2 * r2);
+        const double r[3] = {r0, r1, r2};
+        G.u[d][s] = len > 0.0 ? r[d] / len : 0.0;
+    }
+    G.obj[2 * d + s] = (uint8_t)o;
+}
+__device__ __forceinline__ GhostPlan empty_plan(int c, uint8_t code, const int idx[3]) {
+    GhostPlan G{};
+    G.c = c;
+    G.code = code;
+    for (int f = 0; f < 6; ++f) G.obj[f] = GHOST_STILL;
+    for (int d = 0; d < 3; ++d) G.ijk[d] = (uint16_t)idx[d];
+    return G;
+}
+
 // Plans of the ghost-neighbour list of the current classification (static scenes).
 static __global__ void __launch_bounds__(128) k_ghost_prep(const SolveParams* __restrict__ Pp) {
     const SolveParams& P = *Pp;
     const int n = min(min(*P.ghost_count, P.ghost_cap), P.plan_cap);
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
-        GhostPlan G;
-        G.c = P.ghost_list[q];
+        const int c = P.ghost_list[q];
         int idx[3];
-        cell_ijk(P, G.c, idx[0], idx[1], idx[2]);
-        G.code = P.cls[G.c];
-        G.pad[0] = G.pad[1] = 0;
-        G.pad1 = 0;
-        G.pad2[0] = G.pad2[1] = 0;
+        cell_ijk(P, c, idx[0], idx[1], idx[2]);
+        GhostPlan G = empty_plan(c, P.cls[c], idx);
         const long long strides[3] = {P.SX, P.SY, 1};
-        for (int d = 0; d < 3; ++d) {
-            G.ijk[d] = (uint16_t)idx[d];
-            for (int s = 0; s < 2; ++s) {
-                const int f = 2 * d + s;
-                G.obj[f] = GHOST_STILL;
-                G.u[d][s] = 0.0;
-                if (!((G.code >> f) & 1u)) continue;
-                const int sgn = s ? 1 : -1;
-                if (P.fc_rows) {
-                    const int row = fc_row(P, G.c + sgn * strides[d], 2 * d + (s ? 0 : 1));
-                    if (row >= 0) {  // (else, which classification rules out, the cell's own pressure)
-                        G.obj[f] = GHOST_COUPLED;
-                        G.u[d][s] = (double)row;
-                    }
-                    continue;
+        for (int f = 0; f < 6; ++f) {
+            if (!((G.code >> f) & 1u)) continue;
+            const int d = f >> 1, s = f & 1;
+            const long long nb = c + (s ? 1 : -1) * strides[d];
+            if (P.fc_rows) {
+                const int row = fc_row(P, nb, 2 * d + (s ? 0 : 1));
+                if (row >= 0) {  // (else, which classification rules out, the cell's own pressure)
+                    G.obj[f] = GHOST_COUPLED;
+                    G.u[d][s] = (double)row;
                 }
-                const unsigned gobj = P.gobj[G.c + sgn * strides[d]];
-                const unsigned o = gobj & 0x7F;
-                if ((gobj & GOBJ_CONSTRAINT) || o >= (unsigned)P.n_obj || P.obj[o].accel_kind == 0) continue;
-                // the face a quarter cell from the solid cell's centre (ghost_pressure)
-                double pos[3] = {P.cpos[0][idx[0]], P.cpos[1][idx[1]], P.cpos[2][idx[2]]};
-                pos[d] = P.cpos[d][idx[d] + sgn];
-                pos[d] += (sgn > 0 ? -1.0 : 1.0) * 0.25 * P.h;
-                const DevObject& O = P.obj[o];
-                if (O.accel_kind == 1) {
-                    G.u[d][s] = O.dir[d];
-                } else {
-                    const double r0 = pos[0] - O.c[0], r1 = pos[1] - O.c[1], r2 = pos[2] - O.c[2];
-                    const double len = sqrt(r0 * r0 + r1 * r1 + r2 * r2);
-                    const double r[3] = {r0, r1, r2};
-                    G.u[d][s] = len > 0.0 ? r[d] / len : 0.0;
-                }
-                G.obj[f] = (uint8_t)o;
+                continue;
             }
+            const unsigned gobj = P.gobj[nb];
+            if (!(gobj & GOBJ_CONSTRAINT)) plan_face(P, G, idx, d, s, gobj & 0x7F);
         }
         P.ghost_plan[q] = G;
     }
@@ -366,8 +371,8 @@ __device__ __forceinline__ void sources_body(const SolveParams& P, int cur, cons
 
 template <typename T>
 __global__ void __launch_bounds__(128) k_ghost_cells(const SolveParams* __restrict__ Pp, int cur,
-                                                     const __grid_constant__ SourceArgs S) {
-    ghost_cells_body<T>(*Pp, cur, blockIdx.x, gridDim.x, &S);
+                                                     bool plans, const __grid_constant__ SourceArgs S) {
+    ghost_cells_body<T>(*Pp, cur, blockIdx.x, gridDim.x, plans, &S);
 }
 
 template <typename T>

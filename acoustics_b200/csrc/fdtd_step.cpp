@@ -31,12 +31,13 @@ using namespace fdtd;
 namespace {
 
 // Classification over the boxes already in s->hP.boxes.
-void classification_launches(fdtd_solver* s, fdtd_status& st, const ClsBoxes* prev) {
+void classification_launches(fdtd_solver* s, int cur, fdtd_status& st, const ClsBoxes* prev) {
     const ClsBoxes& B = s->hP.boxes;
     // pageable source: the copy is staged before the call returns
     cudaError_t e = fdtd::counted_copyAsync(s, &s->dP->boxes, &B, sizeof(ClsBoxes), cudaMemcpyHostToDevice, s->stream);
-    if (e == cudaSuccess) e = launch_classify(s->dP, s->N, B, s->moving, !s->mesh_alloc.empty(), s->stream, prev);
-    s->launches += B.ufirst[B.n] > 0 ? 3 : 2;
+    int l = 0;
+    if (e == cudaSuccess) e = launch_classify(s->dP, s->N, B, s->moving, !s->mesh_alloc.empty(), cur, s->stream, &l, prev);
+    s->launches += l;
     if (e != cudaSuccess) {
         set_error(s, std::string("classification launch: ") + cudaGetErrorString(e));
         st = FDTD_ERR_CUDA;
@@ -133,6 +134,50 @@ fdtd_status join_listeners(fdtd_solver* s) {
     return FDTD_OK;
 }
 
+// The interior's x planes by their distance from the boxes of this step's and the
+// last step's classification: `near` those within PLANES_REACH, `far` the others;
+// both empty when the far ones are too few to start apart.  The classification
+// touches cells one beyond a box, a fresh cell lies in the last step's box and its
+// fit reads p^n and p^{n-1} at most three cells from it, and the cells of both are
+// read one cell further.
+// Only where the interior is long enough to hide the classification behind and the
+// shell leaves it room (us a step, together / apart; two spheres):
+//   FP32  96^3 56.9 / 57.0, 160x150x170 66.7 / 62.9, 256^3 112.6 / 105.5,
+//         320x320x256 140.3 / 131.5, 384x384x256 172.0 / 169.8
+//   FP64 (a shell CTA leaves one interior CTA's registers, which run beside it
+//         anyway)  224x200x210 120.2 / 122.6, 256^3 158.7 / 167.2
+constexpr int PLANES_REACH = 6;
+constexpr long long PLANES_CELLS = 2000000;
+void planes_ahead(const fdtd_solver* s, const ClsBoxes& prev, XRanges& far, XRanges& near) {
+    if (s->precision == FDTD_PRECISION_FP64 || s->n_interior < PLANES_CELLS) return;
+    const int lo = s->region.interior.lo[0], hi = s->region.interior.hi[0];
+    if (hi <= lo) return;
+    std::vector<char> reach(hi - lo, 0);
+    for (const ClsBoxes* B : {&prev, &s->hP.boxes})
+        for (int b = 0; b < B->n; ++b) {
+            if (B->first[b + 1] == B->first[b]) continue;
+            const int a = std::max(lo, B->lo[b][0] - PLANES_REACH);
+            const int e = std::min(hi, B->lo[b][0] + B->rg[b][0] + PLANES_REACH);
+            for (int x = a; x < e; ++x) reach[x - lo] = 1;
+        }
+    auto push = [](XRanges& X, int a, int e) {
+        X.lo[X.n] = a;
+        X.hi[X.n++] = e;
+    };
+    int n_far = 0;
+    for (int x = lo; x < hi;) {
+        int e = x;
+        while (e < hi && reach[e - lo] == reach[x - lo]) ++e;
+        if (!reach[x - lo]) n_far += e - x;
+        XRanges& X = reach[x - lo] ? near : far;
+        if (X.n == MAX_X_RANGES) n_far = -hi;  // (cannot be: a range per box at most, and one more)
+        else push(X, x, e);
+        x = e;
+    }
+    // (no near plane: nothing waits for the classification, and a range is needed to say so)
+    if (4 * n_far < hi - lo || near.n == 0) far.n = near.n = 0;
+}
+
 // The row a one-launch step left to its successor; newp: the parity of the
 // current pressure.
 fdtd_status flush_lag(fdtd_solver* s, int newp) {
@@ -164,6 +209,7 @@ fdtd_status enqueue_step(fdtd_solver* s, int cur, double* dev_row, bool classify
     }
     const bool fused = s->opt.kernel == FDTD_KERNEL_FUSED;
     bool shell_ahead = false;
+    XRanges near{};  // interior planes left to this step's classification (n = 0: all)
     if (classify) {
         // MAC_Grid::classifyCells_FAST + InterpolateFreshPressureCell (PML_WaveSolver.cpp:807-812)
         const ClsBoxes prev = s->hP.boxes;
@@ -179,32 +225,54 @@ fdtd_status enqueue_step(fdtd_solver* s, int cur, double* dev_row, bool classify
             set_error(s, "a moving body came within two cells of the PML of a reduced-state solve (past its end_time)");
             return FDTD_ERR_UNSUPPORTED;
         }
+        // Interior planes out of reach of the bodies' boxes hold no cell the
+        // classification or the fresh cells touch or read: they start first, on
+        // stream6, beside both.
+        XRanges far{};
+        if (s->moving && fused && s->cls_boxes_current && !s->hP.visc && s->eng.empty() && s->stream6 &&
+            s->boundary_handling == FDTD_BOUNDARY_RASTERIZE && s->region.xb == 2)
+            planes_ahead(s, prev, far, near);
         // Moving bodies clear of the PML: the shell kernel reads nothing the
-        // classification writes, so it starts first, on stream5, beside it.
+        // classification writes, so it starts first too.
         shell_ahead = s->moving && fused && s->cls_boxes_current && s->n_solid_pml == 0 && !s->hP.visc &&
                       s->eng.empty() &&
                       s->stream5 && s->interior.hi[0] > s->interior.lo[0] && boxes_clear_of_shell(s, prev) &&
                       boxes_clear_of_shell(s, s->hP.boxes);
-        if (shell_ahead) {
-            RegionLaunch R = s->region;
-            R.skip |= 1 | 4;  // the shell only
-            R.sources = 0;
-            R.fc = 0;
-            const StepStreams S5{s->stream5, nullptr, nullptr, s->ev_fork, s->ev_join, s->ev_ghost};
+        if (shell_ahead || far.n > 0) {
             CUDA_TRY(s, cudaEventRecord(s->ev_sfork, s->stream));
-            CUDA_TRY(s, cudaStreamWaitEvent(s->stream5, s->ev_sfork, 0));
-            int l = 0;
-            if (s->precision == FDTD_PRECISION_FP64)
-                CUDA_TRY(s, launch_step_regions_fp64(s->dP, s->hP, R, cur, S5, &l));
-            else
-                CUDA_TRY(s, launch_step_regions_fp32(s->dP, s->hP, R, cur, S5, &l));
-            s->launches += l;
-            s->overlapped_steps++;
-            CUDA_TRY(s, cudaEventRecord(s->ev_sdone, s->stream5));
+            const auto ahead = [&](cudaStream_t on, cudaEvent_t done, int skip, const XRanges& planes) -> fdtd_status {
+                RegionLaunch R = s->region;
+                R.skip |= 4 | skip;  // no ghost list
+                R.x = planes;
+                if (skip & 1) R.sources = 0;
+                R.fc = 0;
+                const StepStreams S{on, nullptr, nullptr, s->ev_fork, s->ev_join, s->ev_ghost};
+                CUDA_TRY(s, cudaStreamWaitEvent(on, s->ev_sfork, 0));
+                int l = 0;
+                if (s->precision == FDTD_PRECISION_FP64)
+                    CUDA_TRY(s, launch_step_regions_fp64(s->dP, s->hP, R, cur, S, &l));
+                else
+                    CUDA_TRY(s, launch_step_regions_fp32(s->dP, s->hP, R, cur, S, &l));
+                s->launches += l;
+                CUDA_TRY(s, cudaEventRecord(done, on));
+                return FDTD_OK;
+            };
+            // (the interior first: its CTAs are short, so the classification's find room sooner)
+            if (far.n > 0) {
+                const fdtd_status fst = ahead(s->stream6, s->ev_fdone, 2, far);
+                if (fst != FDTD_OK) return fst;
+            }
+            if (shell_ahead) {
+                const fdtd_status sst = ahead(s->stream5, s->ev_sdone, 1, XRanges{});
+                if (sst != FDTD_OK) return sst;
+                s->overlapped_steps++;
+            }
         }
         // moving bodies after a classification of the step before: only the units
         // its boxes reached can hold flags other than the defaults
-        classification_launches(s, st, (s->moving && s->cls_boxes_current) ? &prev : nullptr);
+        classification_launches(s, cur, st, (s->moving && s->cls_boxes_current) ? &prev : nullptr);
+        // (the one-launch classification of analytic bodies makes the ghost list's plans)
+        if (s->moving) s->hP.plan_ready = s->cls_boxes_current && s->hP.plan_cap > 0;
         s->cls_boxes_current = true;
         if (st != FDTD_OK) return st;
         if (s->moving) {
@@ -249,6 +317,7 @@ fdtd_status enqueue_step(fdtd_solver* s, int cur, double* dev_row, bool classify
     // advance the constants of a grid without PML cells
     RegionLaunch R = s->region;
     if (shell_ahead) R.skip |= 2;
+    R.x = near;
     const bool no_shell = R.shell.block_first[R.shell.n] == 0;
     const int advance = (!fused || no_shell) ? 1 : 0;
     if (s->precision == FDTD_PRECISION_FP64) {
@@ -273,6 +342,7 @@ fdtd_status enqueue_step(fdtd_solver* s, int cur, double* dev_row, bool classify
         s->launches += l;
     }
     if (shell_ahead) CUDA_TRY(s, cudaStreamWaitEvent(s->stream, s->ev_sdone, 0));
+    if (near.n > 0) CUDA_TRY(s, cudaStreamWaitEvent(s->stream, s->ev_fdone, 0));
     if (s->L > 0 && dev_row) {
         // the phased path keeps p^{n+1} in the same slot as the fused one
         if (listeners_aside(s, classify)) {
@@ -316,8 +386,9 @@ fdtd_status check_device_errors(fdtd_solver* s) {
     CUDA_TRY(s, fdtd::counted_copyAsync(s, &dev_error, s->hP.dev_error, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
     CUDA_TRY(s, fdtd::counted_copyAsync(s, status, s->d_status, sizeof(status), cudaMemcpyDeviceToHost, s->stream));
     CUDA_TRY(s, cudaStreamSynchronize(s->stream));
-    int ghosts = 0;
-    CUDA_TRY(s, fdtd::counted_copy(s, &ghosts, s->d_ghost_count, sizeof(int), cudaMemcpyDeviceToHost));
+    int counts[4] = {0, 0, 0, 0};  // list_counts
+    CUDA_TRY(s, fdtd::counted_copy(s, counts, s->d_ghost_count, sizeof(counts), cudaMemcpyDeviceToHost));
+    const int ghosts = s->moving ? std::max(counts[0], counts[2]) : counts[0];
     if (!s->moving) s->n_ghost = ghosts;
     if (ghosts > s->region.ghost_cap) {
         set_error(s, "ghost-neighbour list overflow (" + std::to_string(ghosts) + " > " +
