@@ -433,18 +433,21 @@ void build_shell_boxes(fdtd_solver* s, int xs) {
     const int* lo = s->interior.lo;
     const int* hi = s->interior.hi;
     auto groups = [&](int z0, int z1) { return z1 > z0 ? (z1 - 1) / V - z0 / V + 1 : 0; };
-    auto add = [&](int x0, int x1, int y0, int y1, int za0, int za1, int zb0, int zb1, bool zp = false) {
+    auto add = [&](int x0, int x1, int y0, int y1, int za0, int za1, int zb0, int zb1, int zp0 = 0, int zp1 = 0) {
         const int nz = (za1 - za0) + (zb1 - zb0);
         if (x1 <= x0 || y1 <= y0 || nz <= 0) return;
         const int b = B.n;
-        B.zp[b] = zp ? 1 : 0;
         B.x0[b] = x0; B.nx[b] = x1 - x0;
         B.y0[b] = y0; B.ny[b] = y1 - y0;
         B.za[b] = za0; B.zae[b] = za1; B.zb[b] = zb0; B.zbe[b] = zb1;
         B.gl[b] = groups(za0, za1);
         B.ng[b] = B.gl[b] + groups(zb0, zb1);
-        B.tu[b] = (B.ny[b] * B.ng[b] + 255) / 256;
-        B.tx[b] = (B.nx[b] + xs - 1) / xs;
+        const int plain = zp1 > zp0 ? (zp1 - zp0) / V : 0;
+        B.ge[b] = B.ng[b] - plain;
+        B.e0[b] = plain ? zp0 / V : 0;
+        B.tu[b] = ((plain ? (B.ny[b] * B.ge[b] + 31) / 32 * 32 : B.ny[b] * B.ge[b]) + B.ny[b] * plain + 255) / 256;
+        B.px[b] = (B.nx[b] + (B.nx[b] + xs - 1) / xs - 1) / ((B.nx[b] + xs - 1) / xs);
+        B.tx[b] = (B.nx[b] + B.px[b] - 1) / B.px[b];
         B.block_first[b + 1] = B.block_first[b] + B.tu[b] * B.tx[b];
         B.cells += (long long)B.nx[b] * B.ny[b] * nz;
         ++B.n;
@@ -453,21 +456,18 @@ void build_shell_boxes(fdtd_solver* s, int xs) {
         add(0, N[0], 0, N[1], 0, N[2], N[2], N[2]);  // every cell is a PML cell
         return;
     }
-    // FP32: each x / y slab as two boxes, the vector groups that hold a z-PML
-    // cell and those that are whole and outside the z PML, so the reduced-state
-    // kernel runs the plain-z columns of a CTA on one specialised path (shell
-    // 52.0 -> 48.9 us at 256^3, 22.8 -> 20.5 us at 192^3); short rows keep one
-    // box (more boxes of few units leave partial tiles: a batch of 48-160 cell
-    // grids lost 1.4 %)
+    // FP32: of each x / y slab row, the vector groups that are whole and outside
+    // the z PML apart from the others, so that the reduced-state kernel runs whole
+    // warps of them on a path without z masks (52.0 -> 48.9 us at 256^3).  Rows
+    // with few of them stay in one piece, where the warps of the others, gathered,
+    // would be the longest (cubes of 88 / 104 / 120 / 136 cells, 16 planes a
+    // thread, apart: 12.4 -> 11.4, 12.4 -> 11.3, 12.4 -> 11.2, 12.9 -> 15.3 us; 4
+    // planes: 7.5 -> 8.3, 7.2 -> 8.1, 9.5 -> 8.1, 11.4 -> 10.0; batches gain 1-4 %
+    // from 88 on, and one of eight solves of 48-100 cells loses 5 % from 64 on)
     const int zs0 = (lo[2] + V - 1) / V * V, zs1 = hi[2] / V * V;
-    const bool split = s->precision != FDTD_PRECISION_FP64 && zs1 - zs0 >= 128;
+    const bool split = s->precision != FDTD_PRECISION_FP64 && zs1 - zs0 >= 88;
     auto slab = [&](int x0, int x1, int y0, int y1) {
-        if (split) {
-            add(x0, x1, y0, y1, 0, zs0, zs1, N[2]);
-            add(x0, x1, y0, y1, zs0, zs1, zs1, zs1, true);
-        } else {
-            add(x0, x1, y0, y1, 0, N[2], N[2], N[2]);
-        }
+        add(x0, x1, y0, y1, 0, N[2], N[2], N[2], split ? zs0 : 0, split ? zs1 : 0);
     };
     slab(0, lo[0], 0, N[1]);
     slab(hi[0], N[0], 0, N[1]);

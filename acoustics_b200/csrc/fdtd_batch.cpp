@@ -49,11 +49,11 @@ struct fdtd_batch {
     int precision = 0;
     cudaStream_t stream = nullptr, stream2 = nullptr, stream3 = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_ghost = nullptr;
-    // listener rows of a step run on stream4 beside the next step; the advance of
-    // the next step (and with it every later kernel) waits on ev_lis[table of the step]
+    // stream4, beside the field kernels of a step: the listener rows of the step
+    // before, then the step's own advance (ev_adv: both done)
     cudaStream_t stream4 = nullptr;
-    cudaEvent_t ev_step = nullptr, ev_lis[2] = {nullptr, nullptr}, ev_lis_join = nullptr;
-    bool lis_pending[2] = {false, false};
+    cudaEvent_t ev_step = nullptr, ev_adv = nullptr, ev_lis_join = nullptr;
+    bool lis_pending = false;  // rows launched on stream4 that the batch stream has not waited for
     // some member's listener stencil may hold a ghost cell, whose rows also read
     // p^n in the buffer the next step writes: rows on the batch stream, before it
     bool rows_inline = false;
@@ -167,6 +167,7 @@ int fill_int_params(std::vector<char>& buf, const char* table, size_t dsz, const
         M.lap_scale = A.lap_scale;
         M.kcalp = A.kcalp;
         M.box = d.interior;
+        M.src = d.src_region;
         M.tu = list[i].tu;
         M.member = list[i].m;
         P.first[i] = ctas;
@@ -298,24 +299,31 @@ fdtd_status enqueue(fdtd_batch* b) {
     L.descs_other = static_cast<char*>(b->d_descs) + (p ^ 1) * b->table_bytes;
     b->flip ^= 1;
     const StepStreams SS{b->stream, b->stream2, b->stream3, b->ev_fork, b->ev_join, b->ev_ghost};
-    cudaError_t e = b->precision == FDTD_PRECISION_FP64
-                        ? launch_batch_fp64(L, SS, &l)
-                        : launch_batch_fp32(L, SS, &l);
-    // listener rows of this step beside the next step
-    const bool rows = L.n_refs > 0 && !b->rows_inline;
-    if (e == cudaSuccess && b->rows_inline && L.n_refs > 0) e = launch_batch_listeners_any(b->precision, L, b->stream, &l);
-    if (e == cudaSuccess && rows) e = cudaEventRecord(b->ev_step, b->stream);
-    if (e == cudaSuccess && rows) e = cudaStreamWaitEvent(b->stream4, b->ev_step, 0);
-    if (e == cudaSuccess && rows) e = launch_batch_listeners_any(b->precision, L, b->stream4, &l);
-    if (e == cudaSuccess && rows) e = cudaEventRecord(b->ev_lis[p], b->stream4);
-    // the rows of the step before read the pressure the next step overwrites and
-    // the table this step's advance marks halted members in
-    if (e == cudaSuccess && b->lis_pending[p ^ 1]) {
-        e = cudaStreamWaitEvent(b->stream, b->ev_lis[p ^ 1], 0);
-        b->lis_pending[p ^ 1] = false;
+    cudaError_t e = cudaSuccess;
+    // The advance reads this step's constants and writes the next step's, and
+    // marks halted members in the next step's table: no field kernel of this step
+    // reads either, so it runs beside them, after the rows of the step before
+    // (which read that table).  Pending rows already wait for the step before.
+    if (!b->lis_pending) {
+        e = cudaEventRecord(b->ev_step, b->stream);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(b->stream4, b->ev_step, 0);
     }
-    if (rows) b->lis_pending[p] = true;
-    if (e == cudaSuccess) e = launch_batch_advance_any(b->precision, L, b->stream, &l);
+    if (e == cudaSuccess) e = launch_batch_advance_any(b->precision, L, b->stream4, &l);
+    if (e == cudaSuccess) e = cudaEventRecord(b->ev_adv, b->stream4);
+    if (e == cudaSuccess)
+        e = b->precision == FDTD_PRECISION_FP64 ? launch_batch_fp64(L, SS, &l) : launch_batch_fp32(L, SS, &l);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(b->stream, b->ev_adv, 0);
+    b->lis_pending = false;
+    if (e == cudaSuccess && L.n_refs > 0) {
+        if (b->rows_inline) {
+            e = launch_batch_listeners_any(b->precision, L, b->stream, &l);
+        } else {
+            e = cudaEventRecord(b->ev_step, b->stream);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(b->stream4, b->ev_step, 0);
+            if (e == cudaSuccess) e = launch_batch_listeners_any(b->precision, L, b->stream4, &l);
+            b->lis_pending = true;
+        }
+    }
     b->launches += l;
     if (e != cudaSuccess) return batch_fail(b, FDTD_ERR_CUDA, std::string("batch launch: ") + cudaGetErrorString(e));
     return FDTD_OK;
@@ -323,10 +331,10 @@ fdtd_status enqueue(fdtd_batch* b) {
 
 // Make the batch stream wait for every listener launch on stream4.
 fdtd_status join_listeners(fdtd_batch* b) {
-    if (!b->lis_pending[0] && !b->lis_pending[1]) return FDTD_OK;
+    if (!b->lis_pending) return FDTD_OK;
     BATCH_TRY(b, cudaEventRecord(b->ev_lis_join, b->stream4));
     BATCH_TRY(b, cudaStreamWaitEvent(b->stream, b->ev_lis_join, 0));
-    b->lis_pending[0] = b->lis_pending[1] = false;
+    b->lis_pending = false;
     return FDTD_OK;
 }
 
@@ -340,7 +348,7 @@ fdtd_status capture(fdtd_batch* b, int n) {
     const long long l0 = b->launches;
     for (int i = 0; i < n && st == FDTD_OK; ++i) st = enqueue(b);
     if (st == FDTD_OK) st = join_listeners(b);  // the graph ends with every row written
-    b->lis_pending[0] = b->lis_pending[1] = false;
+    b->lis_pending = false;
     cudaError_t e = cudaStreamEndCapture(b->stream, &g);
     b->graph_launches = b->launches - l0;
     b->launches = l0;
@@ -401,8 +409,7 @@ fdtd_status fdtd_batch_create(int32_t n, const fdtd_scene_desc* scenes, const in
     BATCH_TRY(nullptr, cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming));
     BATCH_TRY(nullptr, cudaStreamCreateWithFlags(&b->stream4, cudaStreamNonBlocking));
     BATCH_TRY(nullptr, cudaEventCreateWithFlags(&b->ev_step, cudaEventDisableTiming));
-    BATCH_TRY(nullptr, cudaEventCreateWithFlags(&b->ev_lis[0], cudaEventDisableTiming));
-    BATCH_TRY(nullptr, cudaEventCreateWithFlags(&b->ev_lis[1], cudaEventDisableTiming));
+    BATCH_TRY(nullptr, cudaEventCreateWithFlags(&b->ev_adv, cudaEventDisableTiming));
     BATCH_TRY(nullptr, cudaEventCreateWithFlags(&b->ev_lis_join, cudaEventDisableTiming));
     for (int i = 0; i < n; ++i) {
         int32_t id;
@@ -682,7 +689,7 @@ fdtd_status fdtd_batch_destroy(fdtd_batch* b) {
     if (b->ev_fork) cudaEventDestroy(b->ev_fork);
     if (b->ev_join) cudaEventDestroy(b->ev_join);
     if (b->ev_ghost) cudaEventDestroy(b->ev_ghost);
-    for (cudaEvent_t ev : {b->ev_step, b->ev_lis[0], b->ev_lis[1], b->ev_lis_join})
+    for (cudaEvent_t ev : {b->ev_step, b->ev_adv, b->ev_lis_join})
         if (ev) cudaEventDestroy(ev);
     if (b->stream4) cudaStreamDestroy(b->stream4);
     if (b->stream2) cudaStreamDestroy(b->stream2);

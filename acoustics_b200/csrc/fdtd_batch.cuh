@@ -7,11 +7,16 @@
 // constants live on the device, a captured graph of an even number of batched
 // steps replays for any step index.
 //
-// Per step:  k_batch_ghost (third stream)  ||  k_batch_interior (second stream)
-//            ||  k_batch_shell_red / k_batch_shell (PML tiles of the members with
-//            the reduced / full PML state), then k_batch_sources (second
-//            stream, after the ghost list), then k_batch_advance; the listener
-//            rows (k_batch_listeners) on a fourth stream beside the next step.
+// Per step, side by side:
+//            k_batch_shell_red / k_batch_shell (PML tiles of the members with the
+//            reduced / full PML state);
+//            k_batch_interior (second stream) and k_batch_ghost (third stream),
+//            which add the sources to their cells (else k_batch_sources after both);
+//            k_batch_listeners of the step before, then k_batch_advance (fourth
+//            stream).
+// The step is as long as its field kernels: the sources and the advance as
+// kernels after them made it 74.9 us instead of 71.6 (12 solves of 48-128 cells a
+// side, FP32), 25.3 instead of 22.5 (two), 114 instead of 107 (100 of 24-44).
 // The descriptors come in two tables, one per step parity (every member's
 // parity flips each step), so consecutive steps alternate tables and no kernel
 // flips parities on the device.
@@ -30,6 +35,12 @@ namespace fdtd {
 #ifndef FDTD_BATCH_INT_TILES
 #define FDTD_BATCH_INT_TILES 4
 #endif
+
+// the sources of a member's step (of constant parity d.cur)
+template <typename T>
+__device__ __forceinline__ SourceArgs member_sources(const BatchDesc<T>& d) {
+    return source_args(*d.P, d.src_region, d.P->n_src, d.cur);
+}
 
 // The tile-table interior (more members than the parameter-bank table holds):
 // FDTD_BATCH_INT_TILES consecutive tiles per CTA.  The tiles are sorted by
@@ -78,9 +89,11 @@ __global__ void __launch_bounds__(256, XB == 2 ? 4 : 1)
         else hi = mid - 1;
     }
     const BatchIntMember<T>& M = P.m[lo];
-    if (D[M.member].halted) return;
+    const BatchDesc<T>& d = D[M.member];
+    if (d.halted) return;
     const int local = blk - P.first[lo];
     interior_tile<T, XB>(M, M.box, local % M.tu, local / M.tu);
+    interior_sources<T>(M, M.box, local % M.tu, local / M.tu, XB, M.src, [&]() { return member_sources(d); });
 }
 
 // One CTA per shell tile of the tables (all members in one launch).  The
@@ -128,10 +141,11 @@ __global__ void __launch_bounds__(256) k_batch_solid_pml(const BatchDesc<T>* __r
 
 // grid (ghost_blocks, members)
 template <typename T>
-__global__ void __launch_bounds__(128) k_batch_ghost(const BatchDesc<T>* __restrict__ D) {
+__global__ void __launch_bounds__(128) k_batch_ghost(const BatchDesc<T>* __restrict__ D, bool add_sources) {
     const BatchDesc<T>& d = D[blockIdx.y];
     if (!d.active || d.halted || d.ghost_cap == 0) return;
-    ghost_cells_body<T>(*d.P, d.cur, blockIdx.x, gridDim.x, d.P->plan_ready != 0);
+    const SourceArgs src = add_sources ? member_sources(d) : SourceArgs{};
+    ghost_cells_body<T>(*d.P, d.cur, blockIdx.x, gridDim.x, d.P->plan_ready != 0, &src);
 }
 
 // grid (src_blocks, members)
@@ -177,11 +191,32 @@ cudaError_t launch_batch(const BatchLaunch& L, const StepStreams& S, int* launch
     if (e == cudaSuccess) e = cudaStreamWaitEvent(S.s2, S.fork, 0);
     if (e == cudaSuccess && gside) e = cudaStreamWaitEvent(S.s3, S.fork, 0);
     if (e != cudaSuccess) return e;
+    // the sources by the interior's and the ghost list's threads, or by
+    // k_batch_sources after them: the tile-table interior's few CTAs took too long
+    // over a support's cells (200 solves of 24-44 cells: 21.6 -> 74 us,
+    // k_batch_sources 38 us)
+    const bool fuse_src = L.int_params && L.int_ctas > 0;
     if (L.ghost_blocks > 0) {
         // first: a few latency-bound CTAs that run beside the interior's
-        k_batch_ghost<T><<<dim3(L.ghost_blocks, L.n_members), 128, 0, gside ? S.s3 : S.s2>>>(D);
+        k_batch_ghost<T><<<dim3(L.ghost_blocks, L.n_members), 128, 0, gside ? S.s3 : S.s2>>>(D, fuse_src);
         ++l;
         if (gside && (e = cudaEventRecord(S.ghost, S.s3)) != cudaSuccess) return e;
+    }
+    // The shell first: a CTA of it takes half an SM's registers, and the interior's
+    // CTAs then fill what its last waves leave (12 solves of 48-128 cells a side,
+    // FP32, 6.6 M cells: 72.3 us a step with the interior first, 67.7 so; 32 of
+    // them 176 / 172; FP64 146 / 134 and 347 / 335).
+    int n_red = 0;
+    if constexpr (sizeof(T) == 4) {
+        n_red = L.n_shell_red;
+        if (n_red > 0) {
+            k_batch_shell_red<float><<<n_red, dim3(32, 8), red_smem_bytes(), S.s>>>(D, L.shell_tiles);
+            ++l;
+        }
+    }
+    if (L.n_shell > n_red) {
+        k_batch_shell<T><<<L.n_shell - n_red, dim3(32, 8), shell_smem_bytes<T>(), S.s>>>(D, L.shell_tiles + n_red);
+        ++l;
     }
     if (L.int_params && L.int_ctas > 0) {
         const dim3 block(32, 8);
@@ -198,20 +233,8 @@ cudaError_t launch_batch(const BatchLaunch& L, const StepStreams& S, int* launch
         else k_batch_interior<T, 4><<<grid, block, 0, S.s2>>>(D, L.int_tiles, L.n_int);
         ++l;
     }
-    int n_red = 0;
-    if constexpr (sizeof(T) == 4) {
-        n_red = L.n_shell_red;
-        if (n_red > 0) {
-            k_batch_shell_red<float><<<n_red, dim3(32, 8), red_smem_bytes(), S.s>>>(D, L.shell_tiles);
-            ++l;
-        }
-    }
-    if (L.n_shell > n_red) {
-        k_batch_shell<T><<<L.n_shell - n_red, dim3(32, 8), shell_smem_bytes<T>(), S.s>>>(D, L.shell_tiles + n_red);
-        ++l;
-    }
     if (gside && (e = cudaStreamWaitEvent(S.s2, S.ghost, 0)) != cudaSuccess) return e;
-    if (L.src_blocks > 0) {
+    if (L.src_blocks > 0 && !fuse_src) {
         // source cells are non-PML cells: ordered after the interior and ghost updates
         // of their cells, concurrent with the shell
         k_batch_sources<T><<<dim3(L.src_blocks, L.n_members), 256, 0, S.s2>>>(D);
@@ -224,15 +247,16 @@ cudaError_t launch_batch(const BatchLaunch& L, const StepStreams& S, int* launch
     return cudaGetLastError();
 }
 
-// Last kernel of a batched step, one warp per member: write the member's
-// constants of the next step (consts[cur ^ 1]) and, after its last step, mark
-// it halted, so its kernels leave at once from the next step on (the tables
+// Beside a step's field kernels, one warp per member: write the member's
+// constants of the next step (consts[cur ^ 1]) and, in its last step, mark it
+// halted, so its kernels leave at once from the next step on (the tables
 // alternate every step, a halted member's state no longer does).  The flag goes
-// into the next step's table D2 first and into this step's table D one step
-// later, by this kernel of the next step: the listener rows of this step, which
-// run beside the next step and read D, still see the member running.  (That
-// kernel of the next step waits for them.)  Members retire without a new tile
-// table or graph.
+// into the next step's table D2, which no field kernel of this step reads, first
+// and into this step's table D one step later, by this kernel of the next step:
+// the listener rows of this step, which run beside the next step and read D,
+// still see the member running.  (This kernel follows the rows of the step
+// before on its stream; they read D2 and consts[cur ^ 1].)  Members retire
+// without a new tile table or graph.
 template <typename T>
 __global__ void __launch_bounds__(128) k_batch_advance(BatchDesc<T>* __restrict__ D, BatchDesc<T>* __restrict__ D2,
                                                        int n) {

@@ -110,7 +110,11 @@ struct ShellBoxes {
     int za[SHELL_MAX_BOXES], zae[SHELL_MAX_BOXES], zb[SHELL_MAX_BOXES], zbe[SHELL_MAX_BOXES];
     int gl[SHELL_MAX_BOXES], ng[SHELL_MAX_BOXES];
     int tu[SHELL_MAX_BOXES], tx[SHELL_MAX_BOXES];
-    int zp[SHELL_MAX_BOXES];  // every group whole, in the box and outside the z PML
+    int px[SHELL_MAX_BOXES];  // x planes per tile: nx in tx even parts of at most xs planes
+    // z groups of a row that are whole, in the box and outside the z PML: the
+    // ng - ge groups from e0 on (ge = ng: none told apart); the reduced-state tiles
+    // enumerate the others first (shell_tile_red)
+    int ge[SHELL_MAX_BOXES], e0[SHELL_MAX_BOXES];
     int block_first[SHELL_MAX_BOXES + 1];
     int zbox;     // box with compact storage (-1: none)
     int zrw;      // compact row width (elements): (ng + 1) * vz
@@ -465,7 +469,7 @@ struct BatchDesc {
     KArgs<T> a[2];       // kernel arguments by parity
     SolveParams* P;      // the member's device parameters
     Box3 interior;
-    Box3 src_region;
+    Box3 src_region;     // supports of the member's sources (empty: none)
     ShellBoxes shell;
     double* ring;        // listener rows: row (step % ring_cap) of n_lis doubles
     int ring_cap;
@@ -501,6 +505,7 @@ struct BatchIntMember {
     unsigned sx, sy;
     T c2k2, lap_scale, kcalp;
     Box3 box;
+    Box3 src;    // supports of the member's sources (empty: none)
     int tu;      // unit tiles per x-plane tile
     int member;  // descriptor index
 };

@@ -246,11 +246,11 @@ __global__ void __launch_bounds__(256) k_interior(const KArgs<T> A, Box3 box) {
 // the end of every step).  The thread goes over its cells in the supports' box
 // again once they are stored, as k_sources would: factors held beside the
 // stencil's registers spilled at four CTAs per SM.
-template <typename T>
-__device__ __forceinline__ void interior_sources(const KArgs<T>& A, const Box3& box, int tu, int tx, int xb,
-                                                 const SourceArgs& S) {
+// args() is called only by threads with a cell in region r.
+template <typename T, typename AT, typename Args>
+__device__ __forceinline__ void interior_sources(const AT& A, const Box3& box, int tu, int tx, int xb, const Box3& r,
+                                                 const Args& args) {
     constexpr int V = 16 / (int)sizeof(T);
-    const Box3& r = S.region;
     const int x0 = max(box.lo[0] + tx * xb, r.lo[0]), x1 = min(min(box.lo[0] + (tx + 1) * xb, box.hi[0]), r.hi[0]);
     if (x0 >= x1) return;
     const int ng = interior_groups_z(box, V);
@@ -261,29 +261,55 @@ __device__ __forceinline__ void interior_sources(const KArgs<T>& A, const Box3& 
     const int zc = box.lo[2] / V * V + g * V;
     const int z0 = max(zc, r.lo[2]), z1 = min(zc + V, r.hi[2]);  // the region lies inside the box
     if (z0 >= z1) return;
+    const SourceArgs& S = args();
     bool any = false;
     for (int s = 0; s < S.n; ++s) any |= S.consts->src_tf[s] != 0.0;
     if (!any) return;
-    for (int x = x0; x < x1; ++x)
-        for (int z = z0; z < z1; ++z) {
-            const unsigned c = (unsigned)x * A.sx + (unsigned)y * A.sy + z;
-            if ((A.cls[c] & (CLS_BULK | CLS_MASK)) != CLS_BULK) continue;
-            const double add = source_at(S, x, y, z) * S.k;
-            if constexpr (sizeof(T) == 8) {
-                A.pn[c] += add;
-            } else {
-                const float d = A.dinc[c] + (float)add;
-                A.dinc[c] = d;
-                A.pn[c] = A.pc[c] + d;
+    // a plane's cells together: their loads do not wait for one another (one by one:
+    // 256^3 FP32 87 us a step instead of 84.5, 160^3 23.0 instead of 22.1)
+#pragma unroll 1
+    for (int x = x0; x < x1; ++x) {
+        const unsigned c = (unsigned)x * A.sx + (unsigned)y * A.sy + zc;
+        bool on[V];
+        float d[V];
+        T p[V];
+        double add[V];
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+            const bool in = zc + e >= z0 && zc + e < z1;
+            on[e] = in && (A.cls[c + e] & (CLS_BULK | CLS_MASK)) == CLS_BULK;
+            d[e] = sizeof(T) == 4 && in ? A.dinc[c + e] : 0.0f;
+            p[e] = !in ? (T)0 : sizeof(T) == 4 ? A.pc[c + e] : A.pn[c + e];
+            add[e] = 0.0;
+        }
+        for (int s = 0; s < S.n; ++s) {
+            const double tf = S.consts->src_tf[s];
+            const double fxy = S.ax[0][s * S.N[0] + x] * S.ax[1][s * S.N[1] + y];
+#pragma unroll
+            for (int e = 0; e < V; ++e) {
+                const double f = fxy * (on[e] ? S.ax[2][s * S.N[2] + zc + e] : 0.0);
+                if (tf != 0.0) add[e] += f * tf;
             }
         }
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+            if (!on[e]) continue;
+            if constexpr (sizeof(T) == 8) {
+                A.pn[c + e] = p[e] + add[e] * S.k;
+            } else {
+                const float dn = d[e] + (float)(add[e] * S.k);
+                A.dinc[c + e] = dn;
+                A.pn[c + e] = p[e] + dn;
+            }
+        }
+    }
 }
 
 template <typename T, bool VISC = false>
 __global__ void __launch_bounds__(256) k_interior_src(const KArgs<T> A, const Box3 box,
                                                       const __grid_constant__ SourceArgs S) {
     interior_tile<T, 2, VISC>(A, box, blockIdx.x, blockIdx.y);
-    interior_sources<T>(A, box, blockIdx.x, blockIdx.y, 2, S);
+    interior_sources<T>(A, box, blockIdx.x, blockIdx.y, 2, S.region, [&]() -> const SourceArgs& { return S; });
 }
 
 // Masked store of a z vector: one vector store when every cell is selected,
@@ -495,8 +521,8 @@ __device__ __forceinline__ void shell_tile_impl(const KArgs<T>& A, const ShellBo
     unsigned inbox = 0;
 #pragma unroll
     for (int e = 0; e < V; ++e) inbox |= (zg + e >= zr0 && zg + e < zr1 ? 1u : 0u) << e;
-    const int x0 = B.x0[b] + tx * B.xs;
-    const int x1 = min(x0 + B.xs, B.x0[b] + B.nx[b]);
+    const int x0 = B.x0[b] + tx * B.px[b];
+    const int x1 = min(x0 + B.px[b], B.x0[b] + B.nx[b]);
     const int xend = B.x0[b] + B.nx[b];
     const int sx = (int)A.sx, sy = (int)A.sy;
     const unsigned c0 = (unsigned)x0 * A.sx + (unsigned)y * A.sy + zg;  // cell and its three low faces
@@ -697,29 +723,17 @@ __global__ void __launch_bounds__(256) k_interior_planes(const KArgs<T> A, const
     b.lo[0] = X.lo[q];
     b.hi[0] = X.hi[q];
     interior_tile<T, 2>(A, b, blockIdx.x, tx);
-    if constexpr (SRC) interior_sources<T>(A, b, blockIdx.x, tx, 2, S);
+    if constexpr (SRC) interior_sources<T>(A, b, blockIdx.x, tx, 2, S.region, [&]() -> const SourceArgs& { return S; });
 }
 
 inline SourceArgs source_args(const SolveParams& hP, const RegionLaunch& R, int cur) {
-    SourceArgs S{};
-    S.region = R.src_region;
-    S.n = R.sources ? hP.n_src : 0;
-    for (int d = 0; d < 3; ++d) {
-        S.N[d] = hP.N[d];
-        S.ax[d] = hP.src_ax[d];
-    }
-    S.consts = hP.consts + cur;
-    S.k = hP.k;
-    return S;
+    return source_args(hP, R.src_region, R.sources ? hP.n_src : 0, cur);
 }
 
 // Host side: one region-split step (streams: StepStreams).  Launch order: the
-// ghost-cell list (s3), the interior (s2), the shell (s) (FP64: the shell before
-// the interior), then the sources (s2, after the interior and the ghost list,
-// whose cells they add to).
-#ifndef FDTD_SHELL_FIRST_F64
-#define FDTD_SHELL_FIRST_F64 1
-#endif
+// ghost-cell list (s3), the interior (s2), the shell (s) (or the shell before the
+// interior), then, where those do not add them, the sources (s2, after the
+// interior and the ghost list, whose cells they add to).
 template <typename T>
 cudaError_t launch_regions(const SolveParams* dP, const SolveParams& hP, const RegionLaunch& R, int cur,
                            const StepStreams& S, int* launches) {
@@ -761,9 +775,13 @@ cudaError_t launch_regions(const SolveParams* dP, const SolveParams& hP, const R
     if (gside && (e = cudaEventRecord(S.ghost, S.s3)) != cudaSuccess) return e;
     // FP64: the shell first.  A shell CTA (188 registers, the 141 KB ring) takes
     // one per SM and leaves the registers of one interior CTA beside it, which
-    // the interior's CTAs, dispatched after, fill; FP32 CTAs of the two kernels
-    // do not fit one SM together, and the interior goes first.
-    constexpr bool shell_first = sizeof(T) == 8 && FDTD_SHELL_FIRST_F64;
+    // the interior's CTAs, dispatched after, fill.  FP32 CTAs of the two kernels
+    // do not fit one SM together: the interior goes first while the shell is
+    // short, and after it from two waves of shell CTAs on, whose last wave it
+    // fills (us a step, interior / shell first: 160^3 23.6 / 24.6, 192x160x144 with
+    // 1.7 waves 30.4 / 31.4, 224^3 with 2.3 62.0 / 60.6, 384x256x256 119.4 / 117.4).
+    const int nblk = (R.skip & 2) ? 0 : R.shell.block_first[R.shell.n];
+    const bool shell_first = sizeof(T) == 8 || nblk >= 2 * 2 * 148;
     auto launch_interior = [&]() {
         if (has_interior) {
             dim3 block(32, 8);
@@ -786,7 +804,6 @@ cudaError_t launch_regions(const SolveParams* dP, const SolveParams& hP, const R
         }
     };
     if (!shell_first) launch_interior();
-    const int nblk = (R.skip & 2) ? 0 : R.shell.block_first[R.shell.n];
     if (nblk > 0) {
         if constexpr (sizeof(T) == 4) {
             if (R.red && R.tma)

@@ -153,6 +153,19 @@ __device__ __forceinline__ GhostLoad ghost_load(const GhostPlan* plan, int g, in
     return r;
 }
 
+__host__ __device__ __forceinline__ SourceArgs source_args(const SolveParams& P, const Box3& region, int n, int cur) {
+    SourceArgs S{};
+    S.region = region;
+    S.n = n;
+    for (int d = 0; d < 3; ++d) {
+        S.N[d] = P.N[d];
+        S.ax[d] = P.src_ax[d];
+    }
+    S.consts = P.consts + cur;
+    S.k = P.k;
+    return S;
+}
+
 // sum_s G_s(x, t + k/2) at cell (x, y, z), as source_term (the factors' loads do
 // not wait for the time factor)
 __device__ __forceinline__ double source_at(const SourceArgs& S, int x, int y, int z) {

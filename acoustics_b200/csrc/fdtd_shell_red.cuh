@@ -164,10 +164,12 @@ __device__ __forceinline__ void red_unstage(const KArgs<float>& A, RedPlane<shel
     if ((KIND == 0 && EY) || ezm) L.a2 = *reinterpret_cast<const VT*>(sp + 9 * FV);
 }
 
-// ZP: every group of box b is whole, in the box and outside the z PML (every
-// per-cell z mask is then known: all cells in, none absorbing along z).
+// Group gi of row yl of box b.  ZP: the group is whole, in the box and outside
+// the z PML (every per-cell z mask is then known: all cells in, none absorbing
+// along z).
 template <int KIND, bool EY, bool PF, bool ZP = false>
-__device__ __forceinline__ void shell_tile_red_impl(const KArgs<float>& A, const ShellBoxes& B, int b, int u, int tx) {
+__device__ __forceinline__ void shell_tile_red_impl(const KArgs<float>& A, const ShellBoxes& B, int b, int yl, int gi,
+                                                    int tx) {
     using T = float;
     constexpr bool CMP = KIND == 2;
     constexpr bool EX = KIND == 0;
@@ -175,18 +177,16 @@ __device__ __forceinline__ void shell_tile_red_impl(const KArgs<float>& A, const
     constexpr unsigned ALL = (1u << V) - 1u;
     using VT = Vec<T, V>;
     const int ng = B.ng[b];
-    const int yl = u / ng;
-    const int gi = u - yl * ng;
     const int y = B.y0[b] + yl;
-    const bool first = gi < B.gl[b];
+    const bool first = ZP || gi < B.gl[b];
     const int zg = first ? (B.za[b] / V + gi) * V : (B.zb[b] / V + (gi - B.gl[b])) * V;
     const int zr0 = first ? B.za[b] : B.zb[b], zr1 = first ? B.zae[b] : B.zbe[b];
     unsigned inbox = 0;
 #pragma unroll
     for (int e = 0; e < V; ++e) inbox |= (zg + e >= zr0 && zg + e < zr1 ? 1u : 0u) << e;
     if constexpr (ZP) inbox = ALL;
-    const int x0 = B.x0[b] + tx * B.xs;
-    const int x1 = min(x0 + B.xs, B.x0[b] + B.nx[b]);
+    const int x0 = B.x0[b] + tx * B.px[b];
+    const int x1 = min(x0 + B.px[b], B.x0[b] + B.nx[b]);
     const int sx = (int)A.sx, sy = (int)A.sy;
     const unsigned c0 = (unsigned)x0 * A.sx + (unsigned)y * A.sy + zg;
     int csx = sx, spare = 0;
@@ -383,29 +383,37 @@ __device__ __forceinline__ void shell_tile_red_impl(const KArgs<float>& A, const
 }
 
 // Box kind: the z-slab pair is B.zbox; an x slab absorbs along x on its first
-// plane; otherwise a y slab.  Uniform per CTA except EY (per row).
+// plane; otherwise a y slab.  A box's units are its rows' z groups, those with a
+// cell in the z PML first and, from the next warp on, the plain ones: a warp then
+// runs one of the two paths (and rarely both kinds of row).
 __device__ __forceinline__ void shell_tile_red(const KArgs<float>& A, const ShellBoxes& B, int b, int tu, int tx) {
     const int u = tu * 256 + threadIdx.x + 32 * threadIdx.y;
-    if (u >= B.ny[b] * B.ng[b]) return;
+    const int ge = B.ge[b], np = B.ng[b] - ge, ny = B.ny[b];
+    const int eu = np > 0 ? (ny * ge + 31) & ~31 : ny * ge;
+    const bool zp = u >= eu;
+    const int ul = zp ? u - eu : u, per = zp ? np : ge;
+    if (ul >= ny * per) return;
+    const int yl = ul / per;
+    int gi = ul - yl * per;
+    if (zp) gi += B.e0[b];
+    else if (gi >= B.e0[b]) gi += np;
     // columns with two absorbing axes hold more state per plane: they load one
     // plane at a time (PF_EY), the others issue the next plane's loads first
     constexpr bool PF = FDTD_SHELL_RED_PREFETCH != 0, PF_EY = FDTD_SHELL_RED_PREFETCH == 2;
-    // (B.zp is uniform per CTA: the plain-z boxes take their own path without divergence)
     if (b == B.zbox) {
-        shell_tile_red_impl<2, false, PF>(A, B, b, u, tx);
+        shell_tile_red_impl<2, false, PF>(A, B, b, yl, gi, tx);
     } else if (__ldg(A.axflag[0] + B.x0[b]) & AXF_PML) {
-        const int y = B.y0[b] + u / B.ng[b];
-        if (__ldg(A.axflag[1] + y) & AXF_PML) {
-            if (B.zp[b]) shell_tile_red_impl<0, true, PF_EY, true>(A, B, b, u, tx);
-            else shell_tile_red_impl<0, true, PF_EY>(A, B, b, u, tx);
+        if (__ldg(A.axflag[1] + B.y0[b] + yl) & AXF_PML) {
+            if (zp) shell_tile_red_impl<0, true, PF_EY, true>(A, B, b, yl, gi, tx);
+            else shell_tile_red_impl<0, true, PF_EY>(A, B, b, yl, gi, tx);
         } else {
-            if (B.zp[b]) shell_tile_red_impl<0, false, PF, true>(A, B, b, u, tx);
-            else shell_tile_red_impl<0, false, PF>(A, B, b, u, tx);
+            if (zp) shell_tile_red_impl<0, false, PF, true>(A, B, b, yl, gi, tx);
+            else shell_tile_red_impl<0, false, PF>(A, B, b, yl, gi, tx);
         }
-    } else if (B.zp[b]) {
-        shell_tile_red_impl<1, true, PF_EY, true>(A, B, b, u, tx);
+    } else if (zp) {
+        shell_tile_red_impl<1, true, PF_EY, true>(A, B, b, yl, gi, tx);
     } else {
-        shell_tile_red_impl<1, true, PF_EY>(A, B, b, u, tx);
+        shell_tile_red_impl<1, true, PF_EY>(A, B, b, yl, gi, tx);
     }
 }
 
