@@ -251,11 +251,15 @@ fdtd_status rebuild(fdtd_batch* b) {
     if ((st_ = grow(b, &b->d_shell, &b->shell_cap, st.size())) != FDTD_OK) return st_;
     if ((st_ = grow(b, &b->d_refs, &b->refs_cap, refs.size())) != FDTD_OK) return st_;
     BATCH_TRY(b, cudaStreamSynchronize(b->stream));
-    BATCH_TRY(b, cudaMemcpy(dd, descs.data(), descs.size(), cudaMemcpyHostToDevice));
-    if (!it.empty()) BATCH_TRY(b, cudaMemcpy(b->d_int, it.data(), it.size() * sizeof(BatchTile), cudaMemcpyHostToDevice));
-    if (!st.empty()) BATCH_TRY(b, cudaMemcpy(b->d_shell, st.data(), st.size() * sizeof(BatchTile), cudaMemcpyHostToDevice));
-    if (!refs.empty())
-        BATCH_TRY(b, cudaMemcpy(b->d_refs, refs.data(), refs.size() * sizeof(ListenerRef), cudaMemcpyHostToDevice));
+    // (in the batch stream's order, like every use of the tables)
+    auto put = [&](void* dst, const void* src, size_t bytes) {
+        return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, b->stream) : cudaSuccess;
+    };
+    BATCH_TRY(b, put(dd, descs.data(), descs.size()));
+    BATCH_TRY(b, put(b->d_int, it.data(), it.size() * sizeof(BatchTile)));
+    BATCH_TRY(b, put(b->d_shell, st.data(), st.size() * sizeof(BatchTile)));
+    BATCH_TRY(b, put(b->d_refs, refs.data(), refs.size() * sizeof(ListenerRef)));
+    BATCH_TRY(b, cudaStreamSynchronize(b->stream));
     BatchLaunch& L = b->L;
     L.descs = b->d_descs;
     b->table_bytes = tbytes;

@@ -366,12 +366,12 @@ fdtd_status build_fully_coupled(fdtd_solver* s) {
     s->fc_alloc.push_back(d_ew);
     CUDA_TRY(s, cudaMalloc(&d_eu, eu.size() * sizeof(int)));
     s->fc_alloc.push_back(d_eu);
-    CUDA_TRY(s, cudaMemcpy(d_ew, ew.data(), ew.size() * sizeof(double), cudaMemcpyHostToDevice));
-    CUDA_TRY(s, cudaMemcpy(d_eu, eu.data(), eu.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CUDA_TRY(s, cudaMemcpy(d_rows, rows.data(), nrow * sizeof(FcRow), cudaMemcpyHostToDevice));
-    CUDA_TRY(s, cudaMemcpy(d_idx, idx.data(), np * sizeof(int), cudaMemcpyHostToDevice));
-    CUDA_TRY(s, cudaMemset(d_vec, 0, 9 * nrow * sizeof(double)));
-    CUDA_TRY(s, cudaMemset(d_st, 0, 4 * sizeof(int)));
+    CUDA_TRY(s, counted_copy(s, d_ew, ew.data(), ew.size() * sizeof(double), cudaMemcpyHostToDevice));
+    CUDA_TRY(s, counted_copy(s, d_eu, eu.data(), eu.size() * sizeof(int), cudaMemcpyHostToDevice));
+    CUDA_TRY(s, counted_copy(s, d_rows, rows.data(), nrow * sizeof(FcRow), cudaMemcpyHostToDevice));
+    CUDA_TRY(s, counted_copy(s, d_idx, idx.data(), np * sizeof(int), cudaMemcpyHostToDevice));
+    CUDA_TRY(s, cudaMemsetAsync(d_vec, 0, 9 * nrow * sizeof(double), s->stream));
+    CUDA_TRY(s, cudaMemsetAsync(d_st, 0, 4 * sizeof(int), s->stream));
     P.fc_rows = (const FcRow*)d_rows;
     P.fc_idx = (const int*)d_idx;
     P.fc_b = (double*)d_vec;
@@ -403,8 +403,7 @@ extern "C" fdtd_status fdtd_solver_boundary_info(fdtd_solver* s, int64_t* n_rows
     if (last_iterations) {
         *last_iterations = 0;
         if (P.fc_status) {
-            CUDA_TRY(s, cudaStreamSynchronize(s->stream));
-            CUDA_TRY(s, cudaMemcpy(last_iterations, P.fc_status, sizeof(int32_t), cudaMemcpyDeviceToHost));
+            CUDA_TRY(s, counted_copy(s, last_iterations, P.fc_status, sizeof(int32_t), cudaMemcpyDeviceToHost));
         }
     }
     return FDTD_OK;

@@ -159,9 +159,13 @@ inline void count_transfer(fdtd_solver* s, size_t n, cudaMemcpyKind kind) {
     if (kind == cudaMemcpyHostToDevice) s->bytes_h2d += (long long)n;
     else if (kind == cudaMemcpyDeviceToHost) s->bytes_d2h += (long long)n;
 }
+// A copy in the order of the solver's stream, done on return.  (The default stream
+// orders nothing before kernels on non-blocking streams: cudaMemcpy from pageable
+// memory may return before the device has the data, and cudaMemset always.)
 inline cudaError_t counted_copy(fdtd_solver* s, void* dst, const void* src, size_t n, cudaMemcpyKind kind) {
     count_transfer(s, n, kind);
-    return cudaMemcpy(dst, src, n, kind);
+    const cudaError_t e = cudaMemcpyAsync(dst, src, n, kind, s->stream);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(s->stream);
 }
 inline cudaError_t counted_copyAsync(fdtd_solver* s, void* dst, const void* src, size_t n, cudaMemcpyKind kind,
                                      cudaStream_t stream) {
