@@ -101,10 +101,33 @@ std::vector<KeptArena> g_arenas;  // oldest first
 constexpr size_t ARENAS_KEPT = 256;
 constexpr size_t ARENAS_KEPT_BYTES = (size_t)16 << 30;
 
+// Streams and pinned buffers of destroyed solvers and batches, kept the same way:
+// creating and destroying a solver's streams took 0.26 + 0.27 ms of the 1.5 that a
+// solver of 80^3 cells took in all (now 0.2), a pinned allocation that needs a new
+// page of the driver's 1.3 ms.
+struct KeptStream {
+    int device, priority;
+    cudaStream_t stream;
+};
+struct KeptHost {
+    void* ptr;
+    size_t bytes;
+};
+std::vector<KeptStream> g_streams;
+std::vector<KeptHost> g_host;
+constexpr size_t STREAMS_KEPT = 256;              // per process
+constexpr size_t HOST_KEPT_BYTES = (size_t)32 << 20;  // per process
+
 void free_kept(int device) {
     std::vector<KeptArena> drop;
+    std::vector<KeptStream> streams;
+    std::vector<KeptHost> host;  // (pinned buffers belong to no device: all)
     {
         std::lock_guard<std::mutex> lk(g_arena_mu);
+        std::vector<KeptStream> keep_s;
+        for (const auto& k : g_streams) (device < 0 || k.device == device ? streams : keep_s).push_back(k);
+        g_streams.swap(keep_s);
+        host.swap(g_host);
         std::vector<KeptArena> keep;
         for (const auto& a : g_arenas) (device < 0 || a.device == device ? drop : keep).push_back(a);
         g_arenas.swap(keep);
@@ -115,9 +138,76 @@ void free_kept(int device) {
         cudaSetDevice(a.device);
         cudaFree(a.ptr);
     }
+    for (const auto& k : streams) {
+        cudaSetDevice(k.device);
+        cudaStreamDestroy(k.stream);
+    }
+    for (const auto& k : host) cudaFreeHost(k.ptr);
     if (cur >= 0) cudaSetDevice(cur);
 }
 }  // namespace
+
+// A non-blocking stream of the current device.
+cudaError_t stream_acquire(int device, int priority, cudaStream_t* out) {
+    {
+        std::lock_guard<std::mutex> lk(g_arena_mu);
+        for (size_t i = g_streams.size(); i-- > 0;)
+            if (g_streams[i].device == device && g_streams[i].priority == priority) {
+                *out = g_streams[i].stream;
+                g_streams.erase(g_streams.begin() + i);
+                return cudaSuccess;
+            }
+    }
+    return cudaStreamCreateWithPriority(out, cudaStreamNonBlocking, priority);
+}
+
+// Give back a stream with no work left on it.
+void stream_release(int device, int priority, cudaStream_t st) {
+    if (!st) return;
+    {
+        std::lock_guard<std::mutex> lk(g_arena_mu);
+        if (g_streams.size() < STREAMS_KEPT) {
+            g_streams.push_back({device, priority, st});
+            return;
+        }
+    }
+    cudaStreamDestroy(st);
+}
+
+// Pinned host memory, block_bytes of it (at least bytes, at most twice that).
+cudaError_t host_acquire(size_t bytes, void** ptr, size_t* block_bytes) {
+    {
+        std::lock_guard<std::mutex> lk(g_arena_mu);
+        int best = -1;
+        for (int i = 0; i < (int)g_host.size(); ++i) {
+            if (g_host[i].bytes < bytes || g_host[i].bytes / 2 > bytes) continue;
+            if (best < 0 || g_host[i].bytes < g_host[best].bytes) best = i;
+        }
+        if (best >= 0) {
+            *ptr = g_host[best].ptr;
+            *block_bytes = g_host[best].bytes;
+            g_host.erase(g_host.begin() + best);
+            return cudaSuccess;
+        }
+    }
+    const cudaError_t e = cudaMallocHost(ptr, bytes);
+    if (e == cudaSuccess) *block_bytes = bytes;
+    return e;
+}
+
+void host_release(void* ptr, size_t block_bytes) {
+    if (!ptr) return;
+    {
+        std::lock_guard<std::mutex> lk(g_arena_mu);
+        size_t total = block_bytes;
+        for (const auto& k : g_host) total += k.bytes;
+        if (total <= HOST_KEPT_BYTES) {
+            g_host.push_back({ptr, block_bytes});
+            return;
+        }
+    }
+    cudaFreeHost(ptr);
+}
 
 cudaError_t arena_acquire(int device, size_t bytes, void** ptr, size_t* block_bytes) {
     {
@@ -367,6 +457,18 @@ struct Carver {
     }
 };
 
+// The tables of a scene, gathered on the host and copied to the device at once:
+// one by one (57 copies) they took 0.45 ms of the 1.2 that a solver of 80^3 cells
+// took in all, now 0.03.
+struct Tables {
+    char* base;
+    std::vector<char> blob;
+    Tables(const void* first, const void* end) : base((char*)first), blob((const char*)end - (const char*)first, 0) {}
+    void put(const void* dst, const void* src, size_t bytes) {
+        if (bytes) std::memcpy(&blob[(const char*)dst - base], src, bytes);
+    }
+};
+
 fdtd_status upload_params(fdtd_solver* s) {
     CUDA_TRY(s, fdtd::counted_copyAsync(s, s->dP, &s->hP, sizeof(SolveParams), cudaMemcpyHostToDevice, s->stream));
     return FDTD_OK;
@@ -517,11 +619,19 @@ static void build_engquist(fdtd_solver* s) {
         return s->tab[0].pml_cell[a[0]] || s->tab[1].pml_cell[a[1]] || s->tab[2].pml_cell[a[2]];
     };
     auto edge1 = [&](int d, int i) { return i == 1 || i == N[d] - 2; };
-    for (int i = 0; i < N[0]; ++i)
+    // (rows inside the PML hold none; of a row off the outer ring only the cells
+    // next to its ends may be one: visiting all cells took 0.2-0.5 ms of a creation
+    // at 80^3)
+    for (int i = 0; i < N[0]; ++i) {
+        if (s->tab[0].pml_cell[i]) continue;
         for (int j = 0; j < N[1]; ++j) {
+            if (s->tab[1].pml_cell[j]) continue;
             const bool all_z = edge1(0, i) || edge1(1, j);
             for (int l = 0; l < N[2]; ++l) {
-                if (!all_z && l != 1 && l != N[2] - 2) continue;
+                if (!all_z && l != 1 && l != N[2] - 2) {
+                    if (l > 1 && l < N[2] - 2) l = N[2] - 3;  // on to N[2] - 2
+                    continue;
+                }
                 const int ijk[3] = {i, j, l};
                 if (is_pml(ijk)) continue;
                 int n0[3], n1[3];
@@ -595,6 +705,7 @@ static void build_engquist(fdtd_solver* s) {
                 s->eng.push_back(e);
             }
         }
+    }
 }
 
 // Cells the interior kernel updates: the non-PML box less the cells on the
@@ -839,10 +950,6 @@ static void carve_arena(fdtd_solver* s, const fdtd_scene_desc* sc, const fdtd_op
         cv.add(&P.lapv[0], n * w);
         cv.add(&P.lapv[1], n * w);
     }
-    // per-axis spatial factors of the sources
-    s->region.src_region = source_region(s);
-    if (!s->sources.empty())
-        for (int d = 0; d < 3; ++d) cv.add((void**)&P.src_ax[d], s->sources.size() * (size_t)N[d] * 8);
     // compact storage of the z-slab box (region-split path)
     const ShellBoxes& SB = s->shell;
     if (o.kernel == FDTD_KERNEL_FUSED && SB.zbox >= 0) {
@@ -854,11 +961,15 @@ static void carve_arena(fdtd_solver* s, const fdtd_scene_desc* sc, const fdtd_op
         }
     }
     cv.add((void**)&P.consts, 2 * sizeof(StepConsts));
+    // what a call reads at its end, side by side (status_bytes)
     cv.add((void**)&P.dev_error, 16);
     cv.add((void**)&s->d_status, 16);
+    cv.add((void**)&s->d_ghost_count, 16);
+    // the tables of a scene, side by side (Tables): the per-axis spatial factors of
+    // the sources first, coef_f[2] last
+    s->region.src_region = source_region(s);
+    for (int d = 0; d < 3; ++d) cv.add((void**)&P.src_ax[d], std::max<size_t>(1, s->sources.size() * (size_t)N[d]) * 8);
     cv.add((void**)&P.listeners, std::max<size_t>(1, s->listeners.size()) * 8);
-    cv.add((void**)&P.lis_rows, (size_t)std::max(1, s->L) * 64 * sizeof(LisRow));
-    cv.add((void**)&P.lis_plan, (size_t)std::max(1, s->L) * sizeof(LisPlan));
     for (int d = 0; d < 3; ++d) {
         cv.add((void**)&P.pml_cell[d], N[d]);
         cv.add((void**)&P.pml_face[d], N[d] + 1);
@@ -878,6 +989,8 @@ static void carve_arena(fdtd_solver* s, const fdtd_scene_desc* sc, const fdtd_op
         cv.add((void**)&P.coef_d[d], (N[d] + 8) * sizeof(AxisCoef<double>));
         cv.add((void**)&P.coef_f[d], (N[d] + 8) * sizeof(AxisCoef<float>));
     }
+    cv.add((void**)&P.lis_rows, (size_t)std::max(1, s->L) * 64 * sizeof(LisRow));
+    cv.add((void**)&P.lis_plan, (size_t)std::max(1, s->L) * sizeof(LisPlan));
     s->lis_cap_steps = std::max(256, o.graph_steps);
     cv.add((void**)&s->d_lis, (size_t)s->lis_cap_steps * std::max(1, s->L) * 8);
     // ghost-neighbour list: at most 6 bulk neighbours per solid cell; solid cells lie
@@ -899,7 +1012,6 @@ static void carve_arena(fdtd_solver* s, const fdtd_scene_desc* sc, const fdtd_op
         cells += 2.0 * sc->n_constraints * ((double)N[0] * N[1] + (double)N[1] * N[2] + (double)N[0] * N[2]);
         s->region.ghost_cap = (int)std::min<double>(cells, (double)n);
         cv.add((void**)&s->d_ghost_list, (size_t)s->region.ghost_cap * 4);
-        cv.add((void**)&s->d_ghost_count, 16);
         // plans of its cells: static scenes, and moving analytic bodies (k_cls_tiles)
         bool mesh = false;
         for (int i = 0; i < sc->n_objects; ++i) mesh = mesh || sc->objects[i].shape == FDTD_SHAPE_MESH;
@@ -991,9 +1103,10 @@ fdtd_status fdtd_solver_create(const fdtd_scene_desc* sc, const fdtd_options* op
         // blocks of the PML shell that runs beside it on stream5
         int least = 0, greatest = 0;
         CUDA_TRY(nullptr, cudaDeviceGetStreamPriorityRange(&least, &greatest));
-        CUDA_TRY(nullptr, cudaStreamCreateWithPriority(&s->stream, cudaStreamNonBlocking, greatest));
+        s->main_priority = greatest;
+        CUDA_TRY(nullptr, stream_acquire(o.device, greatest, &s->stream));
     } else {
-        CUDA_TRY(nullptr, cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
+        CUDA_TRY(nullptr, stream_acquire(o.device, 0, &s->stream));
     }
     {
         // moving bodies: the interior and ghost-list CTAs go before the remaining
@@ -1002,18 +1115,19 @@ fdtd_status fdtd_solver_create(const fdtd_scene_desc* sc, const fdtd_options* op
         int least = 0, greatest = 0;
         CUDA_TRY(nullptr, cudaDeviceGetStreamPriorityRange(&least, &greatest));
         const int pr = any_moving ? greatest : least;
-        CUDA_TRY(nullptr, cudaStreamCreateWithPriority(&s->stream2, cudaStreamNonBlocking, pr));
-        CUDA_TRY(nullptr, cudaStreamCreateWithPriority(&s->stream3, cudaStreamNonBlocking, pr));
+        s->side_priority = pr;
+        CUDA_TRY(nullptr, stream_acquire(o.device, pr, &s->stream2));
+        CUDA_TRY(nullptr, stream_acquire(o.device, pr, &s->stream3));
     }
     CUDA_TRY(nullptr, cudaEventCreateWithFlags(&s->ev_ghost, cudaEventDisableTiming));
-    CUDA_TRY(nullptr, cudaStreamCreateWithFlags(&s->stream4, cudaStreamNonBlocking));
+    CUDA_TRY(nullptr, stream_acquire(o.device, 0, &s->stream4));
     CUDA_TRY(nullptr, cudaEventCreateWithFlags(&s->ev_step, cudaEventDisableTiming));
     CUDA_TRY(nullptr, cudaEventCreateWithFlags(&s->ev_lis[0], cudaEventDisableTiming));
     CUDA_TRY(nullptr, cudaEventCreateWithFlags(&s->ev_lis[1], cudaEventDisableTiming));
     CUDA_TRY(nullptr, cudaEventCreateWithFlags(&s->ev_lis_join, cudaEventDisableTiming));
-    CUDA_TRY(nullptr, cudaStreamCreateWithFlags(&s->stream5, cudaStreamNonBlocking));
     if (any_moving) {
-        CUDA_TRY(nullptr, cudaStreamCreateWithFlags(&s->stream6, cudaStreamNonBlocking));
+        CUDA_TRY(nullptr, stream_acquire(o.device, 0, &s->stream5));
+        CUDA_TRY(nullptr, stream_acquire(o.device, 0, &s->stream6));
         CUDA_TRY(nullptr, cudaEventCreateWithFlags(&s->ev_fdone, cudaEventDisableTiming));
     }
     CUDA_TRY(nullptr, cudaEventCreateWithFlags(&s->ev_sfork, cudaEventDisableTiming));
@@ -1166,6 +1280,7 @@ fdtd_status fdtd_solver_create(const fdtd_scene_desc* sc, const fdtd_options* op
         D.wt = g.width_time;
         D.scale = 1. / 3.6836 * g.normalize_constant;
     }
+    Tables tables(P.src_ax[0], (const char*)P.coef_f[2] + (N[2] + 8) * sizeof(AxisCoef<float>));
     // Gaussian sources (GaussianPressureSource.cpp:6-30): zero outside the box
     // x_s +- 2 sigma_s (strict, per axis), exp(-|x - x_s|^2 / 2 sigma_s^2) * scale
     // inside, the product of one factor per axis
@@ -1182,26 +1297,26 @@ fdtd_status fdtd_solver_create(const fdtd_scene_desc* sc, const fdtd_options* op
                     g[i * N[d] + x] = v;
                 }
             }
-            CUDA_TRY(s.get(), fdtd::counted_copy(s.get(), (void*)P.src_ax[d], g.data(), g.size() * 8, cudaMemcpyHostToDevice));
+            tables.put(P.src_ax[d], g.data(), g.size() * 8);
         }
     // tables
     for (int d = 0; d < 3; ++d) {
         auto& T = s->tab[d];
         std::vector<float> f1(T.pupd.begin(), T.pupd.end()), f2(T.pdiv.begin(), T.pdiv.end());
         std::vector<float> f3(T.vupd.begin(), T.vupd.end()), f4(T.vgrad.begin(), T.vgrad.end());
-        CUDA_TRY(s.get(), fdtd::counted_copy(s.get(), (void*)P.pml_cell[d], T.pml_cell.data(), N[d], cudaMemcpyHostToDevice));
-        CUDA_TRY(s.get(), fdtd::counted_copy(s.get(), (void*)P.pml_face[d], T.pml_face.data(), N[d] + 1, cudaMemcpyHostToDevice));
-        CUDA_TRY(s.get(), fdtd::counted_copy(s.get(), (void*)P.cpos[d], T.cpos.data(), N[d] * 8, cudaMemcpyHostToDevice));
-        CUDA_TRY(s.get(), fdtd::counted_copy(s.get(), (void*)P.fpos[d], T.fpos.data(), (N[d] + 1) * 8, cudaMemcpyHostToDevice));
-        CUDA_TRY(s.get(), fdtd::counted_copy(s.get(), (void*)P.pupd[d], T.pupd.data(), N[d] * 8, cudaMemcpyHostToDevice));
-        CUDA_TRY(s.get(), fdtd::counted_copy(s.get(), (void*)P.pdiv[d], T.pdiv.data(), N[d] * 8, cudaMemcpyHostToDevice));
-        CUDA_TRY(s.get(), fdtd::counted_copy(s.get(), (void*)P.vupd[d], T.vupd.data(), (N[d] + 1) * 8, cudaMemcpyHostToDevice));
-        CUDA_TRY(s.get(), fdtd::counted_copy(s.get(), (void*)P.vgrad[d], T.vgrad.data(), (N[d] + 1) * 8, cudaMemcpyHostToDevice));
-        CUDA_TRY(s.get(), fdtd::counted_copy(s.get(), (void*)P.pupd_f[d], f1.data(), N[d] * 4, cudaMemcpyHostToDevice));
-        CUDA_TRY(s.get(), fdtd::counted_copy(s.get(), (void*)P.pdiv_f[d], f2.data(), N[d] * 4, cudaMemcpyHostToDevice));
-        CUDA_TRY(s.get(), fdtd::counted_copy(s.get(), (void*)P.vupd_f[d], f3.data(), (N[d] + 1) * 4, cudaMemcpyHostToDevice));
-        CUDA_TRY(s.get(), fdtd::counted_copy(s.get(), (void*)P.vgrad_f[d], f4.data(), (N[d] + 1) * 4, cudaMemcpyHostToDevice));
-        CUDA_TRY(s.get(), fdtd::counted_copy(s.get(), (void*)s->d_csig[d], T.csig.data(), N[d] * 8, cudaMemcpyHostToDevice));
+        tables.put(P.pml_cell[d], T.pml_cell.data(), N[d]);
+        tables.put(P.pml_face[d], T.pml_face.data(), N[d] + 1);
+        tables.put(P.cpos[d], T.cpos.data(), N[d] * 8);
+        tables.put(P.fpos[d], T.fpos.data(), (N[d] + 1) * 8);
+        tables.put(P.pupd[d], T.pupd.data(), N[d] * 8);
+        tables.put(P.pdiv[d], T.pdiv.data(), N[d] * 8);
+        tables.put(P.vupd[d], T.vupd.data(), (N[d] + 1) * 8);
+        tables.put(P.vgrad[d], T.vgrad.data(), (N[d] + 1) * 8);
+        tables.put(P.pupd_f[d], f1.data(), N[d] * 4);
+        tables.put(P.pdiv_f[d], f2.data(), N[d] * 4);
+        tables.put(P.vupd_f[d], f3.data(), (N[d] + 1) * 4);
+        tables.put(P.vgrad_f[d], f4.data(), (N[d] + 1) * 4);
+        tables.put(s->d_csig[d], T.csig.data(), N[d] * 8);
         // packed flags and coefficient quads of the shell kernel
         std::vector<uint8_t> fl(N[d] + 8, 0);
         std::vector<AxisCoef<double>> cd(N[d] + 8, AxisCoef<double>{0.0, 0.0, 0.0, 0.0});
@@ -1226,15 +1341,18 @@ fdtd_status fdtd_solver_create(const fdtd_scene_desc* sc, const fdtd_options* op
             cf[i].pupd = (float)cd[i].pupd;
             cf[i].pdiv = (float)cd[i].pdiv;
         }
-        CUDA_TRY(s.get(), fdtd::counted_copy(s.get(), (void*)P.axflag[d], fl.data(), fl.size(), cudaMemcpyHostToDevice));
-        CUDA_TRY(s.get(), fdtd::counted_copy(s.get(), (void*)P.coef_d[d], cd.data(), cd.size() * sizeof(cd[0]), cudaMemcpyHostToDevice));
-        CUDA_TRY(s.get(), fdtd::counted_copy(s.get(), (void*)P.coef_f[d], cf.data(), cf.size() * sizeof(cf[0]), cudaMemcpyHostToDevice));
+        tables.put(P.axflag[d], fl.data(), fl.size());
+        tables.put(P.coef_d[d], cd.data(), cd.size() * sizeof(cd[0]));
+        tables.put(P.coef_f[d], cf.data(), cf.size() * sizeof(cf[0]));
     }
     if (s->L > 0)
-        CUDA_TRY(s.get(), fdtd::counted_copy(s.get(), (void*)P.listeners, s->listeners.data(), s->listeners.size() * 8, cudaMemcpyHostToDevice));
+        tables.put(P.listeners, s->listeners.data(), s->listeners.size() * 8);
+    CUDA_TRY(s.get(), fdtd::counted_copy(s.get(), tables.base, tables.blob.data(), tables.blob.size(), cudaMemcpyHostToDevice));
     CUDA_TRY(s.get(), inject_failure(FDTD_INJECT_HOST_ALLOC)
                           ? cudaErrorMemoryAllocation
-                          : cudaMallocHost((void**)&s->h_lis_stage, (size_t)s->lis_cap_steps * std::max(1, s->L) * 8));
+                          : host_acquire((size_t)s->lis_cap_steps * std::max(1, s->L) * 8 + status_bytes(s.get()),
+                                         (void**)&s->h_lis_stage, &s->h_lis_bytes));
+    s->h_status = (int*)(s->h_lis_stage + (size_t)s->lis_cap_steps * std::max(1, s->L));
     s->xb = (o.x_chunk == 2 || o.x_chunk == 4 || o.x_chunk == 8) ? o.x_chunk : 2;
     s->region.xb = s->xb;
     // tile_y: x planes each PML-shell thread marches over
@@ -1261,15 +1379,16 @@ fdtd_status fdtd_solver_destroy(fdtd_solver* s) {
     for (void* p : s->mesh_alloc) cudaFree(p);
     if (s->d_solid_pml) cudaFree(s->d_solid_pml);
     if (s->arena) arena_release(s->opt.device, s->arena, s->arena_block);
-    if (s->h_lis_stage) cudaFreeHost(s->h_lis_stage);
+    host_release(s->h_lis_stage, s->h_lis_bytes);
     if (s->rb_host) cudaFreeHost(s->rb_host);
     for (cudaEvent_t ev : s->rb_done)
         if (ev) cudaEventDestroy(ev);
     for (cudaEvent_t ev : {s->ev_fork, s->ev_join, s->ev_ghost, s->ev_step, s->ev_lis[0], s->ev_lis[1], s->ev_lis_join,
                            s->ev_sfork, s->ev_sdone, s->ev_fdone})
         if (ev) cudaEventDestroy(ev);
-    for (cudaStream_t st : {s->stream2, s->stream3, s->stream4, s->stream5, s->stream6, s->stream})
-        if (st) cudaStreamDestroy(st);
+    for (cudaStream_t st : {s->stream2, s->stream3}) stream_release(s->opt.device, s->side_priority, st);
+    for (cudaStream_t st : {s->stream4, s->stream5, s->stream6}) stream_release(s->opt.device, 0, st);
+    stream_release(s->opt.device, s->main_priority, s->stream);
     delete s;
     return FDTD_OK;
 }
@@ -1280,31 +1399,14 @@ fdtd_status fdtd_solver_reset(fdtd_solver* s, double t0) {
     if (!s) return FDTD_ERR_INVALID_ARG;
     CUDA_TRY(s, cudaSetDevice(s->opt.device));
     SolveParams& P = s->hP;
-    const size_t w = s->precision == FDTD_PRECISION_FP64 ? 8 : 4;
     // zero all state (fields, velocities, split pressures, flags; padding included)
     const long long np = s->np;
-    CUDA_TRY(s, cudaMemsetAsync(P.p[0], 0, np * w, s->stream));
-    CUDA_TRY(s, cudaMemsetAsync(P.p[1], 0, np * w, s->stream));
-    if (P.dinc) CUDA_TRY(s, cudaMemsetAsync(P.dinc, 0, np * 4, s->stream));
-    for (int b = 0; b < 2; ++b)
-        if (P.lapv[b]) CUDA_TRY(s, cudaMemsetAsync(P.lapv[b], 0, np * w, s->stream));
-    for (int d = 0; d < 3; ++d) {
-        CUDA_TRY(s, cudaMemsetAsync(P.pd[d], 0, np * w, s->stream));
-        CUDA_TRY(s, cudaMemsetAsync(P.v[0][d], 0, np * w, s->stream));
-        if (P.v[1][d]) CUDA_TRY(s, cudaMemsetAsync(P.v[1][d], 0, np * w, s->stream));
-        if (P.zcount > 0) {
-            CUDA_TRY(s, cudaMemsetAsync(P.zpd[d], 0, P.zcount * w, s->stream));
-            CUDA_TRY(s, cudaMemsetAsync(P.zv[0][d], 0, P.zcount * w, s->stream));
-            CUDA_TRY(s, cudaMemsetAsync(P.zv[1][d], 0, P.zcount * w, s->stream));
-        }
-    }
+    // (one range of the arena, up to the step constants and the error flags)
+    CUDA_TRY(s, cudaMemsetAsync(P.p[0], 0, (char*)(s->d_status + 4) - (char*)P.p[0], s->stream));
     // initFieldRasterized: every cell bulk with valid history (MAC_Grid.cpp:2459-2470, :4170-4180)
     CUDA_TRY(s, cudaMemsetAsync(P.cls, CLS_BULK | CLS_VALID, np, s->stream));
     if (P.eng_buf) CUDA_TRY(s, cudaMemsetAsync(P.eng_buf, 0, s->eng.size() * ENG_BUF * 8, s->stream));
     CUDA_TRY(s, cudaMemsetAsync(P.gobj, GOBJ_NONE, np, s->stream));
-    CUDA_TRY(s, cudaMemsetAsync(P.consts, 0, 2 * sizeof(StepConsts), s->stream));
-    CUDA_TRY(s, cudaMemsetAsync(P.dev_error, 0, sizeof(int), s->stream));
-    CUDA_TRY(s, cudaMemsetAsync(s->d_status, 0, 16, s->stream));
     s->time = t0;
     s->state_time = t0;
     s->step_index = 0;

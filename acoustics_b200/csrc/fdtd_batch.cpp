@@ -403,15 +403,15 @@ fdtd_status fdtd_batch_create(int32_t n, const fdtd_scene_desc* scenes, const in
         return batch_fail(nullptr, FDTD_ERR_INVALID_ARG, "graph_steps must be an even number in [0, 256]");
     b->precision = b->opt.precision;
     BATCH_TRY(nullptr, cudaSetDevice(b->opt.device));
-    BATCH_TRY(nullptr, cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
-    BATCH_TRY(nullptr, cudaStreamCreateWithFlags(&b->stream2, cudaStreamNonBlocking));
-    BATCH_TRY(nullptr, cudaStreamCreateWithFlags(&b->stream3, cudaStreamNonBlocking));
+    BATCH_TRY(nullptr, stream_acquire(b->opt.device, 0, &b->stream));
+    BATCH_TRY(nullptr, stream_acquire(b->opt.device, 0, &b->stream2));
+    BATCH_TRY(nullptr, stream_acquire(b->opt.device, 0, &b->stream3));
     BATCH_TRY(nullptr, cudaEventCreateWithFlags(&b->ev_ghost, cudaEventDisableTiming));
     if (b->precision == FDTD_PRECISION_FP32_COMPENSATED) BATCH_TRY(nullptr, prepare_fp32_kernels());
     else BATCH_TRY(nullptr, prepare_fp64_kernels());
     BATCH_TRY(nullptr, cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming));
     BATCH_TRY(nullptr, cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming));
-    BATCH_TRY(nullptr, cudaStreamCreateWithFlags(&b->stream4, cudaStreamNonBlocking));
+    BATCH_TRY(nullptr, stream_acquire(b->opt.device, 0, &b->stream4));
     BATCH_TRY(nullptr, cudaEventCreateWithFlags(&b->ev_step, cudaEventDisableTiming));
     BATCH_TRY(nullptr, cudaEventCreateWithFlags(&b->ev_adv, cudaEventDisableTiming));
     BATCH_TRY(nullptr, cudaEventCreateWithFlags(&b->ev_lis_join, cudaEventDisableTiming));
@@ -680,8 +680,8 @@ fdtd_status fdtd_batch_release(fdtd_batch* b, int32_t member) {
 fdtd_status fdtd_batch_destroy(fdtd_batch* b) {
     if (!b) return FDTD_OK;
     cudaSetDevice(b->opt.device);
-    if (b->stream) cudaStreamSynchronize(b->stream);
-    if (b->stream4) cudaStreamSynchronize(b->stream4);
+    for (cudaStream_t st : {b->stream, b->stream2, b->stream3, b->stream4})
+        if (st) cudaStreamSynchronize(st);
     for (int i = 0; i < 2; ++i)
         if (b->graph[i]) cudaGraphExecDestroy(b->graph[i]);
     for (auto& mb : b->members)
@@ -695,10 +695,7 @@ fdtd_status fdtd_batch_destroy(fdtd_batch* b) {
     if (b->ev_ghost) cudaEventDestroy(b->ev_ghost);
     for (cudaEvent_t ev : {b->ev_step, b->ev_adv, b->ev_lis_join})
         if (ev) cudaEventDestroy(ev);
-    if (b->stream4) cudaStreamDestroy(b->stream4);
-    if (b->stream2) cudaStreamDestroy(b->stream2);
-    if (b->stream3) cudaStreamDestroy(b->stream3);
-    if (b->stream) cudaStreamDestroy(b->stream);
+    for (cudaStream_t st : {b->stream4, b->stream3, b->stream2, b->stream}) stream_release(b->opt.device, 0, st);
     delete b;
     return FDTD_OK;
 }

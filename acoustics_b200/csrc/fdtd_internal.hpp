@@ -118,7 +118,10 @@ struct fdtd_solver {
     double* d_lap = nullptr;
     int* d_status = nullptr;
     double* d_lis = nullptr;
-    double* h_lis_stage = nullptr;
+    double* h_lis_stage = nullptr;  // (pinned; followed by h_status)
+    size_t h_lis_bytes = 0;
+    int main_priority = 0, side_priority = 0;  // of stream; of stream2 and stream3
+    int* h_status = nullptr;         // host side of what a call reads at its end: dev_error ... d_ghost_count
     int lis_cap_steps = 0;
     int xb = 4;                       // planes per thread of the interior kernel
     fdtd::Box3 interior{};            // non-PML box
@@ -172,6 +175,10 @@ inline cudaError_t counted_copyAsync(fdtd_solver* s, void* dst, const void* src,
     count_transfer(s, n, kind);
     return cudaMemcpyAsync(dst, src, n, kind, stream);
 }
+// bytes of the arena from the error flags to the list lengths (carve_arena)
+inline size_t status_bytes(const fdtd_solver* s) {
+    return (size_t)((const char*)(s->d_ghost_count + 4) - (const char*)s->hP.dev_error);
+}
 void set_error(fdtd_solver* s, const std::string& msg);
 // no listener stencil meets a classification box (fdtd_step.cpp)
 bool listeners_clear_of(const fdtd_solver* s, const ClsBoxes& B);
@@ -194,6 +201,10 @@ int32_t batch_place(fdtd_batch* b, PreparedMember&& pm);
 // one on the same device (fdtd_api.cpp)
 cudaError_t arena_acquire(int device, size_t bytes, void** ptr, size_t* block_bytes);
 void arena_release(int device, void* ptr, size_t block_bytes);
+cudaError_t stream_acquire(int device, int priority, cudaStream_t* out);
+void stream_release(int device, int priority, cudaStream_t st);
+cudaError_t host_acquire(size_t bytes, void** ptr, size_t* block_bytes);
+void host_release(void* ptr, size_t block_bytes);
 // listener plans of a static solve from its current classification (after a restore)
 fdtd_status rebuild_listener_plans(fdtd_solver* s);
 // fdtd_debug_inject_failure: true when this allocation of kind `what` is to fail

@@ -319,12 +319,14 @@ fdtd_status fdtd_gaussian_source_defaults(fdtd_gaussian_source_desc* src, double
  * (PML_WaveSolver.cpp:78-146) + FDTD_AcousticSimulator::ResetStartTime (:458-523). */
 fdtd_status fdtd_solver_create(const fdtd_scene_desc* scene, const fdtd_options* options,
                                fdtd_solver** out);
-/* Releases the solver's streams and events; its device block is kept for the next
- * solver created on the same device (freed when an allocation would fail, when the
- * kept blocks pass 16 GiB or 256 blocks, oldest first, or by
- * fdtd_release_cached_memory). */
+/* Releases the solver's events; its device block is kept for the next solver
+ * created on the same device (freed when an allocation would fail, when the kept
+ * blocks pass 16 GiB or 256 blocks, oldest first, or by
+ * fdtd_release_cached_memory), and so are its streams (256 at most) and its pinned
+ * staging buffer (32 MiB at most), until fdtd_release_cached_memory. */
 fdtd_status fdtd_solver_destroy(fdtd_solver* s);
-/* Free the device blocks kept from destroyed solvers: of one device, or of all (device < 0). */
+/* Free the device blocks and streams kept from destroyed solvers, of one device or of
+ * all (device < 0), and the pinned buffers. */
 void fdtd_release_cached_memory(int32_t device);
 /* Reinitialize_PML_WaveSolver(true, t0) + ResetCellHistory(true) (PML_WaveSolver.cpp:102-146) */
 fdtd_status fdtd_solver_reset(fdtd_solver* s, double start_time);
