@@ -75,11 +75,18 @@ __global__ void __launch_bounds__(256, XB == 2 ? FDTD_BATCH_INT_MINB : 1) k_batc
     }
 }
 
+// (out of line: beside the tile's code it spilled at four CTAs per SM)
+template <typename T>
+__device__ __noinline__ void member_interior_sources(const BatchIntMember<T>& M, const BatchDesc<T>& d, int tu, int tx,
+                                                     int xb) {
+    interior_sources<T>(M, M.box, tu, tx, xb, M.src, [&]() { return member_sources(d); });
+}
+
 // One CTA per interior tile, its member found by a binary search of the
 // parameter-bank table from blockIdx alone (warp-uniform, like its arguments);
 // a member's CTAs enumerate its tiles as the tile table does (x tile outer).
 template <typename T, int XB>
-__global__ void __launch_bounds__(256, XB == 2 ? 4 : 1)
+__global__ void __launch_bounds__(256, XB == 2 ? 4 : XB == 4 ? 2 : 1)  // (FP64, XB = 4: 138 registers else, one CTA per SM)
     k_batch_interior_p(const __grid_constant__ BatchIntParams<T> P, const BatchDesc<T>* __restrict__ D) {
     const int blk = (int)blockIdx.x;
     int lo = 0, hi = P.n - 1;
@@ -93,7 +100,8 @@ __global__ void __launch_bounds__(256, XB == 2 ? 4 : 1)
     if (d.halted) return;
     const int local = blk - P.first[lo];
     interior_tile<T, XB>(M, M.box, local % M.tu, local / M.tu);
-    interior_sources<T>(M, M.box, local % M.tu, local / M.tu, XB, M.src, [&]() { return member_sources(d); });
+    const int tx = local / M.tu, x0 = M.box.lo[0] + tx * XB;
+    if (x0 < M.src.hi[0] && x0 + XB > M.src.lo[0]) member_interior_sources(M, d, local - tx * M.tu, tx, XB);
 }
 
 // One CTA per shell tile of the tables (all members in one launch).  The

@@ -90,8 +90,8 @@ __host__ __device__ constexpr int shell_vz(int word) { return word == 4 ? FDTD_S
 // [za, zae) u [zb, zbe).  Along z it is cut into vector groups of vz cells
 // starting at multiples of vz: gl groups cover [za, zae), the next ng - gl
 // cover [zb, zbe) (groups may reach outside the ranges; those cells are
-// masked).  A thread owns one group of one row for xs x planes; a CTA owns 256
-// consecutive (row, group) units: tu unit tiles x tx plane tiles per box.
+// masked).  A thread owns one group of one row for px x planes (at most xs); a
+// CTA owns 256 consecutive (row, group) units: tu unit tiles x tx plane tiles per box.
 // block_first[] is the prefix sum of CTAs per box.
 //
 // The z-slab pair (box zbox) keeps its split pressures and face velocities in

@@ -496,7 +496,7 @@ __device__ __forceinline__ void shell_load(const KArgs<T>& A, const ShellStore& 
 // One PML-shell tile: unit tile tu (256 consecutive (row, z-group) units of box
 // b, one per thread) by x tile tx.  A thread owns one z group (a vector of
 // shell_vz cells starting at a multiple of its width; cells outside the
-// group's z range are masked) of one row and marches along x over B.xs planes:
+// group's z range are masked) of one row and marches along x over B.px planes:
 // p(x-1), p(x) and the low x face velocity are carried in registers, and (with
 // FDTD_SHELL_PREFETCH) the loads of plane x+1 are issued before plane x is
 // computed and stored.  Face flags (MAC_Grid.cpp:2568-2575, :2631-2633) are
