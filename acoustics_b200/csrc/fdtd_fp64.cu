@@ -703,6 +703,31 @@ __global__ void __launch_bounds__(256) k_cls_tiles(const SolveParams* __restrict
 
 // Listener sampling: fdtd_listeners.cuh (one warp per listener)
 
+// Value of fresh cell c when no cell of its fit's stencil has a history: that of
+// its first bulk neighbour in the order +x, -x, +y, -y, +z, -z (MAC_Grid.cpp:1993-2254).
+// The reference goes over the cells in ascending order, in place.  So a neighbour
+// that is fresh itself gives, on the + side, what it held as a solid cell, zero,
+// and on the - side the value just made for it: `next` then names it, and its value
+// is made again instead of read, since the device makes all of them at once.  (Cells
+// that a body leaves by jumps of more than a cell, or in a gap between two bodies.)
+template <typename Val>
+__device__ __forceinline__ double fresh_from_neighbour(const SolveParams& P, long long c, const Val& val, long long& next) {
+    int idx[3];
+    cell_ijk(P, c, idx[0], idx[1], idx[2]);
+    const long long strides[3] = {P.SX, P.SY, 1};
+    for (int d = 0; d < 3; ++d)
+        for (int s = 1; s >= -1; s -= 2) {
+            if (idx[d] + s < 0 || idx[d] + s >= P.N[d]) continue;
+            const long long n = c + s * strides[d];
+            const uint8_t code = P.cls[n];
+            if (!(code & CLS_BULK)) continue;
+            if (code & CLS_VALID) return val(n);
+            if (s < 0) next = n;
+            return 0.0;
+        }
+    return 0.0;
+}
+
 // ---------------------------------------------------------------------------
 // Fresh-cell interpolation (MAC_Grid::InterpolateFreshPressureCell, MLS branch,
 // MAC_Grid.cpp:1993-2254): a cell that is bulk now but was solid before gets
@@ -712,7 +737,7 @@ __global__ void __launch_bounds__(256) k_cls_tiles(const SolveParams* __restrict
 // copy of the code misses the instruction cache less than several inlined ones.
 template <typename T>
 __device__ __noinline__ double fresh_value(const SolveParams& P, const T* __restrict__ pa, const T* __restrict__ pb,
-                                           bool diff, long long c, double t, int* status) {
+                                           bool diff, long long c, double t, int* status, long long& next) {
     // value of buffer "a" (or a - b when diff) at cell n
     auto val = [&](long long n) -> double { return diff ? (double)pa[n] - (double)pb[n] : (double)pa[n]; };
     int i, j, k;
@@ -774,15 +799,7 @@ __device__ __noinline__ double fresh_value(const SolveParams& P, const T* __rest
             }
             return vals[mid];
         }
-        const int idx[3] = {i, j, k};
-        const long long strides[3] = {P.SX, P.SY, 1};
-        for (int d = 0; d < 3; ++d)
-            for (int s = 1; s >= -1; s -= 2) {
-                if (idx[d] + s < 0 || idx[d] + s >= P.N[d]) continue;
-                const long long n = c + s * strides[d];
-                if (P.cls[n] & CLS_BULK) return val(n);
-            }
-        return 0.0;
+        return fresh_from_neighbour(P, c, val, next);
     }
     double c0 = 0.0;
     if (!householder_ls4_rows8(A, b, nk, c0)) c0 = 0.0;
@@ -794,18 +811,28 @@ __device__ __noinline__ double fresh_value(const SolveParams& P, const T* __rest
 
 template <typename T>
 __device__ __forceinline__ void fresh_cell(const SolveParams& P, int cur, long long c, double t, int* st) {
+    // (the cell itself, or the one its value is a copy of)
+    auto value = [&](const T* pa, const T* pb, bool diff) {
+        double v = 0.0;
+        for (long long at = c; at >= 0;) {
+            long long next = -1;
+            v = fresh_value<T>(P, pa, pb, diff, at, t, st, next);
+            at = next;
+        }
+        return v;
+    };
     if (sizeof(T) == 8) {
-        double* pl = (double*)P.p[cur ^ 1];
-        double* pc = (double*)P.p[cur];
-        const double vl = fresh_value<double>(P, pl, pl, false, c, t, st);
-        const double vc = fresh_value<double>(P, pc, pc, false, c, t, st);
+        T* pl = (T*)P.p[cur ^ 1];
+        T* pc = (T*)P.p[cur];
+        const double vl = value(pl, pl, false);
+        const double vc = value(pc, pc, false);
         pl[c] = vl;
         pc[c] = vc;
     } else {
         // FP32 keeps p^n and the increment; p^{n-1} = p^n - d
-        float* pc = (float*)P.p[cur];
-        const double vc = fresh_value<float>(P, pc, pc, false, c, t, st);
-        const double vl = fresh_value<float>(P, pc, P.dinc, true, c, t, st);
+        T* pc = (T*)P.p[cur];
+        const double vc = value(pc, pc, false);
+        const double vl = value(pc, (const T*)(const void*)P.dinc, true);
         pc[c] = (float)vc;
         P.dinc[c] = (float)(vc - vl);
     }
@@ -866,7 +893,8 @@ __device__ __forceinline__ bool fresh_geometry(const SolveParams& P, long long c
 // the same branches: they share the image point and the stencil flags).
 template <typename T>
 __device__ __noinline__ double fresh_value_half(const SolveParams& P, const FreshGeometry& G, const T* __restrict__ pa,
-                                                const T* __restrict__ pb, bool diff, long long c, double t) {
+                                                const T* __restrict__ pb, bool diff, long long c, double t,
+                                                long long& next) {
     const int q = threadIdx.x & 15;
     const int base = threadIdx.x & 16;  // first lane of this half
     auto sum_rows = [&](double x, int from) {
@@ -930,15 +958,8 @@ __device__ __noinline__ double fresh_value_half(const SolveParams& P, const Fres
             }
             return vm;
         }
-        const int idx[3] = {i, j, k};
-        const long long strides[3] = {P.SX, P.SY, 1};
-        for (int d = 0; d < 3; ++d)
-            for (int s = 1; s >= -1; s -= 2) {
-                if (idx[d] + s < 0 || idx[d] + s >= P.N[d]) continue;
-                const long long n = c + s * strides[d];
-                if (P.cls[n] & CLS_BULK) return diff ? (double)pa[n] - (double)pb[n] : (double)pa[n];
-            }
-        return 0.0;
+        return fresh_from_neighbour(
+            P, c, [&](long long n) { return diff ? (double)pa[n] - (double)pb[n] : (double)pa[n]; }, next);
     }
     // Householder QR of the 8 x 4 block, one row per lane (householder_ls4_rows8)
     double R[4][4];
@@ -1001,7 +1022,8 @@ __device__ __noinline__ double fresh_value_half(const SolveParams& P, const Fres
 // filled, one warp per cell: the half-warp 16 w + q makes the value of buffer w
 // (p^n for w = 0, p^{n-1} for w = 1).  A list that overflowed is replaced by a
 // sweep over every cell, a thread per cell.  Each fresh value reads only cells
-// with a valid history, never another fresh cell, so the order does not matter.
+// with a valid history, never another fresh cell (fresh_from_neighbour), so the
+// order does not matter.
 template <typename T>
 __global__ void __launch_bounds__(128) k_fresh_cells(const SolveParams* __restrict__ Pp, int cur, long long n,
                                                      int* status) {
@@ -1027,15 +1049,19 @@ __global__ void __launch_bounds__(128) k_fresh_cells(const SolveParams* __restri
     const int w = lane >> 4;
     for (int f = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; f < count; f += (gridDim.x * blockDim.x) >> 5) {
         const long long c = P.fresh_list[f];
-        FreshGeometry G;
         double v = 0.0;
-        if (fresh_geometry(P, c, stacks[threadIdx.x >> 5], G)) {
-            // FP32: p^{n-1} is p^n less the increment
-            const T* pa = (const T*)P.p[sizeof(T) == 8 ? cur ^ w : cur];
-            const T* pb = sizeof(T) == 8 ? pa : (const T*)(const void*)P.dinc;
-            v = fresh_value_half<T>(P, G, pa, pb, sizeof(T) == 4 && w, c, t);
-        } else {
-            st = 2;
+        for (long long at = c; at >= 0;) {  // (c itself, or the cell its value is a copy of)
+            FreshGeometry G;
+            long long next = -1;
+            if (fresh_geometry(P, at, stacks[threadIdx.x >> 5], G)) {
+                // FP32: p^{n-1} is p^n less the increment
+                const T* pa = (const T*)P.p[sizeof(T) == 8 ? cur ^ w : cur];
+                const T* pb = sizeof(T) == 8 ? pa : (const T*)(const void*)P.dinc;
+                v = fresh_value_half<T>(P, G, pa, pb, sizeof(T) == 4 && w, at, t, next);
+            } else {
+                st = 2;
+            }
+            at = next;
         }
         const double other = __shfl_xor_sync(0xffffffffu, v, 16);
         if ((lane & 15) != 0) continue;
