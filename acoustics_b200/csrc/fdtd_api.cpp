@@ -481,6 +481,7 @@ fdtd_status run_classification(fdtd_solver* s) {
     int l = 0;  // (as by the step before the first one, whose parity is 0)
     CUDA_TRY(s, launch_classify(s->dP, s->N, B, false, !s->mesh_alloc.empty(), 1, s->stream, &l));
     s->cls_boxes_current = true;
+    if (s->moving) s->cls_objs = s->objs;
     s->launches += l;
     return FDTD_OK;
 }

@@ -38,6 +38,7 @@ struct MeshHost {
     std::vector<MeshTri> tris;  // leaf order
     std::vector<int> top;       // MeshView::top
     std::vector<double> vertices;
+    double edge = 0;            // longest edge
 };
 bool build_mesh(const fdtd_mesh_desc& md, MeshHost& out, std::string& err);
 void mesh_extent(const double* verts, size_t nv, const double R[9], double lo[3], double hi[3]);
@@ -82,6 +83,7 @@ struct fdtd_solver {
     // hP.boxes are the boxes of the classification the cell flags hold (the
     // solid cells lie in them); cleared when the flags are loaded from elsewhere
     bool cls_boxes_current = false;
+    std::vector<fdtd::HostObject> cls_objs;  // moving scenes: the bodies as that classification found them
     bool lis_clear = false;         // listeners_clear_of the boxes of the last reset
     long long overlapped_steps = 0;
     // geometry

@@ -206,6 +206,13 @@ bool build_mesh(const fdtd_mesh_desc& md, MeshHost& out, std::string& err) {
     }
     out.tris.resize(nt);
     for (int k = 0; k < nt; ++k) out.tris[k] = tris[B.order[k]];
+    out.edge = 0.0;
+    for (const MeshTri& T : tris)
+        for (int k = 0; k < 3; ++k) {
+            double e[3];
+            sub3(T.p[(k + 1) % 3], T.p[k], e);
+            out.edge = std::max(out.edge, norm3(e));
+        }
     out.vertices.assign(md.vertices, md.vertices + 3 * (size_t)nv);
     return true;
 }

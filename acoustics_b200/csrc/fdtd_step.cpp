@@ -44,17 +44,64 @@ void classification_launches(fdtd_solver* s, int cur, fdtd_status& st, const Cls
     }
 }
 
-// Every box with cells lies inside the non-PML box, two cells from its faces.
+// Every box with cells lies inside the non-PML box, `cells` cells from its faces.
 // The classification writes pressures only at solid cells (in the boxes of
 // this step) and fresh cells (in those of the step before); the shell kernel
 // reads and writes the PML cells and reads one cell beyond them.
-bool boxes_clear_of_shell(const fdtd_solver* s, const ClsBoxes& B) {
+bool boxes_clear_of_shell(const fdtd_solver* s, const ClsBoxes& B, int cells = 2) {
     for (int b = 0; b < B.n; ++b) {
         if (B.first[b + 1] == B.first[b]) continue;
         for (int d = 0; d < 3; ++d)
-            if (B.lo[b][d] < s->interior.lo[d] + 2 || B.lo[b][d] + B.rg[b][d] > s->interior.hi[d] - 2) return false;
+            if (B.lo[b][d] < s->interior.lo[d] + cells || B.lo[b][d] + B.rg[b][d] > s->interior.hi[d] - cells)
+                return false;
     }
     return true;
+}
+
+// How many cells from a fresh cell, along an axis, the cells of its fit may lie:
+// they enclose the image of the cell's centre behind the nearest body's surface,
+// as far beyond the cell as the surface is away (reflect_against_boundary).  The
+// cell was solid at the last classification, its centre within h/4 of a point of a
+// body that has since moved; so the surface is no farther than h/4 and the way that
+// point went, and the nearest body's no farther than that.  What a body adds:
+//   - an ellipsoid, whose distance is an estimate, too small by its axes' ratio at most;
+//   - a mesh, whose closest point is one of the nearest triangle's, but not always
+//     its nearest (tri_closest_ref): its longest edge.
+// FRESH_ANYWHERE: a cell may have left the scaled box of the body that held it; its
+// value then comes from the first body, wherever that is (lowest_object).
+constexpr int FRESH_ANYWHERE = 1 << 30;
+int fresh_reach(const fdtd_solver* s) {
+    if (s->cls_objs.size() != s->objs.size()) return FRESH_ANYWHERE;
+    double way = 0.0, ratio = 1.0, edge = 0.0;
+    for (size_t i = 0; i < s->objs.size(); ++i) {
+        const HostObject &was = s->cls_objs[i], &now = s->objs[i];
+        if (now.d.shape == FDTD_SHAPE_MESH) edge = std::max(edge, s->meshes[now.d.mesh].edge);
+        if (now.d.shape == FDTD_SHAPE_ELLIPSOID) {
+            const double* a = now.d.size;
+            ratio = std::max(ratio, std::max({a[0], a[1], a[2]}) / std::min({a[0], a[1], a[2]}));
+        }
+        if (now.d.motion == FDTD_MOTION_STATIC) continue;
+        double c2 = 0.0, turn2 = 0.0, r2 = 0.0;
+        for (int d = 0; d < 3; ++d) {
+            const double dc = now.c[d] - was.c[d];
+            const double e = now.d.shape == FDTD_SHAPE_MESH ? std::max(std::fabs(was.mlo[d]), std::fabs(was.mhi[d]))
+                                                            : now.d.size[d];
+            c2 += dc * dc;
+            r2 += e * e;
+            // where distance_to_mesh evaluates the distance (AABB_CHECK_TOLERANCE_SCALE)
+            const double mid = (now.bmax[d] + now.bmin[d]) / 2.0, half = 1.1 * (now.bmax[d] - now.bmin[d]);
+            const double out = 0.25 * s->h * (1.0 + 1e-6);
+            if (!(was.bmin[d] - out > mid - half && was.bmax[d] + out < mid + half)) return FRESH_ANYWHERE;
+        }
+        for (int k = 0; k < 9; ++k) {
+            const double dr = now.d.rotation[k] - was.d.rotation[k];
+            turn2 += dr * dr;
+        }
+        if (now.d.shape == FDTD_SHAPE_SPHERE) turn2 = 0.0;
+        way = std::max(way, std::sqrt(c2) + std::sqrt(turn2 * r2));
+    }
+    const double cells = ((way + 0.25 * s->h) * ratio + edge) / s->h * (1.0 + 1e-6);
+    return cells < 1e6 ? (int)cells + 1 : FRESH_ANYWHERE;  // (NaN and all)
 }
 
 // True when a Gaussian source may contribute at a step starting at time t:
@@ -138,8 +185,8 @@ fdtd_status join_listeners(fdtd_solver* s) {
 // last step's classification: `near` those within PLANES_REACH, `far` the others;
 // both empty when the far ones are too few to start apart.  The classification
 // touches cells one beyond a box, a fresh cell lies in the last step's box and its
-// fit reads p^n and p^{n-1} at most three cells from it, and the cells of both are
-// read one cell further.
+// fit reads p^n and p^{n-1} at most fresh_reach() cells from it (near planes go as
+// far where that is farther), and the cells of both are read one cell further.
 // Only where the interior is long enough to hide the classification behind and the
 // shell leaves it room (us a step, together / apart; two spheres):
 //   FP32  96^3 56.9 / 57.0, 160x150x170 66.7 / 62.9, 256^3 112.6 / 105.5,
@@ -148,16 +195,17 @@ fdtd_status join_listeners(fdtd_solver* s) {
 //         anyway)  224x200x210 120.2 / 122.6, 256^3 158.7 / 167.2
 constexpr int PLANES_REACH = 6;
 constexpr long long PLANES_CELLS = 2000000;
-void planes_ahead(const fdtd_solver* s, const ClsBoxes& prev, XRanges& far, XRanges& near) {
+void planes_ahead(const fdtd_solver* s, const ClsBoxes& prev, int fresh, XRanges& far, XRanges& near) {
     if (s->precision == FDTD_PRECISION_FP64 || s->n_interior < PLANES_CELLS) return;
     const int lo = s->region.interior.lo[0], hi = s->region.interior.hi[0];
-    if (hi <= lo) return;
+    if (hi <= lo || fresh >= hi - lo) return;
+    const int around = std::max(PLANES_REACH, fresh);
     std::vector<char> reach(hi - lo, 0);
     for (const ClsBoxes* B : {&prev, &s->hP.boxes})
         for (int b = 0; b < B->n; ++b) {
             if (B->first[b + 1] == B->first[b]) continue;
-            const int a = std::max(lo, B->lo[b][0] - PLANES_REACH);
-            const int e = std::min(hi, B->lo[b][0] + B->rg[b][0] + PLANES_REACH);
+            const int a = std::max(lo, B->lo[b][0] - around);
+            const int e = std::min(hi, B->lo[b][0] + B->rg[b][0] + around);
             for (int x = a; x < e; ++x) reach[x - lo] = 1;
         }
     auto push = [](XRanges& X, int a, int e) {
@@ -228,15 +276,19 @@ fdtd_status enqueue_step(fdtd_solver* s, int cur, double* dev_row, bool classify
         // Interior planes out of reach of the bodies' boxes hold no cell the
         // classification or the fresh cells touch or read: they start first, on
         // stream6, beside both.
+        const int fresh = s->moving && s->cls_boxes_current ? fresh_reach(s) : FRESH_ANYWHERE;
+        if (s->moving) s->cls_objs = s->objs;
         XRanges far{};
         if (s->moving && fused && s->cls_boxes_current && !s->hP.visc && s->eng.empty() && s->stream6 &&
             s->boundary_handling == FDTD_BOUNDARY_RASTERIZE && s->region.xb == 2)
-            planes_ahead(s, prev, far, near);
+            planes_ahead(s, prev, fresh, far, near);
         // Moving bodies clear of the PML: the shell kernel reads nothing the
-        // classification writes, so it starts first too.
+        // classification writes and writes nothing a fresh cell reads (FP64: p^{n-1},
+        // in the buffer of p^{n+1}), so it starts first too.
         shell_ahead = s->moving && fused && s->cls_boxes_current && s->n_solid_pml == 0 && !s->hP.visc &&
                       s->eng.empty() &&
-                      s->stream5 && s->interior.hi[0] > s->interior.lo[0] && boxes_clear_of_shell(s, prev) &&
+                      s->stream5 && s->interior.hi[0] > s->interior.lo[0] &&
+                      fresh < FRESH_ANYWHERE && boxes_clear_of_shell(s, prev, std::max(2, fresh)) &&
                       boxes_clear_of_shell(s, s->hP.boxes);
         if (shell_ahead || far.n > 0) {
             CUDA_TRY(s, cudaEventRecord(s->ev_sfork, s->stream));
