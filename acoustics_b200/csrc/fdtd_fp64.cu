@@ -1023,9 +1023,11 @@ __device__ __noinline__ double fresh_value_half(const SolveParams& P, const Fres
 // (p^n for w = 0, p^{n-1} for w = 1).  A list that overflowed is replaced by a
 // sweep over every cell, a thread per cell.  Each fresh value reads only cells
 // with a valid history, never another fresh cell (fresh_from_neighbour), so the
-// order does not matter.
+// order does not matter.  (Two CTAs per SM asked for: the compiler made room for three
+// otherwise, with 250 to 850 bytes of spills where two need none, and a step of
+// moving bodies took 0.5 % longer.)
 template <typename T>
-__global__ void __launch_bounds__(128) k_fresh_cells(const SolveParams* __restrict__ Pp, int cur, long long n,
+__global__ void __launch_bounds__(128, 2) k_fresh_cells(const SolveParams* __restrict__ Pp, int cur, long long n,
                                                      int* status) {
     const SolveParams& P = *Pp;
     const double t = P.consts[cur].t;
