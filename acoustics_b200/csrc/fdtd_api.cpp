@@ -479,7 +479,7 @@ fdtd_status run_classification(fdtd_solver* s) {
     classification_boxes(s, B);
     CUDA_TRY(s, fdtd::counted_copyAsync(s, &s->dP->boxes, &B, sizeof(ClsBoxes), cudaMemcpyHostToDevice, s->stream));
     int l = 0;  // (as by the step before the first one, whose parity is 0)
-    CUDA_TRY(s, launch_classify(s->dP, s->N, B, false, !s->mesh_alloc.empty(), 1, s->stream, &l));
+    CUDA_TRY(s, launch_classify(s->dP, s->N, B, false, cls_meshes(s), 1, s->stream, &l));
     s->cls_boxes_current = true;
     if (s->moving) s->cls_objs = s->objs;
     s->launches += l;
@@ -817,7 +817,8 @@ fdtd_status solver_init_geometry(fdtd_solver* s, const fdtd_scene_desc* sc) {
 
 }  // namespace fdtd
 
-static fdtd_status validate_scene(const fdtd_scene_desc* sc) {
+// meshes: the hierarchies of the scene's meshes that objects use, by mesh
+static fdtd_status validate_scene(const fdtd_scene_desc* sc, std::vector<MeshHost>& meshes) {
     if (!sc) return (set_error(nullptr, "scene is NULL"), FDTD_ERR_INVALID_ARG);
     if (!(sc->cell_size > 0) || !(sc->time_step > 0) || !(sc->sound_speed > 0) || !(sc->density > 0))
         return (set_error(nullptr, "cell_size, time_step, sound_speed and density must be positive"), FDTD_ERR_INVALID_ARG);
@@ -856,10 +857,10 @@ static fdtd_status validate_scene(const fdtd_scene_desc* sc) {
         if (o.shape == FDTD_SHAPE_MESH) {
             if (o.mesh < 0 || o.mesh >= sc->n_meshes)
                 return (set_error(nullptr, "object mesh index out of range"), FDTD_ERR_INVALID_ARG);
-            MeshHost m;
+            meshes.resize(sc->n_meshes);
             std::string err;
-            if (!build_mesh(sc->meshes[o.mesh], m, err)) return (set_error(nullptr, err), FDTD_ERR_GEOMETRY);
-
+            if (meshes[o.mesh].tris.empty() && !build_mesh(sc->meshes[o.mesh], meshes[o.mesh], err))
+                return (set_error(nullptr, err), FDTD_ERR_GEOMETRY);
         }
         if (o.accel_kind == FDTD_ACCEL_GAUSSIAN_PULSATION && o.shape != FDTD_SHAPE_SPHERE)
             return (set_error(nullptr, "pulsating acceleration is defined for spheres only"), FDTD_ERR_UNSUPPORTED);
@@ -1066,7 +1067,8 @@ fdtd_status fdtd_gaussian_source_defaults(fdtd_gaussian_source_desc* src, double
 fdtd_status fdtd_solver_create(const fdtd_scene_desc* sc, const fdtd_options* opt, fdtd_solver** out) {
     if (!out) return (set_error(nullptr, "out is NULL"), FDTD_ERR_INVALID_ARG);
     *out = nullptr;
-    fdtd_status st = validate_scene(sc);
+    std::vector<MeshHost> meshes;
+    fdtd_status st = validate_scene(sc, meshes);
     if (st != FDTD_OK) return st;
     fdtd_options o{};
     if (opt) o = *opt;
@@ -1151,17 +1153,11 @@ fdtd_status fdtd_solver_create(const fdtd_scene_desc* sc, const fdtd_options* op
         s->objs.push_back(h);
         if (h.d.motion != FDTD_MOTION_STATIC) s->moving = true;
     }
-    // meshes of the objects: hierarchy and pseudo-normals (validated above)
+    // meshes of the objects: hierarchy and pseudo-normals (made by the validation)
+    s->meshes.swap(meshes);
     s->meshes.resize(sc->n_meshes);
-    for (int i = 0; i < sc->n_objects; ++i) {
-        const int m = sc->objects[i].shape == FDTD_SHAPE_MESH ? sc->objects[i].mesh : -1;
-        if (m < 0 || !s->meshes[m].tris.empty()) continue;
-        std::string err;
-        if (!build_mesh(sc->meshes[m], s->meshes[m], err)) {
-            set_error(nullptr, err);
-            return FDTD_ERR_GEOMETRY;
-        }
-    }
+    for (int m = 0; m < sc->n_meshes; ++m)
+        if (!s->meshes[m].tris.empty()) s->meshes[m].solid = mesh_bounds_solid(sc->meshes[m], s->meshes[m]);
     // keyframe tracks and mesh vertices the objects read after creation: solver-owned copies
     s->kf_store.resize(s->objs.size());
     for (size_t i = 0; i < s->objs.size(); ++i) {
@@ -1218,7 +1214,7 @@ fdtd_status fdtd_solver_create(const fdtd_scene_desc* sc, const fdtd_options* op
         CUDA_TRY(nullptr, fdtd::counted_copy(s.get(), (char*)d + nb, M.tris.data(), tb, cudaMemcpyHostToDevice));
         CUDA_TRY(nullptr, fdtd::counted_copy(s.get(), (char*)d + nb + tb, M.top.data(), pb, cudaMemcpyHostToDevice));
         const MeshView v{(const MeshNode*)d, (const MeshTri*)((char*)d + nb), (int)M.nodes.size(), (int)M.tris.size(),
-                         (const int*)((char*)d + nb + tb), (int)M.top.size()};
+                         (const int*)((char*)d + nb + tb), (int)M.top.size(), M.solid ? 1 : 0};
         for (auto& o : s->objs)
             if (o.d.shape == FDTD_SHAPE_MESH && o.d.mesh == (int)m) o.mview = v;
     }
@@ -1496,7 +1492,8 @@ fdtd_status fdtd_solver_reset(fdtd_solver* s, double t0) {
 
 fdtd_status fdtd_scene_info(const fdtd_scene_desc* sc, const fdtd_options* opt, fdtd_solver_info* info) {
     if (!info) return (set_error(nullptr, "info is NULL"), FDTD_ERR_INVALID_ARG);
-    fdtd_status st = validate_scene(sc);
+    std::vector<MeshHost> meshes;
+    fdtd_status st = validate_scene(sc, meshes);
     if (st != FDTD_OK) return st;
     fdtd_options o{};
     if (opt) o = *opt;

@@ -269,7 +269,7 @@ fdtd_status build_fully_coupled(fdtd_solver* s) {
     for (size_t i = 0; i < hobj.size() && i < s->objs.size(); ++i)
         if (hobj[i].shape == FDTD_SHAPE_MESH) {
             const MeshHost& M = s->meshes[s->objs[i].d.mesh];
-            hobj[i].mesh = MeshView{M.nodes.data(), M.tris.data(), (int)M.nodes.size(), (int)M.tris.size(), nullptr, 0};
+            hobj[i].mesh = MeshView{M.nodes.data(), M.tris.data(), (int)M.nodes.size(), (int)M.tris.size(), nullptr, 0, M.solid ? 1 : 0};
         }
     for (long long ri = 0; ri < nrow; ++ri) {
         FcRow& r = rows[ri];

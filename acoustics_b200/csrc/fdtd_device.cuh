@@ -75,6 +75,9 @@ struct DevSource {
 
 constexpr int CLS_MAX_BOXES_X = FDTD_MAX_OBJECTS + 4;  // CLS_MAX_BOXES
 
+// Mesh bodies a classification meets: none, all bounding solids (MeshView::solid), or not all.
+enum ClsMeshes { CLS_MESHES_NONE, CLS_MESHES_SOLID, CLS_MESHES_LOOSE };
+
 // Non-PML box [lo, hi) of the grid.
 struct Box3 {
     int lo[3];

@@ -118,6 +118,8 @@ __global__ void __launch_bounds__(128) k_cls_boxes(const SolveParams* __restrict
 // by d's sign (a distance changes by no more than the point moves).  In the other
 // bricks the warps share the cells, a walk each bounded by |d| plus the way to
 // the centre, and then the samples of the cells within h/4 of the surface.
+// Neither holds for a mesh that bounds no solid (MeshView::solid), whose sign may
+// change away from its surface: every cell walks, and every sample of a fluid one.
 // Every point that is evaluated is evaluated as is_fluid evaluates it, so the
 // flags are the same bit for bit.
 // A walk is a chain of dependent loads, so what counts is walks in flight: the
@@ -131,6 +133,8 @@ __host__ __device__ inline int cls_bricks(const ClsBoxes& B, int b) {
 
 constexpr int CLS_MESH_WARPS = 8;
 
+// LOOSE: some mesh bounds no solid.
+template <bool LOOSE>
 __global__ void __launch_bounds__(32 * CLS_MESH_WARPS, 3) k_cls_boxes_mesh(const SolveParams* __restrict__ Pp) {
     enum : int { OFF = 0, FLUID = 1, SOLID = 2 };
     __shared__ int stacks[CLS_MESH_WARPS][MESH_WARP_STACK];
@@ -142,6 +146,7 @@ __global__ void __launch_bounds__(32 * CLS_MESH_WARPS, 3) k_cls_boxes_mesh(const
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int* stack = stacks[warp];
     const double h = P.h, reach = sample_reach(P);
+    auto loose = [](const DevObject& O) { return LOOSE && O.shape == 3 && !O.mesh.solid; };
     // the farthest cell centre of a brick lies (h/2, 3h/2, 3h/2) from its centre
     const double brick_r = h * 2.179449471770337 * (1.0 + 1e-6) + reach;
     int b = 0, b0 = 0;  // box of the brick and the bricks of the boxes before it
@@ -173,7 +178,7 @@ __global__ void __launch_bounds__(32 * CLS_MESH_WARPS, 3) k_cls_boxes_mesh(const
         }
         for (int o = 0; o < P.n_obj; ++o) {
             const DevObject& O = P.obj[o];
-            if (beyond_bbox(O, ctr, brick_r)) continue;  // uniform: ctr and O are
+            if (!loose(O) && beyond_bbox(O, ctr, brick_r)) continue;  // uniform: ctr and O are
             __syncthreads();
             if (O.shape != 3) {
                 // analytic: a cell per lane, as is_fluid
@@ -202,24 +207,24 @@ __global__ void __launch_bounds__(32 * CLS_MESH_WARPS, 3) k_cls_boxes_mesh(const
                     centre_d = d;
                     n_near = 0;
                 }
-                if (fabs(d) > brick_r && d < 0.0 && state[lane] == FLUID) state[lane] = SOLID;
+                if (!loose(O) && fabs(d) > brick_r && d < 0.0 && state[lane] == FLUID) state[lane] = SOLID;
             }
             __syncthreads();
             const double dc = centre_d;
-            if (fabs(dc) > brick_r) continue;
+            if (!loose(O) && fabs(dc) > brick_r) continue;
             for (int c = warp; c < 32; c += CLS_MESH_WARPS) {
                 if (state[c] != FLUID) continue;
                 double pos[3], q[3];
                 cell_pos(c, pos);
-                if (beyond_bbox(O, pos, reach)) continue;
+                if (!loose(O) && beyond_bbox(O, pos, reach)) continue;
                 const double x = pos[0] - ctr[0], y = pos[1] - ctr[1], z = pos[2] - ctr[2];
                 const double far = (fabs(dc) + sqrt(x * x + y * y + z * z)) * (1.0 + 1e-6) + 1e-6 * h;
                 to_object_frame(O, pos, q);
                 const double d = mesh_sdf_warp(O.mesh, q, far * far, stack);
                 if (lane == 0) {
-                    if (d < DISTANCE_TOLERANCE) {
+                    if (d < DISTANCE_TOLERANCE && (!loose(O) || in_scaled_bbox(O, pos))) {
                         state[c] = SOLID;
-                    } else if (d <= reach) {
+                    } else if (d <= reach || loose(O)) {
                         const int s = atomicAdd(&n_near, 1);
                         near_cell[s] = c;
                         near_d[s] = d;
@@ -234,7 +239,7 @@ __global__ void __launch_bounds__(32 * CLS_MESH_WARPS, 3) k_cls_boxes_mesh(const
                 cell_pos(c, pos);
                 pos[a] = pos[a] + ((s & 1) ? 1.0 : -1.0) * 0.25 * h;
                 if (!in_scaled_bbox(O, pos)) continue;
-                const double far = (near_d[s / 6] + 0.25 * h) * (1.0 + 1e-6) + 1e-6 * h;
+                const double far = (fabs(near_d[s / 6]) + 0.25 * h) * (1.0 + 1e-6) + 1e-6 * h;
                 to_object_frame(O, pos, q);
                 const double d = mesh_sdf_warp(O.mesh, q, far * far, stack);
                 if (lane == 0 && d < DISTANCE_TOLERANCE) state[c] = SOLID;
@@ -1024,7 +1029,7 @@ __device__ __noinline__ double fresh_value_half(const SolveParams& P, const Fres
 // sweep over every cell, a thread per cell.  Each fresh value reads only cells
 // with a valid history, never another fresh cell (fresh_from_neighbour), so the
 // order does not matter.  (Two CTAs per SM asked for: the compiler made room for three
-// otherwise, with 250 to 850 bytes of spills where two need none, and a step of
+// otherwise, spilling 256 bytes in fresh_value and 112 here, where two need none, and a step of
 // moving bodies took 0.5 % longer.)
 template <typename T>
 __global__ void __launch_bounds__(128, 2) k_fresh_cells(const SolveParams* __restrict__ Pp, int cur, long long n,
@@ -1245,20 +1250,21 @@ cudaError_t launch_static_prep(SolveParams* dP, int precision, int newp, int n_l
     return cudaGetLastError();
 }
 
-cudaError_t launch_classify(const SolveParams* dP, const int N[3], const ClsBoxes& B, bool collect_fresh, bool meshes,
+cudaError_t launch_classify(const SolveParams* dP, const int N[3], const ClsBoxes& B, bool collect_fresh, ClsMeshes meshes,
                             int cur, cudaStream_t s, int* launches, const ClsBoxes* prev) {
     const int fresh = collect_fresh ? 1 : 0;
-    if (prev && !meshes) {
+    if (prev && meshes == CLS_MESHES_NONE) {
         const ClsTiles T = cls_tiles(N, B, *prev);
         if (launches) *launches += 1;
         k_cls_tiles<<<(unsigned)std::max(T.first[T.n], 1), 256, 0, s>>>(dP, T, cur);
         return cudaGetLastError();
     }
     if (launches) *launches += B.ufirst[B.n] > 0 ? 3 : 2;
-    if (meshes) {
+    if (meshes != CLS_MESHES_NONE) {
         long long bricks = 1;  // (one CTA at least: it empties the lists)
         for (int b = 0; b < B.n; ++b) bricks += cls_bricks(B, b);
-        k_cls_boxes_mesh<<<grid_for(bricks, 1), 32 * CLS_MESH_WARPS, 0, s>>>(dP);
+        const auto kernel = meshes == CLS_MESHES_LOOSE ? k_cls_boxes_mesh<true> : k_cls_boxes_mesh<false>;
+        kernel<<<grid_for(bricks, 1), 32 * CLS_MESH_WARPS, 0, s>>>(dP);
     } else {
         k_cls_boxes<<<grid_for(B.first[B.n], 128), 128, 0, s>>>(dP);
     }

@@ -97,16 +97,19 @@ FDTD_HD bool beyond_bbox(const DevObject& o, const double p[3], double reach) {
 // The samples are tried only against the bodies that can reach one: a body
 // whose box, or whose surface, is farther than h/4 from the centre cannot (the
 // distances of spheres, boxes and meshes are exact; an ellipsoid's is an
-// estimate with the exact sign, so its samples are always tried).
+// estimate with the exact sign, so its samples are always tried).  A mesh that
+// bounds no solid may be negative anywhere in its scaled box.
 FDTD_HD bool is_fluid(const SolveParams& P, const double pos[3], int& type) {
     bool fluid = !occupy_by_constraint(P, pos);
     const double reach = sample_reach(P);
     unsigned near = 0;
     for (int o = 0; o < P.n_obj && fluid; ++o) {
-        if (beyond_bbox(P.obj[o], pos, reach)) continue;
-        const double dist = sdf_local(P.obj[o], pos);
+        const DevObject& O = P.obj[o];
+        const bool loose = O.shape == 3 && !O.mesh.solid;
+        if (!loose && beyond_bbox(O, pos, reach)) continue;
+        const double dist = loose ? distance_to_mesh(O, pos) : sdf_local(O, pos);
         if (dist < DISTANCE_TOLERANCE) fluid = false;
-        else if (dist <= reach || P.obj[o].shape == 2) near |= 1u << o;
+        else if (dist <= reach || O.shape == 2 || loose) near |= 1u << o;
     }
     for (int d = 0; d < 3 && fluid && near; ++d) {
         for (int s = -1; s <= 1 && fluid; s += 2) {

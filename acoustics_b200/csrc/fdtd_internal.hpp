@@ -39,8 +39,11 @@ struct MeshHost {
     std::vector<int> top;       // MeshView::top
     std::vector<double> vertices;
     double edge = 0;            // longest edge
+    bool solid = false;         // MeshView::solid
 };
 bool build_mesh(const fdtd_mesh_desc& md, MeshHost& out, std::string& err);
+// MeshView::solid of a mesh that build_mesh made of md; false where in doubt
+bool mesh_bounds_solid(const fdtd_mesh_desc& md, const MeshHost& M);
 void mesh_extent(const double* verts, size_t nv, const double R[9], double lo[3], double hi[3]);
 // A host object of scene object i at rest (mesh extent set; pose and box not yet).
 HostObject make_host_object(const fdtd_scene_desc* sc, int i);
@@ -182,6 +185,12 @@ inline size_t status_bytes(const fdtd_solver* s) {
     return (size_t)((const char*)(s->d_ghost_count + 4) - (const char*)s->hP.dev_error);
 }
 void set_error(fdtd_solver* s, const std::string& msg);
+inline ClsMeshes cls_meshes(const fdtd_solver* s) {
+    ClsMeshes k = CLS_MESHES_NONE;
+    for (const MeshHost& m : s->meshes)
+        if (!m.tris.empty()) k = m.solid && k != CLS_MESHES_LOOSE ? CLS_MESHES_SOLID : CLS_MESHES_LOOSE;
+    return k;
+}
 // no listener stencil meets a classification box (fdtd_step.cpp)
 bool listeners_clear_of(const fdtd_solver* s, const ClsBoxes& B);
 // moving bodies two cells clear of the PML through [start_time, end_time]

@@ -51,9 +51,9 @@ cudaError_t launch_listeners(const SolveParams* dP, int precision, int newp, int
 // (3 launches; the last only when some box has cells).  With `prev` (the boxes
 // of the classification before, when every cell outside them is known to hold
 // the default flags) the first sweep visits only the units those reached.
-// `meshes`: some body is a triangle mesh (the solid test by warps).
+// `meshes`: the scene's mesh bodies (the solid test by warps).
 // Analytic bodies then take one launch (k_cls_tiles).  cur: the step's parity.
-cudaError_t launch_classify(const SolveParams* dP, const int N[3], const ClsBoxes& B, bool collect_fresh, bool meshes,
+cudaError_t launch_classify(const SolveParams* dP, const int N[3], const ClsBoxes& B, bool collect_fresh, ClsMeshes meshes,
                             int cur, cudaStream_t s, int* launches, const ClsBoxes* prev = nullptr);
 cudaError_t launch_cls_history(const SolveParams* dP, long long ncell, int* count, int* list, int cap, cudaStream_t s);
 cudaError_t launch_fresh_cells(const SolveParams* dP, int precision, int cur, long long ncell, int* d_status,

@@ -58,6 +58,9 @@ struct MeshView {
     // above that), at most MESH_TOP; only device views have them
     const int* top;
     int n_top;
+    // the mesh bounds a solid (mesh_bounds_solid): its signed distance changes sign at
+    // the surface only, so a ball that the surface does not meet lies on one side of it
+    int solid;
 };
 constexpr int MESH_TOP = 32;
 

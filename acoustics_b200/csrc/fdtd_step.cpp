@@ -36,7 +36,7 @@ void classification_launches(fdtd_solver* s, int cur, fdtd_status& st, const Cls
     // pageable source: the copy is staged before the call returns
     cudaError_t e = fdtd::counted_copyAsync(s, &s->dP->boxes, &B, sizeof(ClsBoxes), cudaMemcpyHostToDevice, s->stream);
     int l = 0;
-    if (e == cudaSuccess) e = launch_classify(s->dP, s->N, B, s->moving, !s->mesh_alloc.empty(), cur, s->stream, &l, prev);
+    if (e == cudaSuccess) e = launch_classify(s->dP, s->N, B, s->moving, cls_meshes(s), cur, s->stream, &l, prev);
     s->launches += l;
     if (e != cudaSuccess) {
         set_error(s, std::string("classification launch: ") + cudaGetErrorString(e));
@@ -81,6 +81,8 @@ int fresh_reach(const fdtd_solver* s) {
             ratio = std::max(ratio, std::max({a[0], a[1], a[2]}) / std::min({a[0], a[1], a[2]}));
         }
         if (now.d.motion == FDTD_MOTION_STATIC) continue;
+        // (solid cells of a mesh that bounds no solid may lie far from its surface)
+        if (now.d.shape == FDTD_SHAPE_MESH && !s->meshes[now.d.mesh].solid) return FRESH_ANYWHERE;
         double c2 = 0.0, turn2 = 0.0, r2 = 0.0;
         for (int d = 0; d < 3; ++d) {
             const double dc = now.c[d] - was.c[d];
