@@ -92,6 +92,15 @@ FDTD_HD bool beyond_bbox(const DevObject& o, const double p[3], double reach) {
     return false;
 }
 
+// p lies in the body's scaled box, where distance_to_mesh evaluates the distance.
+FDTD_HD bool in_scaled_bbox(const DevObject& o, const double p[3]) {
+    for (int d = 0; d < 3; ++d) {
+        const double sd = o.bdim[d] * AABB_CHECK_TOLERANCE_SCALE;
+        if (!(p[d] < (o.bcen[d] + sd) && p[d] > (o.bcen[d] - sd))) return false;
+    }
+    return true;
+}
+
 // isFluid lambda of classifyCells_FAST (MAC_Grid.cpp:3566-3577): the centre and
 // the six points centre +- h/4 along each axis must be outside every object.
 // The samples are tried only against the bodies that can reach one: a body
@@ -107,7 +116,7 @@ FDTD_HD bool is_fluid(const SolveParams& P, const double pos[3], int& type) {
         const DevObject& O = P.obj[o];
         const bool loose = O.shape == 3 && !O.mesh.solid;
         if (!loose && beyond_bbox(O, pos, reach)) continue;
-        const double dist = loose ? distance_to_mesh(O, pos) : sdf_local(O, pos);
+        const double dist = loose && !in_scaled_bbox(O, pos) ? DBL_MAX : sdf_local(O, pos);
         if (dist < DISTANCE_TOLERANCE) fluid = false;
         else if (dist <= reach || O.shape == 2 || loose) near |= 1u << o;
     }
@@ -121,15 +130,6 @@ FDTD_HD bool is_fluid(const SolveParams& P, const double pos[3], int& type) {
     }
     if (!fluid) type = occupy_by_constraint(P, pos) ? 1 : 0;
     return fluid;
-}
-
-// p lies in the body's scaled box, where distance_to_mesh evaluates the distance.
-FDTD_HD bool in_scaled_bbox(const DevObject& o, const double p[3]) {
-    for (int d = 0; d < 3; ++d) {
-        const double sd = o.bdim[d] * AABB_CHECK_TOLERANCE_SCALE;
-        if (!(p[d] < (o.bcen[d] + sd) && p[d] > (o.bcen[d] - sd))) return false;
-    }
-    return true;
 }
 
 // FDTD_Objects::LowestObjectDistance (FDTD_Objects.cpp:240-257): first object
