@@ -90,11 +90,11 @@ constexpr int NOALLOC_PLANES = 2;
 __global__ void __launch_bounds__(256) k_noalloc_step(const double* __restrict__ pc, const double* pl, double* pn, int ny,
                                                       int nz, int lo0, int lo1, int lo2, int bx, int by, int bz,
                                                       double c2k2, double scale) {
-    const int u = blockIdx.x * 256 + threadIdx.x;
+    const int u = blockIdx.y * 256 + threadIdx.x;
     if (u >= by * bz) return;
     const int row = u / bz;
     const int sx = ny * nz;  // the grid has fewer than 2^31 cells
-    const int x0 = blockIdx.y * NOALLOC_PLANES, nx = min(NOALLOC_PLANES, bx - x0);
+    const int x0 = blockIdx.x * NOALLOC_PLANES, nx = min(NOALLOC_PLANES, bx - x0);
     const int c0 = (lo0 + x0) * sx + (lo1 + row) * nz + lo2 + (u - row * bz);
     double col[NOALLOC_PLANES + 2], ym[NOALLOC_PLANES], yp[NOALLOC_PLANES], zm[NOALLOC_PLANES], zp[NOALLOC_PLANES],
         old[NOALLOC_PLANES];
@@ -194,7 +194,9 @@ fdtd_status fdtd_interior_step_noalloc(const double* p_curr, const double* p_pre
     const uintptr_t bytes = (uintptr_t)dims[0] * dims[1] * dims[2] * sizeof(double);
     const uintptr_t a = (uintptr_t)p_curr, b = (uintptr_t)p_next;
     if (b >= a + bytes || a >= b + bytes) {
-        const dim3 grid((unsigned)((by * bz + 255) / 256), (unsigned)((bx + NOALLOC_PLANES - 1) / NOALLOC_PLANES));
+        // x tiles in the dimension without a limit in reach: at most 2^19 of them, and
+        // 2^12 blocks of columns, of the FDTD_NOALLOC_MAX_CELLS a box may have
+        const dim3 grid((unsigned)((bx + NOALLOC_PLANES - 1) / NOALLOC_PLANES), (unsigned)((by * bz + 255) / 256));
         k_noalloc_step<<<grid, 256, 0, s>>>(p_curr, p_prev, p_next, dims[1], dims[2], lo[0], lo[1], lo[2], bx, by, bz,
                                             c2k2, lap_scale);
         const cudaError_t e = cudaGetLastError();
