@@ -1374,6 +1374,8 @@ fdtd_status fdtd_solver_destroy(fdtd_solver* s) {
     free_fully_coupled(s);
     free_shell_tma(s);
     for (void* p : s->mesh_alloc) cudaFree(p);
+    if (s->held) cudaFree(s->held);
+    if (s->ev_held) cudaEventDestroy(s->ev_held);
     if (s->d_solid_pml) cudaFree(s->d_solid_pml);
     if (s->arena) arena_release(s->opt.device, s->arena, s->arena_block);
     host_release(s->h_lis_stage, s->h_lis_bytes);

@@ -733,6 +733,10 @@ __device__ __forceinline__ double fresh_from_neighbour(const SolveParams& P, lon
     return 0.0;
 }
 
+__device__ __forceinline__ bool in_pml(const SolveParams& P, int i, int j, int k) {
+    return P.pml_cell[0][i] || P.pml_cell[1][j] || P.pml_cell[2][k];
+}
+
 // ---------------------------------------------------------------------------
 // Fresh-cell interpolation (MAC_Grid::InterpolateFreshPressureCell, MLS branch,
 // MAC_Grid.cpp:1993-2254): a cell that is bulk now but was solid before gets
@@ -743,8 +747,9 @@ __device__ __forceinline__ double fresh_from_neighbour(const SolveParams& P, lon
 template <typename T>
 __device__ __noinline__ double fresh_value(const SolveParams& P, const T* __restrict__ pa, const T* __restrict__ pb,
                                            bool diff, long long c, double t, int* status, long long& next) {
-    // value of buffer "a" (or a - b when diff) at cell n
+    // value of buffer "a" (or a - b when diff) at cell n, of the stencil in the PML where it is held
     auto val = [&](long long n) -> double { return diff ? (double)pa[n] - (double)pb[n] : (double)pa[n]; };
+    const bool held = !diff && pb != pa;
     int i, j, k;
     cell_ijk(P, c, i, j, k);
     const double cp[3] = {P.cpos[0][i], P.cpos[1][j], P.cpos[2][k]};
@@ -770,7 +775,7 @@ __device__ __noinline__ double fresh_value(const SolveParams& P, const T* __rest
         int ni, nj, nn;
         cell_ijk(P, n, ni, nj, nn);
         code[q] = P.cls[n];
-        vals[q] = val(n);
+        vals[q] = held && in_pml(P, ni, nj, nn) ? (double)pb[n] : val(n);
         npos[q][0] = P.cpos[0][ni];
         npos[q][1] = P.cpos[1][nj];
         npos[q][2] = P.cpos[2][nn];
@@ -815,7 +820,8 @@ __device__ __noinline__ double fresh_value(const SolveParams& P, const T* __rest
 }
 
 template <typename T>
-__device__ __forceinline__ void fresh_cell(const SolveParams& P, int cur, long long c, double t, int* st) {
+__device__ __forceinline__ void fresh_cell(const SolveParams& P, int cur, long long c, double t, int* st,
+                                           const T* held) {
     // (the cell itself, or the one its value is a copy of)
     auto value = [&](const T* pa, const T* pb, bool diff) {
         double v = 0.0;
@@ -829,7 +835,7 @@ __device__ __forceinline__ void fresh_cell(const SolveParams& P, int cur, long l
     if (sizeof(T) == 8) {
         T* pl = (T*)P.p[cur ^ 1];
         T* pc = (T*)P.p[cur];
-        const double vl = value(pl, pl, false);
+        const double vl = value(pl, held ? held : pl, false);
         const double vc = value(pc, pc, false);
         pl[c] = vl;
         pc[c] = vc;
@@ -934,7 +940,8 @@ __device__ __noinline__ double fresh_value_half(const SolveParams& P, const Fres
     if (in_stencil) {
         const long long n = cidx(P, ni, nj, nn);
         valid = (P.cls[n] & CLS_VALID) != 0;
-        vq = diff ? (double)pa[n] - (double)pb[n] : (double)pa[n];
+        const bool held = !diff && pb != pa && in_pml(P, ni, nj, nn);
+        vq = diff ? (double)pa[n] - (double)pb[n] : held ? (double)pb[n] : (double)pa[n];
         pq[0] = P.cpos[0][ni];
         pq[1] = P.cpos[1][nj];
         pq[2] = P.cpos[2][nn];
@@ -1033,7 +1040,7 @@ __device__ __noinline__ double fresh_value_half(const SolveParams& P, const Fres
 // moving bodies took 0.5 % longer.)
 template <typename T>
 __global__ void __launch_bounds__(128, 2) k_fresh_cells(const SolveParams* __restrict__ Pp, int cur, long long n,
-                                                     int* status) {
+                                                     int* status, const T* held) {
     const SolveParams& P = *Pp;
     const double t = P.consts[cur].t;
     const int count = list_counts(P, cur)[1];
@@ -1046,7 +1053,7 @@ __global__ void __launch_bounds__(128, 2) k_fresh_cells(const SolveParams* __res
             const long long c = cidx(P, i, j, k);
             const uint8_t code = P.cls[c];
             if (!(code & CLS_BULK) || (code & CLS_VALID)) continue;
-            fresh_cell<T>(P, cur, c, t, &st);
+            fresh_cell<T>(P, cur, c, t, &st, held);
         }
         if (st) atomicMax(status, st);
         return;
@@ -1061,9 +1068,9 @@ __global__ void __launch_bounds__(128, 2) k_fresh_cells(const SolveParams* __res
             FreshGeometry G;
             long long next = -1;
             if (fresh_geometry(P, at, stacks[threadIdx.x >> 5], G)) {
-                // FP32: p^{n-1} is p^n less the increment
+                // FP32: p^{n-1} is p^n less the increment; FP64: in the PML held apart, or not
                 const T* pa = (const T*)P.p[sizeof(T) == 8 ? cur ^ w : cur];
-                const T* pb = sizeof(T) == 8 ? pa : (const T*)(const void*)P.dinc;
+                const T* pb = sizeof(T) == 4 ? (const T*)(const void*)P.dinc : w && held ? held : pa;
                 v = fresh_value_half<T>(P, G, pa, pb, sizeof(T) == 4 && w, at, t, next);
             } else {
                 st = 2;
@@ -1308,11 +1315,11 @@ cudaError_t launch_cls_history(const SolveParams* dP, long long ncell, int* coun
 }
 
 cudaError_t launch_fresh_cells(const SolveParams* dP, int precision, int cur, long long ncell, int* d_status,
-                               cudaStream_t s) {
+                               cudaStream_t s, const double* held) {
     // the list, a warp per cell (a few thousand cells a step at most)
     const int grid = 4 * 148;
-    if (precision == 0) k_fresh_cells<double><<<grid, 128, 0, s>>>(dP, cur, ncell, d_status);
-    else k_fresh_cells<float><<<grid, 128, 0, s>>>(dP, cur, ncell, d_status);
+    if (precision == 0) k_fresh_cells<double><<<grid, 128, 0, s>>>(dP, cur, ncell, d_status, held);
+    else k_fresh_cells<float><<<grid, 128, 0, s>>>(dP, cur, ncell, d_status, nullptr);
     return cudaGetLastError();
 }
 

@@ -87,6 +87,10 @@ struct fdtd_solver {
     // solid cells lie in them); cleared when the flags are loaded from elsewhere
     bool cls_boxes_current = false;
     std::vector<fdtd::HostObject> cls_objs;  // moving scenes: the bodies as that classification found them
+    // FP64, made when first needed: p^{n-1} for fits that may lie in the PML, whose shell
+    // starts ahead and writes over it
+    double* held = nullptr;
+    cudaEvent_t ev_held = nullptr;
     bool lis_clear = false;         // listeners_clear_of the boxes of the last reset
     long long overlapped_steps = 0;
     // geometry

@@ -56,8 +56,9 @@ cudaError_t launch_listeners(const SolveParams* dP, int precision, int newp, int
 cudaError_t launch_classify(const SolveParams* dP, const int N[3], const ClsBoxes& B, bool collect_fresh, ClsMeshes meshes,
                             int cur, cudaStream_t s, int* launches, const ClsBoxes* prev = nullptr);
 cudaError_t launch_cls_history(const SolveParams* dP, long long ncell, int* count, int* list, int cap, cudaStream_t s);
+// held: where the PML cells' p^{n-1} is read (null: where p^{n+1} goes; FP64)
 cudaError_t launch_fresh_cells(const SolveParams* dP, int precision, int cur, long long ncell, int* d_status,
-                               cudaStream_t s);
+                               cudaStream_t s, const double* held = nullptr);
 
 // plain FP64 path, one kernel per reference phase
 cudaError_t launch_phased_fp64(const SolveParams* dP, const int N[3], int cur, double* lap, cudaStream_t s,

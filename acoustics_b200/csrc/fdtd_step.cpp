@@ -228,6 +228,20 @@ void planes_ahead(const fdtd_solver* s, const ClsBoxes& prev, int fresh, XRanges
     if (4 * n_far < hi - lo || near.n == 0) far.n = near.n = 0;
 }
 
+// Room to hold p^{n-1} (FP64); false: none to be had.
+bool make_held(fdtd_solver* s) {
+    void* d = nullptr;
+    if (cudaMalloc(&d, (size_t)s->np * 8) != cudaSuccess ||
+        (!s->ev_held && cudaEventCreateWithFlags(&s->ev_held, cudaEventDisableTiming) != cudaSuccess)) {
+        cudaGetLastError();
+        if (d) cudaFree(d);
+        return false;
+    }
+    s->held = (double*)d;
+    s->arena_bytes += (size_t)s->np * 8;
+    return true;
+}
+
 // The row a one-launch step left to its successor; newp: the parity of the
 // current pressure.
 fdtd_status flush_lag(fdtd_solver* s, int newp) {
@@ -285,13 +299,17 @@ fdtd_status enqueue_step(fdtd_solver* s, int cur, double* dev_row, bool classify
             s->boundary_handling == FDTD_BOUNDARY_RASTERIZE && s->region.xb == 2)
             planes_ahead(s, prev, fresh, far, near);
         // Moving bodies clear of the PML: the shell kernel reads nothing the
-        // classification writes and writes nothing a fresh cell reads (FP64: p^{n-1},
-        // in the buffer of p^{n+1}), so it starts first too.
+        // classification writes, so it starts first too.  In FP64 it writes p^{n+1} over
+        // p^{n-1}, which a fresh cell's fit that lies in the PML (a body gone many cells
+        // in this step) then reads from a copy made before.
         shell_ahead = s->moving && fused && s->cls_boxes_current && s->n_solid_pml == 0 && !s->hP.visc &&
                       s->eng.empty() &&
-                      s->stream5 && s->interior.hi[0] > s->interior.lo[0] &&
-                      fresh < FRESH_ANYWHERE && boxes_clear_of_shell(s, prev, std::max(2, fresh)) &&
+                      s->stream5 && s->interior.hi[0] > s->interior.lo[0] && boxes_clear_of_shell(s, prev) &&
                       boxes_clear_of_shell(s, s->hP.boxes);
+        const bool hold = shell_ahead && s->precision == FDTD_PRECISION_FP64 &&
+                          !(fresh < FRESH_ANYWHERE && boxes_clear_of_shell(s, prev, fresh));
+        if (hold && !s->held) shell_ahead = make_held(s);
+        const double* held = hold && shell_ahead ? s->held : nullptr;
         if (shell_ahead || far.n > 0) {
             CUDA_TRY(s, cudaEventRecord(s->ev_sfork, s->stream));
             const auto ahead = [&](cudaStream_t on, cudaEvent_t done, int skip, const XRanges& planes) -> fdtd_status {
@@ -316,6 +334,12 @@ fdtd_status enqueue_step(fdtd_solver* s, int cur, double* dev_row, bool classify
                 const fdtd_status fst = ahead(s->stream6, s->ev_fdone, 2, far);
                 if (fst != FDTD_OK) return fst;
             }
+            if (held) {
+                // (the classification zeroes cells of bodies meanwhile, which are not PML cells)
+                CUDA_TRY(s, cudaStreamWaitEvent(s->stream5, s->ev_sfork, 0));
+                CUDA_TRY(s, cudaMemcpyAsync(s->held, s->hP.p[cur ^ 1], (size_t)s->np * 8, cudaMemcpyDeviceToDevice, s->stream5));
+                CUDA_TRY(s, cudaEventRecord(s->ev_held, s->stream5));
+            }
             if (shell_ahead) {
                 const fdtd_status sst = ahead(s->stream5, s->ev_sdone, 1, XRanges{});
                 if (sst != FDTD_OK) return sst;
@@ -330,7 +354,8 @@ fdtd_status enqueue_step(fdtd_solver* s, int cur, double* dev_row, bool classify
         s->cls_boxes_current = true;
         if (st != FDTD_OK) return st;
         if (s->moving) {
-            CUDA_TRY(s, launch_fresh_cells(s->dP, s->precision, cur, s->ncell, s->d_status, s->stream));
+            if (held) CUDA_TRY(s, cudaStreamWaitEvent(s->stream, s->ev_held, 0));
+            CUDA_TRY(s, launch_fresh_cells(s->dP, s->precision, cur, s->ncell, s->d_status, s->stream, held));
             s->launches++;
             if (s->boundary_handling == FDTD_BOUNDARY_FULLY_COUPLED) {
                 // the coupled rows of this step's ghost faces (host build from the new flags)
