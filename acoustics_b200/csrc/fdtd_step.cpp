@@ -1125,8 +1125,17 @@ struct SnapHeader {
     int32_t precision, kernel, cur, n_obj;
     int64_t step_index;
     double time, state_time;
+    int64_t total;  // bytes, this header's too
 };
-const uint64_t SNAP_MAGIC = 0x314e53445446ULL;  // "FTDSN1"
+// The regions are raw copies, so a change of what they hold (StepConsts, HostObject, the
+// arrays of a solve) is another layout and takes another number.
+const uint64_t SNAP_MAGIC = 0x324e53445446ULL;  // "FTDSN2"
+
+size_t snap_total(fdtd_solver* s, const std::vector<std::pair<void*, size_t>>& regs) {
+    size_t total = sizeof(SnapHeader) + s->objs.size() * sizeof(HostObject);
+    for (const auto& r : regs) total += r.second;
+    return total;
+}
 
 std::vector<std::pair<void*, size_t>> snap_regions(fdtd_solver* s) {
     const SolveParams& P = s->hP;
@@ -1211,8 +1220,7 @@ extern "C" {
 fdtd_status fdtd_solver_snapshot(fdtd_solver* s, void* buffer, int64_t* bytes) {
     if (!s || !bytes) return FDTD_ERR_INVALID_ARG;
     auto regs = snap_regions(s);
-    size_t total = sizeof(SnapHeader) + s->objs.size() * sizeof(HostObject);
-    for (auto& r : regs) total += r.second;
+    const size_t total = snap_total(s, regs);
     if (!buffer) {
         *bytes = (int64_t)total;
         return FDTD_OK;
@@ -1220,7 +1228,7 @@ fdtd_status fdtd_solver_snapshot(fdtd_solver* s, void* buffer, int64_t* bytes) {
     if (*bytes < (int64_t)total) return (set_error(s, "snapshot buffer too small"), FDTD_ERR_INVALID_ARG);
     CUDA_TRY(s, cudaSetDevice(s->opt.device));
     SnapHeader h{SNAP_MAGIC, s->ncell, s->precision, s->opt.kernel, s->cur, (int32_t)s->objs.size(),
-                 s->step_index, s->time, s->state_time};
+                 s->step_index, s->time, s->state_time, (int64_t)total};
     char* p = (char*)buffer;
     std::memcpy(p, &h, sizeof(h));
     p += sizeof(h);
@@ -1240,12 +1248,11 @@ fdtd_status fdtd_solver_restore(fdtd_solver* s, const void* buffer, int64_t byte
     SnapHeader h;
     if (bytes < (int64_t)sizeof(h)) return (set_error(s, "snapshot truncated"), FDTD_ERR_INVALID_ARG);
     std::memcpy(&h, buffer, sizeof(h));
-    if (h.magic != SNAP_MAGIC || h.ncell != s->ncell || h.precision != s->precision || h.kernel != s->opt.kernel ||
-        h.n_obj != (int32_t)s->objs.size())
-        return (set_error(s, "snapshot does not match this solver"), FDTD_ERR_INVALID_ARG);
     auto regs = snap_regions(s);
-    size_t total = sizeof(SnapHeader) + s->objs.size() * sizeof(HostObject);
-    for (auto& r : regs) total += r.second;
+    const size_t total = snap_total(s, regs);
+    if (h.magic != SNAP_MAGIC || h.ncell != s->ncell || h.precision != s->precision || h.kernel != s->opt.kernel ||
+        h.n_obj != (int32_t)s->objs.size() || h.total != (int64_t)total)
+        return (set_error(s, "snapshot does not match this solver"), FDTD_ERR_INVALID_ARG);
     if (bytes < (int64_t)total) return (set_error(s, "snapshot truncated"), FDTD_ERR_INVALID_ARG);
     CUDA_TRY(s, cudaSetDevice(s->opt.device));
     CUDA_TRY(s, cudaStreamSynchronize(s->stream));

@@ -468,7 +468,10 @@ fdtd_status fdtd_interior_step_noalloc(const double* p_curr, const double* p_pre
                                        double c2k2, double lap_scale, void* stream);
 
 /* Snapshot / restore of the resident state (_SaveSimulationSnapshot,
- * FDTD_AcousticSimulator.cpp:381-415).  bytes: query with buffer NULL. */
+ * FDTD_AcousticSimulator.cpp:381-415).  bytes: query with buffer NULL.  The
+ * snapshot is a raw image that names its layout and length: one of another
+ * layout (an older library's) or of a solver with other arrays is refused with
+ * FDTD_ERR_INVALID_ARG; room behind it in the buffer does not matter. */
 fdtd_status fdtd_solver_snapshot(fdtd_solver* s, void* buffer, int64_t* bytes);
 fdtd_status fdtd_solver_restore(fdtd_solver* s, const void* buffer, int64_t bytes);
 
