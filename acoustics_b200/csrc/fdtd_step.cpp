@@ -678,12 +678,23 @@ fdtd_status fdtd_solver_time_kernel(fdtd_solver* s, int32_t which, int32_t n_lau
     // only, whatever the host's launch rate (a step forks to three streams)
     fdtd_status jst = join_listeners(s);
     if (jst != FDTD_OK) return jst;
+    // moving bodies: the list of the last classification, whose lengths are those of
+    // its parity, in the launches of both (the next step's pair is empty again below)
+    int* const counts = s->d_ghost_count;
+    if (s->moving)
+        CUDA_TRY(s, cudaMemcpyAsync(counts + 2 * s->cur, counts + 2 * (s->cur ^ 1), 2 * sizeof(int),
+                                    cudaMemcpyDeviceToDevice, s->stream));
+    const bool one = which == 0 && s->region.one;
     CUDA_TRY(s, cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
     int c = s->cur;
     for (int i = 0; i < n_launches; ++i) {
         cudaError_t e;
         if (which == 4) {
             e = launch_listeners(s->dP, s->precision, c, s->L, s->d_lis, s->stream);
+        } else if (one) {
+            e = s->precision == FDTD_PRECISION_FP64
+                    ? launch_one_fp64(s->dP, s->hP, R, c, s->n_ghost, nullptr, s->stream, nullptr)
+                    : launch_one_fp32(s->dP, s->hP, R, c, s->n_ghost, nullptr, s->stream, nullptr);
         } else if (s->precision == FDTD_PRECISION_FP64) {
             if (s->opt.kernel == FDTD_KERNEL_PHASED) e = launch_phased_fp64(s->dP, s->N, c, phased_lap(s, c), s->stream, nullptr);
             else e = launch_step_regions_fp64(s->dP, s->hP, R, c, step_streams(s), nullptr);
@@ -715,6 +726,7 @@ fdtd_status fdtd_solver_time_kernel(fdtd_solver* s, int32_t which, int32_t n_lau
     if (ge == cudaSuccess) ge = cudaEventRecord(e1, s->stream);
     if (ge == cudaSuccess) ge = cudaEventSynchronize(e1);
     if (ge == cudaSuccess) ge = cudaEventElapsedTime(elapsed_ms, e0, e1);
+    if (ge == cudaSuccess && s->moving) ge = cudaMemsetAsync(counts + 2 * s->cur, 0, 2 * sizeof(int), s->stream);
     cudaGraphExecDestroy(x);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);

@@ -435,10 +435,12 @@ fdtd_status fdtd_solver_transfer_bytes(fdtd_solver* s, int64_t* host_to_device, 
  * fields are left in an unspecified state; use a solver created for measurement. */
 fdtd_status fdtd_solver_time_stencil(fdtd_solver* s, int32_t n_launches, float* elapsed_ms);
 /* The same for one part of the step: which = 0 the step kernels (as
- * fdtd_solver_time_stencil),
+ * fdtd_solver_time_stencil; the one launch of a solve whose step is one),
  * 1 the interior kernel, 2 the PML-shell kernel, 3 the ghost-cell list kernel,
- * 4 the listener kernel.  Parts 1-4 need FDTD_KERNEL_FUSED.  The fields are
- * left in an unspecified state (timing only). */
+ * 4 the listener kernel.  Parts 1-4 need FDTD_KERNEL_FUSED; 1-3 are the kernels
+ * of a step in several launches, for a solve that steps by one too.  Bodies stay
+ * where they are: the ghost-cell list is the last classification's.  The fields
+ * are left in an unspecified state (timing only). */
 fdtd_status fdtd_solver_time_kernel(fdtd_solver* s, int32_t which, int32_t n_launches, float* elapsed_ms);
 
 /* Interior leapfrog step that allocates nothing.  No counterpart in the
