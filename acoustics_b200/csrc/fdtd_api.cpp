@@ -1379,7 +1379,7 @@ fdtd_status fdtd_solver_destroy(fdtd_solver* s) {
     if (s->d_solid_pml) cudaFree(s->d_solid_pml);
     if (s->arena) arena_release(s->opt.device, s->arena, s->arena_block);
     host_release(s->h_lis_stage, s->h_lis_bytes);
-    if (s->rb_host) cudaFreeHost(s->rb_host);
+    host_release(s->rb_stage, s->rb_bytes);
     for (cudaEvent_t ev : s->rb_done)
         if (ev) cudaEventDestroy(ev);
     for (cudaEvent_t ev : {s->ev_fork, s->ev_join, s->ev_ghost, s->ev_step, s->ev_lis[0], s->ev_lis[1], s->ev_lis_join,

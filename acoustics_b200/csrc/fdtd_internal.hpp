@@ -153,9 +153,10 @@ struct fdtd_solver {
     long long last_launches = 0;
     long long graph_launches_per_exec = 0;
     fdtd::TmaStep* tma = nullptr;     // tiles and tensor maps of the TMA-staged shell (reduced state)
-    // read-backs (fields, cells): mapped host staging made on first use, a part and
-    // an event per worker
-    void* rb_host = nullptr;
+    // read-backs (fields, cells): pinned staging as large as any so far needed, a part
+    // and an event per worker
+    void* rb_stage = nullptr;
+    size_t rb_bytes = 0;
     cudaEvent_t rb_done[fdtd::READBACK_WORKERS] = {};
     const double* d_csig[3] = {nullptr, nullptr, nullptr};  // absorption at the cell centres
     // bytes this handle copied between host and device memory since creation
