@@ -1064,7 +1064,10 @@ fdtd_status fdtd_gaussian_source_defaults(fdtd_gaussian_source_desc* src, double
     return FDTD_OK;
 }
 
-fdtd_status fdtd_solver_create(const fdtd_scene_desc* sc, const fdtd_options* opt, fdtd_solver** out) {
+}  // extern "C"
+
+fdtd_status fdtd::solver_create(const fdtd_scene_desc* sc, const fdtd_options* opt, fdtd_solver** out,
+                                const std::function<void()>& on_memory) {
     if (!out) return (set_error(nullptr, "out is NULL"), FDTD_ERR_INVALID_ARG);
     *out = nullptr;
     std::vector<MeshHost> meshes;
@@ -1197,6 +1200,7 @@ fdtd_status fdtd_solver_create(const fdtd_scene_desc* sc, const fdtd_options* op
     }
     s->arena = base;
     s->arena_block = block;
+    if (on_memory) on_memory();
     s->arena_bytes = cv.off;
     for (auto& r : cv.req) *r.first = (char*)base + r.second;
     const long long ncell = s->ncell;
@@ -1359,6 +1363,12 @@ fdtd_status fdtd_solver_create(const fdtd_scene_desc* sc, const fdtd_options* op
     if (st != FDTD_OK) return st;
     *out = s.release();
     return FDTD_OK;
+}
+
+extern "C" {
+
+fdtd_status fdtd_solver_create(const fdtd_scene_desc* sc, const fdtd_options* opt, fdtd_solver** out) {
+    return fdtd::solver_create(sc, opt, out, nullptr);
 }
 
 void fdtd_release_cached_memory(int32_t device) { fdtd::free_kept(device); }

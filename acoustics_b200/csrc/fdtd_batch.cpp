@@ -463,7 +463,7 @@ namespace fdtd {
 
 fdtd_status batch_prepare(const fdtd_options& batch_opt, const fdtd_scene_desc* scene, int32_t steps_total,
                           const void* snapshot, int64_t snapshot_bytes, const double* rows, int64_t steps_done,
-                          PreparedMember* out, std::string* err) {
+                          PreparedMember* out, std::string* err, const std::function<void()>& on_memory) {
     auto fail = [&](fdtd_status code, const std::string& m, fdtd_solver* s) {
         if (s) fdtd_solver_destroy(s);
         *err = m;
@@ -481,7 +481,7 @@ fdtd_status batch_prepare(const fdtd_options& batch_opt, const fdtd_scene_desc* 
     o.graph_steps = 0;
     o.shell_staging = FDTD_SHELL_STAGING_RING;  // the batch kernels stage per thread
     fdtd_solver* s = nullptr;
-    fdtd_status st = fdtd_solver_create(scene, &o, &s);
+    fdtd_status st = solver_create(scene, &o, &s, on_memory);
     if (st != FDTD_OK) return fail(st, fdtd_last_error(), nullptr);
     if (s->moving) return fail(FDTD_ERR_UNSUPPORTED, "moving bodies are stepped by fdtd_solver, not in batches", s);
     if (!s->eng.empty()) return fail(FDTD_ERR_UNSUPPORTED, "batched members have a PML on every side", s);

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <array>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -211,7 +212,10 @@ struct PreparedMember {
 };
 fdtd_status batch_prepare(const fdtd_options& batch_opt, const fdtd_scene_desc* scene, int32_t steps_total,
                           const void* snapshot, int64_t snapshot_bytes, const double* rows, int64_t steps_done,
-                          PreparedMember* out, std::string* err);
+                          PreparedMember* out, std::string* err, const std::function<void()>& on_memory = nullptr);
+// fdtd_solver_create; on_memory is called as soon as the solver holds its device block
+fdtd_status solver_create(const fdtd_scene_desc* sc, const fdtd_options* opt, fdtd_solver** out,
+                          const std::function<void()>& on_memory);
 int32_t batch_place(fdtd_batch* b, PreparedMember&& pm);
 // Device blocks for solver arenas, kept after a solver is destroyed for the next
 // one on the same device (fdtd_api.cpp)

@@ -108,6 +108,7 @@ struct Request {
     fdtd_status prep_status = FDTD_OK;
     std::string prep_err;
     bool in_prep = false;           // handed to the preparer, not yet placed (it reads snap and rows)
+    bool backed = false;            // holds its device memory, or was refused it
 };
 
 }  // namespace
@@ -129,6 +130,7 @@ struct fdtd_server {
     std::deque<int64_t> to_prepare;      // admitted, waiting for the preparer
     std::vector<int64_t> prepared;       // made, waiting to join the batch
     int64_t preparing = 0;               // admitted and not yet placed
+    int64_t unbacked = 0;                // of these, those that do not hold their device memory yet
     fdtd_batch* batch = nullptr;
     std::string create_err;
     bool ready = false, failed_start = false;
@@ -244,10 +246,17 @@ void preparer_main(fdtd_server* S) {
         fdtd::PreparedMember pm;
         std::string err;
         const bool resumed = r->evicted_steps >= 0;
+        const auto backed = [S, r] {
+            std::lock_guard<std::mutex> g(S->mu);
+            if (r->backed) return;
+            r->backed = true;
+            if (--S->unbacked == 0) S->cv_done.notify_all();
+        };
         const fdtd_status st =
             fdtd::batch_prepare(S->opt, &r->scene.d, r->steps, resumed ? r->snap.data() : nullptr,
                                 resumed ? (int64_t)r->snap.size() : 0, resumed && !r->rows.empty() ? r->rows.data() : nullptr,
-                                resumed ? r->evicted_steps : 0, &pm, &err);
+                                resumed ? r->evicted_steps : 0, &pm, &err, backed);
+        backed();  // (refused before it came to that)
         std::lock_guard<std::mutex> g(S->mu);
         r->prep = std::move(pm);
         r->prep_status = st;
@@ -295,7 +304,9 @@ void worker_main(fdtd_server* S) {
                 S->queue.pop_front();
                 S->used_bytes += S->reqs[id]->bytes;
                 S->reqs[id]->in_prep = true;
+                S->reqs[id]->backed = false;
                 S->preparing++;
+                S->unbacked++;
                 S->to_prepare.push_back(id);
                 handed = true;
             }
@@ -522,6 +533,10 @@ fdtd_status fdtd_server_wait(fdtd_server* S, int64_t id, double timeout_s) {
     if (timeout_s < 0) S->cv_done.wait(lk, pred);
     else if (!S->cv_done.wait_for(lk, std::chrono::duration<double>(timeout_s), pred))
         return (fdtd::set_error(nullptr, "wait timed out"), FDTD_ERR_TIMEOUT);
+    // Requests are admitted on the memory that finished ones give back.  A client that
+    // allocates when its result is there must not take it first: they hold it by then,
+    // or do within a few milliseconds (a creation takes 0.2 ms; a long queue more).
+    S->cv_done.wait_for(lk, std::chrono::milliseconds(5), [&] { return S->stop || (S->unbacked == 0 && !admissible(S)); });
     Request* r = find(S, id);
     return r && (r->state == FDTD_REQ_FAILED || r->state == FDTD_REQ_CANCELLED) ? r->status : FDTD_OK;
 }

@@ -571,7 +571,9 @@ fdtd_status fdtd_server_submit(fdtd_server* srv, const fdtd_scene_desc* scene, i
 /* state (FDTD_REQ_*), steps done, and for failed requests the status */
 fdtd_status fdtd_server_poll(fdtd_server* srv, int64_t request, int32_t* state, int64_t* steps_done,
                              int32_t* status);
-/* block until the request is done or failed; FDTD_ERR_TIMEOUT after timeout_s (< 0: no limit) */
+/* block until the request is done or failed; FDTD_ERR_TIMEOUT after timeout_s (< 0: no limit).
+ * Requests admitted on the memory it gives back hold theirs by then (waited for up to 5 ms
+ * more), so that a client that allocates at once does not take it from them. */
 fdtd_status fdtd_server_wait(fdtd_server* srv, int64_t request, double timeout_s);
 /* steps x n_listeners doubles and the latency; the request is forgotten afterwards */
 fdtd_status fdtd_server_result(fdtd_server* srv, int64_t request, double* out, int64_t count, int64_t* steps,
