@@ -447,6 +447,7 @@ static __device__ __noinline__ double mesh_closest_ref_warp(const MeshView& M, c
         d2 = fabs(tri_closest_ref(q, M.tris[t], c));
         id = M.tris[t].id;
     });
+    tri = max(tri, 0);  // (none is nearer than infinity: a point as far away as a double allows)
     const double ds = tri_closest_ref(q, M.tris[tri], cp);
     return ds >= 0.0 ? sqrt(ds) : -sqrt(-ds);
 }
