@@ -106,7 +106,7 @@ __host__ __device__ constexpr int shell_vz(int word) { return word == 4 ? FDTD_S
 // shares with other boxes stay in the grid arrays: it reads its high x / y
 // faces at the far box ends from there, and writes its low x / y faces at
 // x = x0 / y = y0 to both (the x / y slabs read them as their high faces).
-constexpr int SHELL_MAX_BOXES = 9;
+constexpr int SHELL_MAX_BOXES = 5;  // four x / y slabs and the z-slab pair
 struct ShellBoxes {
     int n, xs, vz;
     int x0[SHELL_MAX_BOXES], nx[SHELL_MAX_BOXES], y0[SHELL_MAX_BOXES], ny[SHELL_MAX_BOXES];
@@ -216,7 +216,7 @@ struct RegionLaunch {
 };
 
 // Two copies indexed by the step parity: the kernels of a step read
-// consts[cur]; one thread of the step writes consts[cur^1] for the next step.
+// consts[cur]; one warp of the step writes consts[cur^1] for the next step.
 struct StepConsts {
     double t;                       // simulation time at the start of the step
     double src_tf[FDTD_MAX_SOURCES];  // exp(-((t+k/2 - t0)/wt)^2/2)
@@ -224,7 +224,8 @@ struct StepConsts {
     int64_t step;
 };
 
-// One cell of the ghost-neighbour list of a static scene with what its update
+// One cell of the ghost-neighbour list (of a static scene, and of moving analytic
+// bodies, whose classification makes it each step) with what its update
 // needs besides pressures and the step's factors: its flags, place, and per
 // direction f = 2 axis + (sign > 0) with a solid neighbour the body whose
 // acceleration moves that face (GHOST_STILL: none) and the component along the axis
@@ -359,14 +360,15 @@ struct SolveParams {
     int* ghost_count;             // its cells and, next to it, the fresh cells (list_counts)
     int ghost_cap;
     int moving;                   // some body moves
-    GhostPlan* ghost_plan;        // [plan_cap] the list's cells prepared (static scenes)
+    GhostPlan* ghost_plan;        // [plan_cap] the list's cells prepared (static scenes, moving analytic bodies)
     int plan_cap;
     int plan_ready;               // ghost_plan valid for the current classification
     ClsBoxes boxes;               // iteration boxes of the latest classification
     int* fresh_list;              // bulk cells without a valid history (found by the classification sweep)
     int fresh_cap;
     int precision;                // 0 fp64, 1 fp32 compensated
-    // FULLY_COUPLED ghost cells (static scenes; null under RASTERIZE)
+    // FULLY_COUPLED ghost cells (made again after each classification of moving
+    // bodies; null under RASTERIZE)
     const FcRow* fc_rows;         // [fc_n] one row per ghost face, owners ascending, directions ascending
     const int* fc_idx;            // [np] per ghost (solid) cell: (first row << 6) | bulk-direction mask; -1 elsewhere
     double* fc_b;                 // [fc_n] right-hand side of the step
@@ -577,14 +579,6 @@ __host__ __device__ __forceinline__ void dense_ijk(const SolveParams& P, long lo
 // emptied it) and empties the other.
 __device__ __forceinline__ int* list_counts(const SolveParams& P, int cur) {
     return P.ghost_count + (P.moving ? 2 * cur : 0);
-}
-
-// Some Gaussian source contributes at the step of parity `cur` (its time
-// factor has not underflowed to zero).
-__device__ __forceinline__ bool sources_on(const SolveParams& P, int cur) {
-    bool any = false;
-    for (int s = 0; s < P.n_src; ++s) any |= P.consts[cur].src_tf[s] != 0.0;
-    return any;
 }
 
 // sum_s G_s(x, t + k/2) at cell (x, y, z) (GaussianPressureSource.cpp:6-30): the

@@ -22,10 +22,14 @@ namespace fdtd {
 // Cell classification (MAC_Grid::classifyCells_FAST, MAC_Grid.cpp:3455-3891)
 // ---------------------------------------------------------------------------
 
-// A classification is two launches.  k_cls_boxes visits the cells of the
+// A moving step's classification of analytic bodies is one launch (k_cls_tiles).
+// The others (the first of a solve, a static scene's, mesh bodies) take up to three.
+// k_cls_boxes (k_cls_boxes_mesh) visits the cells of the
 // iteration boxes (each cell once) and makes their new bulk / valid bits, the
 // solid test of MAC_Grid.cpp:3608-3653 with the zeroing of solid pressures
-// (MAC_Grid.cpp:3796-3798).  k_cls_sweep then visits every cell as "quads":
+// (MAC_Grid.cpp:3796-3798).  k_cls_sweep, or k_cls_sweep_prev where only the cells
+// that the boxes before reached can hold other flags than the defaults, and
+// k_cls_near beside the boxes then visit cells as "quads":
 // four cells of one z row, read and written as one 32-bit word (rows start at
 // multiples of 8 bytes, and a quad never reaches past its row's padding), one
 // quad per thread.  A cell outside every box is bulk with

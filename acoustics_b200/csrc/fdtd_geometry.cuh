@@ -67,13 +67,6 @@ FDTD_HD double distance_to_mesh(const DevObject& o, const double p[3]) {
     return sdf_local(o, p);
 }
 
-// FDTD_Objects::OccupyByObject (FDTD_Objects.cpp:35-49)
-FDTD_HD int occupy_by_object(const SolveParams& P, const double p[3]) {
-    for (int o = 0; o < P.n_obj; ++o)
-        if (distance_to_mesh(P.obj[o], p) < DISTANCE_TOLERANCE) return o;
-    return -1;
-}
-
 // FDTD_Objects::OccupyByConstraint + FDTD_PlaneConstraint::Inside (FDTD_PlaneConstraint.h:33-38)
 FDTD_HD bool occupy_by_constraint(const SolveParams& P, const double p[3]) {
     for (int i = 0; i < P.n_plane; ++i)
@@ -102,7 +95,8 @@ FDTD_HD bool in_scaled_bbox(const DevObject& o, const double p[3]) {
 }
 
 // isFluid lambda of classifyCells_FAST (MAC_Grid.cpp:3566-3577): the centre and
-// the six points centre +- h/4 along each axis must be outside every object.
+// the six points centre +- h/4 along each axis must be outside every object
+// (FDTD_Objects::OccupyByObject, FDTD_Objects.cpp:35-49).
 // The samples are tried only against the bodies that can reach one: a body
 // whose box, or whose surface, is farther than h/4 from the centre cannot (the
 // distances of spheres, boxes and meshes are exact; an ellipsoid's is an

@@ -9,7 +9,8 @@ namespace fdtd {
 
 // Streams of one step.  The step is enqueued on s and ends on s; in between the
 // ghost-cell list runs on s3 (launched first: a few latency-bound CTAs next to
-// the interior's), the interior and then the sources on s2, the PML shell on s.
+// the interior's), the interior on s2 (then the sources, where the two do not add
+// them), the PML shell on s.
 // s2 / s3 may be null (everything on s).
 struct StepStreams {
     cudaStream_t s, s2, s3;

@@ -212,10 +212,9 @@ FDTD_MHD double tri_closest_ref(const double q[3], const MeshTri& T, double cp[3
 
 // Both queries walk the hierarchy nearer child first and skip a box farther
 // than the best squared distance so far (ties are still visited).
-// mesh_sdf: exact signed distance (pseudo-normal sign).  `bound2`: a squared
-// distance known to be no smaller than the answer's (boxes beyond it are skipped).
-FDTD_MHD double mesh_sdf(const MeshView& M, const double q[3], double bound2 = DBL_MAX) {
-    double best = bound2, best_s = 0.0;
+// mesh_sdf: exact signed distance (pseudo-normal sign).
+FDTD_MHD double mesh_sdf(const MeshView& M, const double q[3]) {
+    double best = DBL_MAX, best_s = 0.0;
     int best_id = INT_MAX;
     int stack[MESH_STACK];
     int sp = 0;

@@ -5,22 +5,25 @@
 //                (MAC_Grid.cpp:187-299 + :921-944).  Only pressure words move:
 //                p^n (neighbours from the CTA's rows), p^{n-1} or the increment,
 //                p^{n+1}, plus one classification byte.
-//   k_pml_shell  the six slab boxes of the PML shell: face velocities
-//                (MAC_Grid.cpp:461-479) and split-field pressures (:496-508).
+//   k_pml_shell  the PML shell's boxes (two x and two y slabs, the pair of z slabs
+//                between them): face velocities (MAC_Grid.cpp:461-479) and
+//                split-field pressures (:496-508).
 //
 // Face ownership: a PML face is written by the cell to its right; the one face
 // layer whose right cell is not a PML cell (x = W h on the low side) is written
 // by its left (PML) cell, so the interior kernel never touches velocities.
 //
-// Cells next to a solid (a compact list built by the classification) and the
-// Gaussian sources while they are active have kernels of their own, so the
-// interior kernel is a pure 7-point leapfrog.
+// Cells next to a solid (a compact list built by the classification) have a kernel
+// of their own, so the interior kernel is a pure 7-point leapfrog.  Both add the
+// Gaussian sources, while they are active, to the cells they own (k_sources does
+// it after them where the interior takes an explicit chunk of x planes).
 //
-// Interior mapping: a CTA of 32 (z) x 8 (y) threads, each thread owns XB
-// consecutive x planes of one (y, z) column.  All loads of the XB planes
-// (p^n at XB+2 planes, y neighbours, p^{n-1}/increment, classification) are
-// issued before any arithmetic so that every thread keeps ~5*XB independent
-// HBM requests in flight; z neighbours come from the warp with shuffles.
+// Interior mapping: a CTA takes 256 consecutive units of the box, one per thread;
+// a unit is a z group (16 bytes: 4 FP32 or 2 FP64 cells) of one (x, y) row, at XB
+// consecutive x planes.  All loads of the XB planes (p^n at XB+2 planes, y
+// neighbours, p^{n-1}/increment, classification) are issued before any arithmetic
+// so that every thread keeps ~5*XB independent HBM requests in flight; z neighbours
+// come from the lanes beside it with shuffles (interior_tile).
 #pragma once
 #include "fdtd_device.cuh"
 #include "fdtd_coupled.cuh"
