@@ -748,12 +748,13 @@ __device__ __forceinline__ bool in_pml(const SolveParams& P, int i, int j, int k
 // ---------------------------------------------------------------------------
 // Out of line: the few fresh cells of a step run this once per launch, and one
 // copy of the code misses the instruction cache less than several inlined ones.
-template <typename T>
+// HELD: p^{n-1} of PML cells is read from pb, where that is not pa.
+template <typename T, bool HELD>
 __device__ __noinline__ double fresh_value(const SolveParams& P, const T* __restrict__ pa, const T* __restrict__ pb,
                                            bool diff, long long c, double t, int* status, long long& next) {
     // value of buffer "a" (or a - b when diff) at cell n, of the stencil in the PML where it is held
     auto val = [&](long long n) -> double { return diff ? (double)pa[n] - (double)pb[n] : (double)pa[n]; };
-    const bool held = !diff && pb != pa;
+    const bool held = HELD && pb != pa;
     int i, j, k;
     cell_ijk(P, c, i, j, k);
     const double cp[3] = {P.cpos[0][i], P.cpos[1][j], P.cpos[2][k]};
@@ -823,7 +824,7 @@ __device__ __noinline__ double fresh_value(const SolveParams& P, const T* __rest
     return c0 + P.rho * an * fabs(travelled);
 }
 
-template <typename T>
+template <typename T, bool HELD>
 __device__ __forceinline__ void fresh_cell(const SolveParams& P, int cur, long long c, double t, int* st,
                                            const T* held) {
     // (the cell itself, or the one its value is a copy of)
@@ -831,7 +832,7 @@ __device__ __forceinline__ void fresh_cell(const SolveParams& P, int cur, long l
         double v = 0.0;
         for (long long at = c; at >= 0;) {
             long long next = -1;
-            v = fresh_value<T>(P, pa, pb, diff, at, t, st, next);
+            v = fresh_value<T, HELD>(P, pa, pb, diff, at, t, st, next);
             at = next;
         }
         return v;
@@ -839,7 +840,7 @@ __device__ __forceinline__ void fresh_cell(const SolveParams& P, int cur, long l
     if (sizeof(T) == 8) {
         T* pl = (T*)P.p[cur ^ 1];
         T* pc = (T*)P.p[cur];
-        const double vl = value(pl, held ? held : pl, false);
+        const double vl = value(pl, HELD ? held : pl, false);
         const double vc = value(pc, pc, false);
         pl[c] = vl;
         pc[c] = vc;
@@ -906,7 +907,7 @@ __device__ __forceinline__ bool fresh_geometry(const SolveParams& P, long long c
 // add nothing, so the result is bit-equal to householder_ls4_rows8 over the
 // same rows.  All 32 lanes must call it with the same cell (both halves take
 // the same branches: they share the image point and the stencil flags).
-template <typename T>
+template <typename T, bool HELD>
 __device__ __noinline__ double fresh_value_half(const SolveParams& P, const FreshGeometry& G, const T* __restrict__ pa,
                                                 const T* __restrict__ pb, bool diff, long long c, double t,
                                                 long long& next) {
@@ -944,7 +945,7 @@ __device__ __noinline__ double fresh_value_half(const SolveParams& P, const Fres
     if (in_stencil) {
         const long long n = cidx(P, ni, nj, nn);
         valid = (P.cls[n] & CLS_VALID) != 0;
-        const bool held = !diff && pb != pa && in_pml(P, ni, nj, nn);
+        const bool held = HELD && pb != pa && in_pml(P, ni, nj, nn);
         vq = diff ? (double)pa[n] - (double)pb[n] : held ? (double)pb[n] : (double)pa[n];
         pq[0] = P.cpos[0][ni];
         pq[1] = P.cpos[1][nj];
@@ -1042,7 +1043,7 @@ __device__ __noinline__ double fresh_value_half(const SolveParams& P, const Fres
 // order does not matter.  (Two CTAs per SM asked for: the compiler made room for three
 // otherwise, spilling 256 bytes in fresh_value and 112 here, where two need none, and a step of
 // moving bodies took 0.5 % longer.)
-template <typename T>
+template <typename T, bool HELD>
 __global__ void __launch_bounds__(128, 2) k_fresh_cells(const SolveParams* __restrict__ Pp, int cur, long long n,
                                                      int* status, const T* held) {
     const SolveParams& P = *Pp;
@@ -1057,7 +1058,7 @@ __global__ void __launch_bounds__(128, 2) k_fresh_cells(const SolveParams* __res
             const long long c = cidx(P, i, j, k);
             const uint8_t code = P.cls[c];
             if (!(code & CLS_BULK) || (code & CLS_VALID)) continue;
-            fresh_cell<T>(P, cur, c, t, &st, held);
+            fresh_cell<T, HELD>(P, cur, c, t, &st, held);
         }
         if (st) atomicMax(status, st);
         return;
@@ -1074,8 +1075,8 @@ __global__ void __launch_bounds__(128, 2) k_fresh_cells(const SolveParams* __res
             if (fresh_geometry(P, at, stacks[threadIdx.x >> 5], G)) {
                 // FP32: p^{n-1} is p^n less the increment; FP64: in the PML held apart, or not
                 const T* pa = (const T*)P.p[sizeof(T) == 8 ? cur ^ w : cur];
-                const T* pb = sizeof(T) == 4 ? (const T*)(const void*)P.dinc : w && held ? held : pa;
-                v = fresh_value_half<T>(P, G, pa, pb, sizeof(T) == 4 && w, at, t, next);
+                const T* pb = sizeof(T) == 4 ? (const T*)(const void*)P.dinc : HELD && w ? held : pa;
+                v = fresh_value_half<T, HELD>(P, G, pa, pb, sizeof(T) == 4 && w, at, t, next);
             } else {
                 st = 2;
             }
@@ -1322,8 +1323,9 @@ cudaError_t launch_fresh_cells(const SolveParams* dP, int precision, int cur, lo
                                cudaStream_t s, const double* held) {
     // the list, a warp per cell (a few thousand cells a step at most)
     const int grid = 4 * 148;
-    if (precision == 0) k_fresh_cells<double><<<grid, 128, 0, s>>>(dP, cur, ncell, d_status, held);
-    else k_fresh_cells<float><<<grid, 128, 0, s>>>(dP, cur, ncell, d_status, nullptr);
+    if (precision != 0) k_fresh_cells<float, false><<<grid, 128, 0, s>>>(dP, cur, ncell, d_status, nullptr);
+    else if (held) k_fresh_cells<double, true><<<grid, 128, 0, s>>>(dP, cur, ncell, d_status, held);
+    else k_fresh_cells<double, false><<<grid, 128, 0, s>>>(dP, cur, ncell, d_status, nullptr);
     return cudaGetLastError();
 }
 
