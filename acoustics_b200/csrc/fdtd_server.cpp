@@ -336,6 +336,7 @@ void worker_main(fdtd_server* S) {
                 r->snap.shrink_to_fit();
                 r->rows.clear();
                 r->rows.shrink_to_fit();
+                S->cv_done.notify_all();
                 continue;
             }
             if (r->prep_status != FDTD_OK) {
@@ -566,7 +567,8 @@ fdtd_status fdtd_server_result(fdtd_server* S, int64_t id, double* out, int64_t 
 fdtd_status fdtd_server_drain(fdtd_server* S, double timeout_s) {
     if (!S) return FDTD_ERR_INVALID_ARG;
     std::unique_lock<std::mutex> lk(S->mu);
-    auto pred = [&] { return S->stop || (S->queue.empty() && S->running.empty()); };
+    // (a request with the preparer is in neither: it counts until it is placed)
+    auto pred = [&] { return S->stop || (S->queue.empty() && S->preparing == 0 && S->running.empty()); };
     if (timeout_s < 0) S->cv_done.wait(lk, pred);
     else if (!S->cv_done.wait_for(lk, std::chrono::duration<double>(timeout_s), pred))
         return (fdtd::set_error(nullptr, "drain timed out"), FDTD_ERR_TIMEOUT);
