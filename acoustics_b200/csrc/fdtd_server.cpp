@@ -131,6 +131,7 @@ struct fdtd_server {
     std::vector<int64_t> prepared;       // made, waiting to join the batch
     int64_t preparing = 0;               // admitted and not yet placed
     int64_t unbacked = 0;                // of these, those that do not hold their device memory yet
+    bool stepping = false;               // the worker is in a chunk of steps: it admits after it
     fdtd_batch* batch = nullptr;
     std::string create_err;
     bool ready = false, failed_start = false;
@@ -361,6 +362,7 @@ void worker_main(fdtd_server* S) {
         {
             std::lock_guard<std::mutex> g(S->mu);
             any_running = !S->running.empty();
+            S->stepping = any_running;
         }
         if (!any_running) continue;
         int32_t n_active = 0;
@@ -369,6 +371,7 @@ void worker_main(fdtd_server* S) {
         std::vector<std::pair<int32_t, int64_t>> members;
         {
             std::lock_guard<std::mutex> g(S->mu);
+            S->stepping = false;
             members.assign(S->running.begin(), S->running.end());
         }
         for (auto& mr : members) {
@@ -537,7 +540,8 @@ fdtd_status fdtd_server_wait(fdtd_server* S, int64_t id, double timeout_s) {
     // Requests are admitted on the memory that finished ones give back.  A client that
     // allocates when its result is there must not take it first: they hold it by then,
     // or do within a few milliseconds (a creation takes 0.2 ms; a long queue more).
-    S->cv_done.wait_for(lk, std::chrono::milliseconds(5), [&] { return S->stop || (S->unbacked == 0 && !admissible(S)); });
+    S->cv_done.wait_for(lk, std::chrono::milliseconds(5),
+                        [&] { return S->stop || (S->unbacked == 0 && (S->stepping || !admissible(S))); });
     Request* r = find(S, id);
     return r && (r->state == FDTD_REQ_FAILED || r->state == FDTD_REQ_CANCELLED) ? r->status : FDTD_OK;
 }
